@@ -293,6 +293,9 @@ struct rla_sketch {
     uint32_t *extra = nullptr;     // deferred items: 32 words (one per lane) per extra round
     int64_t extra_rounds_cap = 0;
     int batch_mode = 0;            // 1: CountSketch schedule over 512-element batches (see rla_sketch.cu)
+    bool bl_ok = false;            // bucket lists built for the current draws (rla_sparse_tile.cu)
+    uint32_t *bl_words = nullptr;  // per chunk of long indices: entries sorted by (window, warp, bucket)
+    int2 *bl_lists = nullptr;      // per (chunk, window, warp): first word and word count, in fours
     int64_t *tp_ptr = nullptr;     // sparse-operand plan (rla_sparse_op.cu): [s+1] offsets per bucket
     int32_t *tp_idx = nullptr;     // [L*nnz] entries j*nnz+slot by bucket, j increasing
     uint64_t tp_version = 0;       // draw_count the plan was built for

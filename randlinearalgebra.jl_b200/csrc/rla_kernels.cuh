@@ -36,6 +36,13 @@ template <class T>
 int sparse_expand(rla_ctx *ctx, const rla_sketch *sk, const T *X, int64_t x_es, int64_t x_vs, int64_t nv, T *Y,
                   int64_t y_es, int64_t y_vs, double alpha, double beta);
 
+// SparseSign / CountSketch compress on 32-vector tiles (rla_sparse_tile.cu): tile_plan_build
+// makes the bucket lists for the current draws and sets sk->bl_ok when they cover the sketch.
+int tile_plan_build(rla_ctx *ctx, rla_sketch *sk);
+template <class T>
+int tile_compress(rla_ctx *ctx, const rla_sketch *sk, const T *X, int64_t x_es, int64_t x_vs, int64_t nv, T *Y,
+                  int64_t y_es, int64_t y_vs, T alpha, T beta, bool beta_zero);
+
 // SRHT / FJLT (rla_wht.cu)
 // Builds sk->sign_tl (per-thread sign masks of the fused compress kernel) from sk->signbits.
 int build_srht_sign_table(rla_ctx *ctx, rla_sketch *sk);

@@ -66,12 +66,12 @@ size_t req_bytes(const rla_request &r) {
 // depends on the request alone, so a request's result is the same alone and in any mix.
 bool groupable(const rla_request &r) { return r.kind == RLA_REQ_SVD && r.k <= 128 && r.m * r.n <= ((int64_t)1 << 22); }
 
-// Estimated device bytes of a resident sketch: SparseSign draws (bucket, sign, schedule
-// word per entry) and their per-tile schedule, or a dense Gaussian operator.
+// Estimated device bytes of a resident sketch: SparseSign draws (bucket, sign, list word per
+// entry, about half as many filling words again), or a dense Gaussian operator.
 size_t sketch_bytes(int kind, int64_t s, int64_t L) {
     if (kind == RLA_GAUSSIAN) return (size_t)(4 * s * L) + 4096;
     const int64_t nnz = std::min<int64_t>(8, s);
-    return (size_t)(L * (9 * nnz + 20)) + 4096;
+    return (size_t)(L * (9 * nnz + 12 * std::min<int64_t>(nnz, s / 640 + 1))) + 65536;
 }
 
 struct CacheEntry {

@@ -427,7 +427,13 @@ static int srht_tables(rla_ctx *ctx, rla_sketch *sk) {
 }
 
 static int build_meta(rla_ctx *ctx, rla_sketch *sk) {
+    // SparseSign: the tile kernel takes every layout.  CountSketch: it takes the strided vectors of
+    // a Right sketch (A*S on column-major A); contiguous ones keep the batch schedule below.
+    if (sk->nnz > 1 || sk->p.card == RLA_RIGHT) RLA_TRY(tile_plan_build(ctx, sk));
+    if (sk->bl_ok && sk->nnz > 1) return RLA_OK;
     if (sk->s > (1 << 22)) return RLA_OK;  // compression dimension beyond the packed form: strided/expand paths only
+    if (!sk->meta)
+        RLA_CUDA_TRY(ctx, cudaMalloc(&sk->meta, sizeof(uint32_t) * (size_t)ceil_div(sk->L, 128) * 128 * sk->nnz));
     sk->batch_mode = (sk->nnz == 1 && sk->s <= 65536) ? 1 : 0;
     if (sk->batch_mode) {
         const int64_t nb = ceil_div(sk->L, CS_BATCH);
@@ -572,7 +578,7 @@ int sketch_redraw_async(rla_ctx *ctx, rla_sketch *sk) {
 static void free_sketch_buffers(rla_sketch *sk) {
     void *ptrs[] = {sk->bucket, sk->negative, sk->meta, sk->rows, sk->signbits, sk->sign_tl, sk->tile_flags, sk->extra, sk->p2_ptr, sk->p2_list,
                     sk->k_ptr, sk->k_col, sk->k_val, sk->kt_ptr, sk->kt_row, sk->kt_val, sk->dense,
-                    sk->sidx, sk->splan, sk->sweights, sk->s_err, sk->tp_ptr, sk->tp_idx};
+                    sk->sidx, sk->splan, sk->sweights, sk->s_err, sk->tp_ptr, sk->tp_idx, sk->bl_words, sk->bl_lists};
     for (void *p : ptrs)
         if (p) cudaFree(p);
 }
@@ -638,7 +644,6 @@ int rla_sketch_create(rla_ctx *ctx, const rla_sketch_params *pp, rla_sketch **ou
             size_t ne = (size_t)(sk->L * sk->nnz);
             alloc((void **)&sk->bucket, ne * 4);
             alloc((void **)&sk->negative, ne);
-            alloc((void **)&sk->meta, (size_t)ceil_div(sk->L, 128) * 128 * sk->nnz * 4);
             break;
         }
         case RLA_SRHT:

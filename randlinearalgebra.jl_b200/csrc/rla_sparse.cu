@@ -17,6 +17,7 @@
 //    the bucket is warp-uniform, bins are [bucket][lane] (conflict-free).
 //  * expand (S'*A, A*S' ...): a gather, one thread per output element.
 #include "rla_internal.cuh"
+#include "rla_kernels.cuh"
 
 namespace rla {
 
@@ -689,6 +690,11 @@ int sparse_compress(rla_ctx *ctx, const rla_sketch *sk, const T *X, int64_t x_es
     const bool beta_zero = beta == 0.0;
     const T a = (T)(alpha * sk->scale);
     if (nv == 0) return RLA_OK;
+    // nnz > 1: the tile kernel for every layout (150001 -> 1332 of 333 columns: 257 us against 603 us
+    // below); nnz = 1: for strided vectors, while contiguous ones keep the batch kernel, whose
+    // warps read each element's word once and fill HBM better (s = 4096 would take four windows).
+    if (sk->bl_ok && (x_es != 1 || !sk->batch_mode))
+        return tile_compress<T>(ctx, sk, X, x_es, x_vs, nv, Y, y_es, y_vs, a, (T)beta, beta_zero);
     if (x_es == 1) {
         // contiguous vectors
         if (!sk->tile_flags)

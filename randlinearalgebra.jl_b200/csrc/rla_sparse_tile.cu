@@ -1,0 +1,580 @@
+// rla_sparse_tile.cu -- SparseSign / CountSketch compress on tiles of 128-byte rows.
+//
+// Y(b, v) = sum over the entries (j, b) of the sketch of sign(j, b) * X(j, v): every input
+// element is used nnz times, so the pass is bound by shared-memory traffic, not by HBM, unless
+// one access moves a full row of useful values.  A tile holds R = 640 long indices of 32 (Float32)
+// or 16 (Float64) vectors, one 128-byte row per long index, and 8 lanes ("an octet") handle one
+// entry with 16-byte accesses: reading row j and adding to the bins of bucket b are then one
+// conflict-free wavefront each whatever j and b are, and a warp instruction serves four entries.
+// The entries of a chunk of R long indices are kept sorted by bucket (built when the sketch is
+// drawn) and cut into groups of four entries of one bucket, the last group of a bucket filled up
+// with a row of zeros: a step of the kernel adds one group per octet to its bucket, with no
+// branches.  With e = R * nnz / s entries per bucket and chunk and g = ceil(e/4) groups,
+//   wavefronts per bucket and chunk = g * (4 rows + 2 bins + 1/4 words).
+// Measured (unprofiled call): 150001 -> 1332 (nnz 8) of 333 Float32 columns 257 us, 603 us with one
+// output vector per warp and private bins; 3000 -> 100 (nnz 8) of 30011 Float32 rows 307 us,
+// 1526 us with lane = vector bins; 4096 -> 512 of 256 Float64 columns 40 against 71 us.  The
+// shared-memory pipe is 73 % busy at the second size.  Entry by entry with an end-of-run
+// flag instead of filled groups takes fewer wavefronts and half again as many instructions: 258
+// and 308 us.
+// A CTA of 16 warps walks (vector tile, bucket window, chunk) units; each warp owns the
+// buckets congruent to it modulo 16, so there are no atomics and the result is reproducible bit
+// for bit.  Vectors that are contiguous in j (columns of a column-major A) are transposed on the
+// way into shared memory, strided ones (rows) copied as they are.  The next unit's elements are
+// loaded into registers while the current one is summed.
+//
+// The tile takes 80 KB, the bins the rest: a window holds 1040 buckets (R = 640 is the largest
+// that leaves 1024); a larger s takes several windows, each staging X again.
+#include "rla_internal.cuh"
+#include "rla_kernels.cuh"
+
+namespace rla {
+
+constexpr int BL_WARPS = 16;       // warps of the compress CTA, lists per (chunk, window)
+constexpr int BL_BUILD_WARPS = 8;  // warps of the plan builder
+constexpr int BL_R = 640;          // long indices per chunk
+constexpr int BL_MAX_SW = 1040, BL_MAX_WIN = 8, BL_MAX_NNZ = 32;
+constexpr int BL_PITCH = 144;      // bytes between bins of consecutive buckets (128 + 16)
+constexpr int BL_PF = 10;          // 16-byte loads per thread and unit
+static_assert(BL_R * 8 == BL_PF * BL_WARPS * 32, "a unit is BL_PF 16-byte loads per thread");
+// Entry word: bits 4..16 byte offset of row j with its swizzle, bits 17..30 offset of the
+// bucket's bins in 16-byte units (used from the first word of a group), bit 31 sign.
+constexpr uint32_t BL_ROW_MASK = 0x1fff0u, BL_BIN_MASK = 0x3fff0u;
+constexpr int BL_BIN_SHIFT = 17;
+constexpr uint32_t BL_ZERO_ROW = (uint32_t)BL_R << 7;  // row R of the tile holds zeros
+constexpr int BL_SLOW = 1 << 30;   // list flag: two octets may update one bucket in the same step
+constexpr int BL_AHEAD = 7;         // steps whose words a lane holds
+constexpr int BL_SLACK = 2 * BL_AHEAD * 16;  // words read ahead of the end of a list (and never used)
+constexpr int BL_TILE_BYTES = (BL_R + 1) * 128;
+
+template <class T>
+struct TileCfg {
+    static constexpr int VR = 16 / (int)sizeof(T);  // elements per 16 bytes
+    static constexpr int C = 8 * VR;                // vectors per tile
+};
+template <class T>
+struct TileVec;
+template <>
+struct TileVec<float> {
+    using type = float4;
+};
+template <>
+struct TileVec<double> {
+    using type = double2;
+};
+
+// Row j keeps 16-byte slot q at q ^ swz(j): the transposing stores of a warp (8 lanes along j
+// in steps of VR, 4 vectors) then hit distinct banks.
+template <class T>
+__host__ __device__ constexpr int tile_swz(int j) {
+    constexpr int VR = TileCfg<T>::VR;
+    return (j / VR + (8 / VR) * (j % VR)) & 7;
+}
+template <class T>
+__device__ __forceinline__ uint32_t tile_off(int j, int c) {
+    constexpr int VR = TileCfg<T>::VR;
+    return ((uint32_t)j << 7) | ((uint32_t)((c / VR) ^ tile_swz<T>(j)) << 4) | ((uint32_t)(c % VR) * (uint32_t)sizeof(T));
+}
+
+// ------------------------------------------------------------------------------------
+// Plan: per (chunk, window, warp) the groups of the warp's buckets in bucket order, cut into four
+// equal parts, one per octet, interleaved so that a step's words are 64 consecutive bytes.  The
+// groups of a bucket that crosses a cut are added by both octets, in different steps unless the
+// bucket has more groups than a part: such lists are marked BL_SLOW.  Filling groups point at the
+// zero row and at a bin past the last one.  With few buckets (s * G < 256) a bucket is kept G
+// times (long index modulo G picks the copy), so that the warps' shares are even; the copies are
+// added when the bins are written.
+// ------------------------------------------------------------------------------------
+struct BlGeom {
+    int nwin, sw, G, spw;  // windows, buckets per window, copies, keys (bucket copies) per warp
+    int64_t nchunk, cap;   // cap: words reserved per chunk, a multiple of 16
+};
+
+static bool bl_geometry(const rla_sketch *sk, BlGeom *g) {
+    if (sk->nnz > BL_MAX_NNZ || sk->s > (int64_t)BL_MAX_WIN * BL_MAX_SW) return false;
+    g->nwin = (int)ceil_div(sk->s, BL_MAX_SW);
+    g->sw = (int)ceil_div(sk->s, g->nwin);
+    g->G = 1;
+    if (g->nwin == 1)
+        while (g->G < 16 && g->sw * g->G < 256 && (int64_t)BL_R * sk->nnz >= 8 * (int64_t)g->sw * g->G) g->G *= 2;
+    g->spw = ceil_div_i((int64_t)g->sw * g->G, BL_WARPS);
+    g->nchunk = ceil_div(sk->L, BL_R);
+    const int64_t ne = (int64_t)BL_R * sk->nnz, keys = (int64_t)g->nwin * BL_WARPS * g->spw;
+    g->cap = (ne + 3 * std::min(ne, keys) + 15 * BL_WARPS * g->nwin + 15) / 16 * 16 + BL_SLACK;
+    return true;
+}
+
+// One CTA per chunk: a stable counting sort by (window, warp, bucket).  Warp w counts and later
+// places rows [w*R/8, (w+1)*R/8) in increasing order; ranks inside a warp access come from
+// match_any, so the order of a bucket's entries is the order of the long indices.
+template <class T>
+__global__ void __launch_bounds__(BL_BUILD_WARPS * 32) bl_build_kernel(const int32_t *bucket, const uint8_t *negative,
+                                                                       int64_t L, int nnz, BlGeom g, uint32_t *words,
+                                                                       int2 *lists) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int K = g.nwin * BL_WARPS * g.spw, nlist = g.nwin * BL_WARPS;
+    uint16_t *hist = reinterpret_cast<uint16_t *>(smem_raw);  // [8][K] counts, then offsets inside the bucket
+    uint16_t *tot = hist + BL_BUILD_WARPS * K;                // [K]
+    uint16_t *koff = tot + K;                                 // [K] first group of the bucket in its list
+    __shared__ int lstart[BL_MAX_WIN * BL_WARPS], lpart[BL_MAX_WIN * BL_WARPS], lslow[BL_MAX_WIN * BL_WARPS];
+    const int t = threadIdx.x, nt = blockDim.x, lane = t & 31, w = t >> 5;
+    const int64_t chunk = blockIdx.x, row0 = chunk * BL_R;
+    for (int i = t; i < BL_BUILD_WARPS * K; i += nt) hist[i] = 0;
+    __syncthreads();
+    constexpr int rows_w = BL_R / BL_BUILD_WARPS;
+    const int rlo = w * rows_w;
+    const int rcnt = (int)max((int64_t)0, min((int64_t)rows_w, L - row0 - rlo));
+    const int ne = rcnt * nnz;
+    const int64_t base = (row0 + rlo) * nnz;
+    uint16_t *myh = hist + w * K;
+    uint32_t *out = words + chunk * g.cap;
+    for (int pass = 0; pass < 2; ++pass) {
+        for (int i0 = 0; i0 < ne; i0 += 32) {
+            const int i = i0 + lane;
+            const bool valid = i < ne;
+            const int jl = rlo + (valid ? i / nnz : 0);
+            const uint32_t b = valid ? (uint32_t)bucket[base + i] : 0u;
+            const int win = (int)(b / (uint32_t)g.sw);
+            const int vlb = (jl & (g.G - 1)) * g.sw + (int)b - win * g.sw;
+            const int list = win * BL_WARPS + (vlb & (BL_WARPS - 1));
+            const int key = list * g.spw + vlb / BL_WARPS;
+            const unsigned grp = __match_any_sync(FULL, valid ? key : -1 - lane);
+            const int rank = __popc(grp & ((1u << lane) - 1u));
+            const int before = valid ? myh[key] : 0;
+            __syncwarp();
+            if (valid && rank == 0) myh[key] = (uint16_t)(before + __popc(grp));
+            __syncwarp();
+            if (pass == 1 && valid) {
+                const uint32_t neg = (uint32_t)negative[base + i];
+                const int r = before + rank, k = koff[key] + r / 4, part = lpart[list];
+                const int o = k / part, q = k - o * part;
+                out[lstart[list] + ((q * 4 + o) << 2) + (r & 3)] =
+                    tile_off<T>(jl, 0) | ((uint32_t)(vlb * (BL_PITCH / 16)) << BL_BIN_SHIFT) | (neg << 31);
+            }
+        }
+        if (pass == 1) break;
+        __syncthreads();
+        for (int k = t; k < K; k += nt) {  // counts -> exclusive offsets over the warps
+            int run = 0;
+#pragma unroll
+            for (int q = 0; q < BL_BUILD_WARPS; ++q) {
+                const int c = hist[q * K + k];
+                hist[q * K + k] = (uint16_t)run;
+                run += c;
+            }
+            tot[k] = (uint16_t)run;
+        }
+        __syncthreads();
+        for (int l = t; l < nlist; l += nt) {
+            int run = 0, most = 0;
+            for (int k = l * g.spw; k < (l + 1) * g.spw; ++k) {
+                const int ng = (tot[k] + 3) / 4;
+                koff[k] = (uint16_t)run;
+                run += ng;
+                most = max(most, ng);
+            }
+            const int part = (run + 3) / 4, slow = most > part;
+            lpart[l] = part;
+            lslow[l] = slow;
+        }
+        __syncthreads();
+        if (t == 0) {
+            int run = 0;
+            for (int l = 0; l < nlist; ++l) {
+                lstart[l] = run;
+                run += 16 * lpart[l];
+            }
+        }
+        __syncthreads();
+        for (int l = t; l < nlist; l += nt)
+            lists[chunk * nlist + l] = make_int2(lstart[l] / 16, lpart[l] | (lslow[l] ? BL_SLOW : 0));
+        const int all = lstart[nlist - 1] + 16 * lpart[nlist - 1];
+        const uint32_t fill = BL_ZERO_ROW | ((uint32_t)(g.sw * g.G * (BL_PITCH / 16)) << BL_BIN_SHIFT);
+        for (int i = t; i < all + BL_SLACK; i += nt) out[i] = fill;
+        __syncthreads();
+    }
+}
+
+int tile_plan_build(rla_ctx *ctx, rla_sketch *sk) {
+    BlGeom g;
+    sk->bl_ok = false;
+    if (!bl_geometry(sk, &g)) return RLA_OK;
+    const int nlist = g.nwin * BL_WARPS, K = nlist * g.spw;
+    if (!sk->bl_words) RLA_CUDA_TRY(ctx, cudaMalloc(&sk->bl_words, sizeof(uint32_t) * (size_t)(g.nchunk * g.cap)));
+    if (!sk->bl_lists) RLA_CUDA_TRY(ctx, cudaMalloc(&sk->bl_lists, sizeof(int2) * (size_t)(g.nchunk * nlist)));
+    const size_t smem = sizeof(uint16_t) * (size_t)K * (BL_BUILD_WARPS + 2);
+    auto go = [&](auto kern) -> int {
+        RLA_CUDA_TRY(ctx, set_smem_max(kern));
+        kern<<<(unsigned)g.nchunk, BL_BUILD_WARPS * 32, smem, ctx->stream>>>(sk->bucket, sk->negative, sk->L, (int)sk->nnz, g,
+                                                                             sk->bl_words, sk->bl_lists);
+        return check_launch(ctx, "bl_build");
+    };
+    RLA_TRY(sk->p.dtype == RLA_F32 ? go(bl_build_kernel<float>) : go(bl_build_kernel<double>));
+    sk->bl_ok = true;
+    return RLA_OK;
+}
+
+// ------------------------------------------------------------------------------------
+// Compress
+// ------------------------------------------------------------------------------------
+template <class T>
+struct TileParams {
+    const T *X;
+    int64_t x_ld;  // contiguous: element (j, v) at X[j + v*x_ld]; strided: at X[v + j*x_ld]
+    int64_t L, nv, s;
+    const uint32_t *words;
+    const int2 *lists;
+    BlGeom g;
+    T *Y;
+    int64_t y_es, y_vs;
+    T alpha, beta;
+    int beta_zero;
+    T *partials;  // [slot][sw][C]
+    Split split;  // over (tile, window, chunk), chunk fastest
+};
+
+// +-x0 +-x1 +-x2 +-x3 + y, 16 bytes per lane
+__device__ __forceinline__ float4 octet_sum(float4 x0, float4 x1, float4 x2, float4 x3, uint4 w, float4 y) {
+    auto sg = [](uint32_t u) {
+        const float f = __uint_as_float((u & 0x80000000u) | 0x3f800000u);
+        return make_float2(f, f);
+    };
+    const float2 s0 = sg(w.x), s1 = sg(w.y), s2 = sg(w.z), s3 = sg(w.w);
+    float2 lo = __fmul2_rn(make_float2(x0.x, x0.y), s0), hi = __fmul2_rn(make_float2(x0.z, x0.w), s0);
+    lo = __ffma2_rn(make_float2(x1.x, x1.y), s1, lo);
+    hi = __ffma2_rn(make_float2(x1.z, x1.w), s1, hi);
+    lo = __ffma2_rn(make_float2(x2.x, x2.y), s2, lo);
+    hi = __ffma2_rn(make_float2(x2.z, x2.w), s2, hi);
+    lo = __ffma2_rn(make_float2(x3.x, x3.y), s3, lo);
+    hi = __ffma2_rn(make_float2(x3.z, x3.w), s3, hi);
+    lo = __fadd2_rn(lo, make_float2(y.x, y.y));
+    hi = __fadd2_rn(hi, make_float2(y.z, y.w));
+    return make_float4(lo.x, lo.y, hi.x, hi.y);
+}
+__device__ __forceinline__ double2 octet_sum(double2 x0, double2 x1, double2 x2, double2 x3, uint4 w, double2 y) {
+    auto sg = [](double x, uint32_t u) {
+        return __longlong_as_double(__double_as_longlong(x) ^ ((long long)(u & 0x80000000u) << 32));
+    };
+    const double a = ((sg(x0.x, w.x) + sg(x1.x, w.y)) + sg(x2.x, w.z)) + sg(x3.x, w.w);
+    const double b = ((sg(x0.y, w.x) + sg(x1.y, w.y)) + sg(x2.y, w.z)) + sg(x3.y, w.w);
+    return make_double2(y.x + a, y.y + b);
+}
+
+// Loads of the next unit, issued where they stand: the compiler would move plain loads down to
+// their use, behind the current unit's sums, and expose their latency.
+__device__ __forceinline__ float4 ld_ahead(const float4 *a) {
+    float4 v;
+    asm volatile("ld.global.nc.L1::no_allocate.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(a));
+    return v;
+}
+__device__ __forceinline__ double2 ld_ahead(const double2 *a) {
+    double2 v;
+    asm volatile("ld.global.nc.L1::no_allocate.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(a));
+    return v;
+}
+__device__ __forceinline__ float ld_ahead(const float *a) {
+    float v;
+    asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(v) : "l"(a));
+    return v;
+}
+__device__ __forceinline__ double ld_ahead(const double *a) {
+    double v;
+    asm volatile("ld.global.nc.f64 %0, [%1];" : "=d"(v) : "l"(a));
+    return v;
+}
+
+// How a unit's elements are read: contiguous vectors with 16-byte aligned starts, contiguous
+// vectors at any alignment (16-byte loads of the aligned windows, rows shifted), strided vectors
+// with 16-byte aligned rows, strided vectors at any alignment.
+enum { TILE_CONTIG = 0, TILE_SHIFT = 1, TILE_ROWS = 2, TILE_ROWS_ANY = 3 };
+
+template <class T, int MODE>
+__global__ void __launch_bounds__(BL_WARPS * 32, 1) tile_compress_kernel(TileParams<T> p) {
+    using V = typename TileVec<T>::type;
+    constexpr int VR = TileCfg<T>::VR, C = TileCfg<T>::C, PE = BL_PITCH / (int)sizeof(T);
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    unsigned char *bin_raw = smem_raw + BL_TILE_BYTES;
+    const T *bins = reinterpret_cast<const T *>(bin_raw);
+    const int t = threadIdx.x, lane = t & 31, wp = t >> 5, l8 = lane & 7;
+    const uint32_t lane16 = (uint32_t)l8 << 4;
+    const int64_t nchunk = p.g.nchunk;
+    const int64_t u0 = p.split.start(blockIdx.x), u1 = p.split.start(blockIdx.x + 1);
+    if (u0 >= u1) return;
+    auto zero_bins = [&]() {
+        for (int i = t; i < (p.g.sw * p.g.G + 1) * (BL_PITCH / 16); i += BL_WARPS * 32) reinterpret_cast<V *>(bin_raw)[i] = V{};
+    };
+    zero_bins();
+    if (t < 8) reinterpret_cast<V *>(smem_raw + BL_ZERO_ROW)[t] = V{};
+    // Contiguous vectors: a thread's column of the tile and its first row; a warp load covers 8
+    // lanes x VR rows of 4 columns, the thread's BL_PF loads consecutive blocks of 8*VR rows.
+    // Strided vectors: a warp load covers 4 rows (16-byte loads) or 32/C rows (element loads).
+    // The swizzle repeats every 8*VR rows, so a thread's shared-memory addresses are one base
+    // per row residue plus compile-time offsets.
+    constexpr int CQ = C / 4, RW = 32 / C;
+    const int my_c = (wp % CQ) * 4 + (lane >> 3), my_r = (wp / CQ) * BL_PF * 8 * VR + l8 * VR;
+    const bool has_tail = MODE == TILE_SHIFT && my_r + BL_PF * 8 * VR == BL_R + 7 * VR;
+    V pf[BL_PF], tail{};
+    int shift = 0;  // rows by which the loaded 16-byte windows start before the thread's rows
+    auto load_unit = [&](int64_t tile, int64_t chunk) {
+        const int64_t j0 = chunk * BL_R, v0 = tile * C;
+        if constexpr (MODE <= TILE_SHIFT) {
+            const T *x = p.X + (v0 + my_c) * p.x_ld + j0;
+            if (MODE == TILE_SHIFT) shift = (int)((reinterpret_cast<uintptr_t>(x) / sizeof(T)) & (VR - 1));
+            // every window of the unit inside its vector: plain loads
+            if (v0 + C <= p.nv && j0 + BL_R + (MODE == TILE_SHIFT ? VR : 0) <= p.L && (MODE == TILE_CONTIG || j0 > 0)) {
+                const V *xv = reinterpret_cast<const V *>(x + my_r - shift);
+#pragma unroll
+                for (int k = 0; k < BL_PF; ++k) pf[k] = ld_ahead(xv + k * 8);
+                if (has_tail) tail = ld_ahead(reinterpret_cast<const V *>(x + BL_R - shift));
+                return;
+            }
+            const int left = v0 + my_c < p.nv ? (int)min((int64_t)BL_R, p.L - j0) : 0;
+            auto load = [&](int r) {
+                V y{};
+                T *ye = reinterpret_cast<T *>(&y);
+#pragma unroll
+                for (int e = 0; e < VR; ++e)
+                    if (r + e >= 0 && r + e < left) ye[e] = ld_ahead(x + r + e);
+                return y;
+            };
+#pragma unroll
+            for (int k = 0; k < BL_PF; ++k) pf[k] = load(my_r + k * 8 * VR - shift);
+            if (has_tail) tail = load(BL_R - shift);
+        } else if constexpr (MODE == TILE_ROWS) {
+            const int r0 = wp * 4 + (lane >> 3);
+            const int64_t v = v0 + l8 * VR;
+            const T *x = p.X + v + (j0 + r0) * p.x_ld;
+            const int64_t step = 64 * p.x_ld;
+            const int left = (int)min((int64_t)BL_R, p.L - j0) - r0, nv = (int)min((int64_t)VR, p.nv - v);
+            if (nv == VR) {
+#pragma unroll
+                for (int k = 0; k < BL_PF; ++k) pf[k] = k * 64 < left ? ld_ahead(reinterpret_cast<const V *>(x + k * step)) : V{};
+            } else {
+#pragma unroll
+                for (int k = 0; k < BL_PF; ++k) {
+                    pf[k] = V{};
+                    T *ye = reinterpret_cast<T *>(&pf[k]);
+#pragma unroll
+                    for (int e = 0; e < VR; ++e)
+                        if (k * 64 < left && e < nv) ye[e] = ld_ahead(x + k * step + e);
+                }
+            }
+        } else {
+            const int r0 = wp * RW + lane / C;
+            const T *x = p.X + v0 + lane % C + (j0 + r0) * p.x_ld;
+            const int64_t step = BL_WARPS * RW * p.x_ld;
+            const int left = v0 + lane % C < p.nv ? (int)min((int64_t)BL_R, p.L - j0) - r0 : 0;
+            T *d = reinterpret_cast<T *>(pf);
+#pragma unroll
+            for (int k = 0; k < BL_PF * VR; ++k) {
+                d[k] = k * BL_WARPS * RW < left ? ld_ahead(x) : T(0);
+                x += step;
+            }
+        }
+    };
+    auto store_unit = [&]() {
+        if constexpr (MODE <= TILE_SHIFT) {
+#pragma unroll
+            for (int i = 0; i < VR; ++i) {
+                const int r = my_r - shift + i;  // negative only in the first block
+                unsigned char *d = smem_raw + r * 128 + (((my_c / VR) ^ tile_swz<T>(r & (8 * VR - 1))) << 4) +
+                                   (my_c % VR) * sizeof(T);
+#pragma unroll
+                for (int k = 0; k < BL_PF; ++k)
+                    if (MODE == TILE_CONTIG || k > 0 || r >= 0)
+                        *reinterpret_cast<T *>(d + k * 8 * VR * 128) = reinterpret_cast<const T *>(&pf[k])[i];
+                if (i < VR - 1 && has_tail && i < shift)
+                    *reinterpret_cast<T *>(smem_raw + tile_off<T>(BL_R - shift + i, my_c)) = reinterpret_cast<const T *>(&tail)[i];
+            }
+        } else if constexpr (MODE == TILE_ROWS) {
+            unsigned char *d = smem_raw + tile_off<T>(wp * 4 + (lane >> 3), l8 * VR);
+#pragma unroll
+            for (int k = 0; k < BL_PF; ++k) *reinterpret_cast<V *>(d + k * 64 * 128) = pf[k];
+        } else {
+            constexpr int M = sizeof(T) == 4 ? 2 : 1;  // loads after which the swizzle repeats
+#pragma unroll
+            for (int m = 0; m < M; ++m) {
+                unsigned char *d = smem_raw + tile_off<T>((m * BL_WARPS + wp) * RW + lane / C, lane % C);
+#pragma unroll
+                for (int k = m; k < BL_PF * VR; k += M)
+                    *reinterpret_cast<T *>(d + (k - m) * BL_WARPS * RW * 128) = reinterpret_cast<const T *>(pf)[k];
+            }
+        }
+    };
+    auto row = [&](uint32_t w) { return *reinterpret_cast<const V *>(smem_raw + ((w & BL_ROW_MASK) ^ lane16)); };
+    auto bins_of = [&](uint32_t w) {
+        return reinterpret_cast<V *>(bin_raw + ((w >> (BL_BIN_SHIFT - 4)) & BL_BIN_MASK) + lane16);
+    };
+    int64_t tile = u0 / nchunk / p.g.nwin, chunk = u0 % nchunk;
+    int win = (int)(u0 / nchunk % p.g.nwin);
+    load_unit(tile, chunk);
+    int2 li_next = __ldg(p.lists + (chunk * p.g.nwin + win) * BL_WARPS + wp);
+    for (int64_t u = u0; u < u1; ++u) {
+        const int2 li = li_next;
+        const int nq = li.y & (BL_SLOW - 1);
+        const uint4 *lp = reinterpret_cast<const uint4 *>(p.words + chunk * p.g.cap) + li.x * 4 + (lane >> 3);
+        uint4 w[BL_AHEAD];
+#pragma unroll
+        for (int i = 0; i < BL_AHEAD; ++i) w[i] = __ldg(lp + 4 * i);
+        store_unit();
+        __syncthreads();
+        const int64_t tile_u = tile, chunk_u = chunk;
+        const int win_u = win;
+        if (u + 1 < u1) {
+            if (++chunk == nchunk) {
+                chunk = 0;
+                if (++win == p.g.nwin) {
+                    win = 0;
+                    ++tile;
+                }
+            }
+            load_unit(tile, chunk);
+            li_next = __ldg(p.lists + (chunk * p.g.nwin + win) * BL_WARPS + wp);
+        }
+        // ---- the octet's groups; the rows of the next group are read before the current one
+        // is added, so that the bin update does not hold them up ----
+        if (!(li.y & BL_SLOW)) {
+            V x0 = row(w[0].x), x1 = row(w[0].y), x2 = row(w[0].z), x3 = row(w[0].w);
+            // words are read BL_AHEAD steps ahead (past the list: the next one's or filling, not
+            // added), so that the first ones read after the next unit's elements, whose
+            // arrival they would wait for, are not needed before those have come
+            for (int q = 0; q < nq; q += BL_AHEAD) {
+                lp += 4 * BL_AHEAD;
+#pragma unroll
+                for (int i = 0; i < BL_AHEAD; ++i) {
+                    if (q + i >= nq) break;
+                    const uint4 wc = w[i], wn = w[(i + 1) % BL_AHEAD];
+                    V *bp = bins_of(wc.x);
+                    V y = *bp;
+                    y = octet_sum(x0, x1, x2, x3, wc, y);
+                    x0 = row(wn.x);
+                    x1 = row(wn.y);
+                    x2 = row(wn.z);
+                    x3 = row(wn.w);
+                    *bp = y;
+                    w[i] = __ldg(lp + 4 * i);
+                    __syncwarp();  // orders these bin updates before the next step's
+                }
+            }
+        } else {  // the octets update the bins one after another
+            for (int q = 0; q < nq; ++q, lp += 4) {
+                const uint4 w = __ldg(lp);
+                for (int o = 0; o < 4; ++o) {
+                    if ((lane >> 3) == o) {
+                        V *bp = bins_of(w.x);
+                        *bp = octet_sum(row(w.x), row(w.y), row(w.z), row(w.w), w, *bp);
+                    }
+                    __syncwarp();
+                }
+            }
+        }
+        __syncthreads();
+        if (chunk_u + 1 < nchunk && u + 1 < u1) continue;
+        // ---- last chunk of this (tile, window) in the CTA's range: write the bins ----
+        const int64_t gbeg = u - chunk_u, v0 = tile_u * C;
+        const int64_t lo = (int64_t)win_u * p.g.sw;
+        const int cnt = (int)min((int64_t)p.g.sw, p.s - lo);
+        const int nc = (int)min((int64_t)C, p.nv - v0);
+        auto bin = [&](int b, int c) {
+            T a = bins[b * PE + c];
+            for (int r = 1; r < p.g.G; ++r) a += bins[(r * p.g.sw + b) * PE + c];
+            return a;
+        };
+        auto put = [&](int b, int c) {
+            T *yp = p.Y + (lo + b) * p.y_es + (v0 + c) * p.y_vs;
+            T r = p.alpha * bin(b, c);
+            if (!p.beta_zero) r += p.beta * *yp;
+            *yp = r;
+        };
+        if (u0 <= gbeg && gbeg + nchunk <= u1) {
+            if (p.y_es == 1) {
+                for (int c = wp; c < nc; c += BL_WARPS)
+                    for (int b = lane; b < cnt; b += 32) put(b, c);
+            } else {
+                for (int i = t; i < cnt * C; i += BL_WARPS * 32)
+                    if (i % C < nc) put(i / C, i % C);
+            }
+        } else {
+            T *part = p.partials + (int64_t)p.split.slot(blockIdx.x, gbeg) * p.g.sw * C;
+            for (int i = t; i < cnt * C; i += BL_WARPS * 32) part[i] = bin(i / C, i % C);
+        }
+        __syncthreads();
+        if (u + 1 < u1) zero_bins();
+    }
+}
+
+// Adds the partial bins of every (tile, window) shared by several CTAs, in CTA order; one CTA
+// per 32 buckets.
+template <class T>
+__global__ void __launch_bounds__(256) tile_reduce_kernel(TileParams<T> p) {
+    constexpr int C = TileCfg<T>::C;
+    __shared__ T tile[32][C + 1];
+    const int64_t grp = blockIdx.x, gbeg = grp * p.g.nchunk;
+    const int gf = p.split.owner(gbeg), gl = p.split.owner(gbeg + p.g.nchunk - 1);
+    if (gf == gl) return;  // written by its only CTA
+    const int64_t lo = (grp % p.g.nwin) * p.g.sw, v0 = (grp / p.g.nwin) * C;
+    const int cnt = (int)min((int64_t)p.g.sw, p.s - lo);
+    const int b0 = blockIdx.y * 32;
+    if (b0 >= cnt) return;
+    const int64_t ps = (int64_t)p.g.sw * C;
+    const T *p0 = p.partials + p.split.slot(gf, gbeg) * ps + b0 * C;
+#pragma unroll
+    for (int q = 0; q < 32 * C / 256; ++q) {
+        const int i = threadIdx.x + 256 * q;
+        T a = T(0);
+        if (b0 + i / C < cnt) {
+            a = p0[i];
+#pragma unroll 4
+            for (int gg = gf + 1; gg <= gl; ++gg) a += p.partials[2 * gg * ps + b0 * C + i];
+        }
+        tile[i / C][i % C] = a;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < 32 * C / 256; ++q) {
+        const int i = threadIdx.x + 256 * q;
+        const int b = p.y_es == 1 ? i % 32 : i / C, c = p.y_es == 1 ? i / 32 : i % C;
+        if (b0 + b >= cnt || v0 + c >= p.nv) continue;
+        T *yp = p.Y + (lo + b0 + b) * p.y_es + (v0 + c) * p.y_vs;
+        T r = p.alpha * tile[b][c];
+        if (!p.beta_zero) r += p.beta * *yp;
+        *yp = r;
+    }
+}
+
+template <class T>
+int tile_compress(rla_ctx *ctx, const rla_sketch *sk, const T *X, int64_t x_es, int64_t x_vs, int64_t nv, T *Y,
+                  int64_t y_es, int64_t y_vs, T alpha, T beta, bool beta_zero) {
+    constexpr int VR = TileCfg<T>::VR, C = TileCfg<T>::C;
+    BlGeom g;
+    if (!sk->bl_ok || !bl_geometry(sk, &g)) return set_error(ctx, RLA_E_UNSUPPORTED, "no bucket lists for this sketch");
+    const int64_t groups = ceil_div(nv, C) * g.nwin, units = groups * g.nchunk;
+    const int W = (int)std::min<int64_t>(ctx->sm_count, units);
+    void *part = nullptr;
+    const bool shared = W > 1 && g.nchunk > 1;
+    if (shared) RLA_TRY(scratch_get(ctx, (size_t)(2 * W) * g.sw * C * sizeof(T), &part));
+    const bool contig = x_es == 1;
+    TileParams<T> p{X, contig ? x_vs : x_es, sk->L, nv, sk->s, sk->bl_words, sk->bl_lists, g, Y, y_es, y_vs,
+                    alpha, beta, beta_zero, (T *)part, Split::make(units, W)};
+    const size_t smem = (size_t)BL_TILE_BYTES + (size_t)(g.sw * g.G + 1) * BL_PITCH;
+    const bool aligned = (nv == 1 && contig) || p.x_ld % VR == 0;
+    const bool vec = aligned && (uintptr_t)X % 16 == 0;
+    auto go = [&](auto kern) -> int {
+        RLA_CUDA_TRY(ctx, set_smem_max(kern));
+        kern<<<W, BL_WARPS * 32, smem, ctx->stream>>>(p);
+        return check_launch(ctx, "tile_compress");
+    };
+    if (contig) RLA_TRY(vec ? go(tile_compress_kernel<T, TILE_CONTIG>) : go(tile_compress_kernel<T, TILE_SHIFT>));
+    else RLA_TRY(vec ? go(tile_compress_kernel<T, TILE_ROWS>) : go(tile_compress_kernel<T, TILE_ROWS_ANY>));
+    if (!shared) return RLA_OK;
+    tile_reduce_kernel<T><<<dim3((unsigned)groups, ceil_div_i(g.sw, 32)), 256, 0, ctx->stream>>>(p);
+    return check_launch(ctx, "tile_reduce");
+}
+
+template int tile_compress<float>(rla_ctx *, const rla_sketch *, const float *, int64_t, int64_t, int64_t, float *, int64_t,
+                                  int64_t, float, float, bool);
+template int tile_compress<double>(rla_ctx *, const rla_sketch *, const double *, int64_t, int64_t, int64_t, double *,
+                                   int64_t, int64_t, double, double, bool);
+
+}  // namespace rla
