@@ -43,6 +43,12 @@ template <class T>
 int tile_compress(rla_ctx *ctx, const rla_sketch *sk, const T *X, int64_t x_es, int64_t x_vs, int64_t nv, T *Y,
                   int64_t y_es, int64_t y_vs, T alpha, T beta, bool beta_zero);
 
+// SparseSign / CountSketch expand on tiles of vectors (rla_sparse_lift.cu); *taken = false when
+// the compression dimension does not fit its staged tile.
+template <class T>
+int sparse_lift(rla_ctx *ctx, const rla_sketch *sk, const T *X, int64_t x_es, int64_t x_vs, int64_t nv, T *Y,
+                int64_t y_es, int64_t y_vs, T alpha, T beta, bool beta_zero, bool *taken);
+
 // SRHT / FJLT (rla_wht.cu)
 // Builds sk->sign_tl (per-thread sign masks of the fused compress kernel) from sk->signbits.
 int build_srht_sign_table(rla_ctx *ctx, rla_sketch *sk);

@@ -811,6 +811,9 @@ template <class T>
 int sparse_expand(rla_ctx *ctx, const rla_sketch *sk, const T *X, int64_t x_es, int64_t x_vs, int64_t nv, T *Y,
                   int64_t y_es, int64_t y_vs, double alpha, double beta) {
     if (nv == 0) return RLA_OK;
+    bool taken = false;
+    RLA_TRY(sparse_lift<T>(ctx, sk, X, x_es, x_vs, nv, Y, y_es, y_vs, (T)(alpha * sk->scale), (T)beta, beta == 0.0, &taken));
+    if (taken) return RLA_OK;
     const int64_t L = sk->L;
     const int out_contig = y_es == 1;
     const int64_t fast = out_contig ? L : nv, slow = out_contig ? nv : L;

@@ -1,0 +1,273 @@
+// rla_sparse_lift.cu -- SparseSign / CountSketch expand (S'*Y, A*S' ...) on tiles of vectors.
+//
+// Y(j, v) = alpha * sum_e sign(j, e) * X(bucket(j, e), v) + beta * Y(j, v), j < L.  The short
+// operand X (s rows) is staged once per tile of vectors in shared memory, one row per bucket, so
+// that LPE lanes read an entry's values with 16-byte accesses: one conflict-free wavefront per 128
+// bytes.  Each warp takes 32 long indices at a time: it packs their entries into 16-bit words,
+// sums the nnz rows of four (32/LPE) long indices per step in registers, and turns the 32 x C
+// block of results through shared memory into 16-byte column stores.  Bound by the row reads
+// (nnz wavefronts per 128 bytes of output; shared-memory pipe 68 % busy, the output's HBM
+// traffic alone would take 32 us): 131072 x 200 Float64, s = 1000, nnz = 8 in 122 us, 436 us with
+// a thread per output element.  The entry loop is unrolled for the usual nnz (154 us without).
+//
+// LPE = 8 / 4 / 2 lanes per entry (rows of 128 / 64 / 32 bytes) for s up to 1158 / 2084 / 3473:
+// the widest row that fits; above, the thread-per-element kernel of rla_sparse.cu.
+#include "rla_internal.cuh"
+#include "rla_kernels.cuh"
+
+namespace rla {
+
+constexpr int LIFT_WARPS = 16, LIFT_MAX_NNZ = 32;
+
+template <class T, int LPE>
+struct LiftCfg {
+    static constexpr int VR = 16 / (int)sizeof(T);  // elements per 16 bytes
+    static constexpr int C = LPE * VR;              // vectors per tile
+    static constexpr int PITCH = LPE * 16 + 16;     // bytes per staged row: 16-byte column writes conflict-free
+    static constexpr int JS = 32 / LPE;             // long indices per step
+    static constexpr int OUT = 32 * LPE * 16;       // bytes of a warp's result block
+};
+
+template <class T>
+struct LiftParams {
+    const T *X;
+    int64_t x_es, x_vs, L, nv, s;
+    const int32_t *bucket;
+    const uint8_t *negative;
+    int nnz, wpj;  // wpj: 16-bit words kept per long index (nnz rounded up to even)
+    T *Y;
+    int64_t y_es, y_vs;
+    T alpha, beta;
+    int beta_zero;
+    int64_t nblk;  // blocks of 32 long indices
+    Split split;   // over (tile, block of LIFT_WARPS * 32 long indices)
+};
+
+__device__ __forceinline__ void lift_add(float4 &a, float4 x, uint32_t sign) {
+    const float s = __uint_as_float(sign | 0x3f800000u);
+    const float2 s2 = make_float2(s, s);
+    const float2 lo = __ffma2_rn(make_float2(x.x, x.y), s2, make_float2(a.x, a.y));
+    const float2 hi = __ffma2_rn(make_float2(x.z, x.w), s2, make_float2(a.z, a.w));
+    a = make_float4(lo.x, lo.y, hi.x, hi.y);
+}
+__device__ __forceinline__ void lift_add(double2 &a, double2 x, uint32_t sign) {
+    const long long m = (long long)sign << 32;
+    a.x += __longlong_as_double(__double_as_longlong(x.x) ^ m);
+    a.y += __longlong_as_double(__double_as_longlong(x.y) ^ m);
+}
+
+// Slot of 16 bytes q of row j in a warp's result block: the column reads below (8 lanes along
+// j in steps of VR, 4 columns) then hit distinct banks for LPE = 8.
+template <class T, int LPE>
+__device__ __forceinline__ int lift_slot(int j, int q) {
+    constexpr int VR = LiftCfg<T, LPE>::VR;
+    return q ^ ((j / VR + (8 / VR) * (j % VR)) & (LPE - 1));
+}
+
+// NNZ: entries per long index when it is a compile-time 1, 2, 4 or 8, else 0 (p.nnz).
+template <class T, int LPE, int NNZ>
+__global__ void __launch_bounds__(LIFT_WARPS * 32, 1) lift_kernel(LiftParams<T> p) {
+    using Cfg = LiftCfg<T, LPE>;
+    using V = std::conditional_t<sizeof(T) == 4, float4, double2>;
+    constexpr int VR = Cfg::VR, C = Cfg::C, JS = Cfg::JS;
+    const int nnz = NNZ ? NNZ : p.nnz, wpj = NNZ ? (NNZ + 1) / 2 * 2 : p.wpj;
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    const int t = threadIdx.x, lane = t & 31, wp = t >> 5;
+    unsigned char *out = smem_raw + wp * Cfg::OUT;
+    uint16_t *words = reinterpret_cast<uint16_t *>(smem_raw + LIFT_WARPS * Cfg::OUT) + wp * 32 * wpj;
+    unsigned char *xs = smem_raw + LIFT_WARPS * (Cfg::OUT + 32 * wpj * 2);
+    const int64_t u0 = p.split.start(blockIdx.x), u1 = p.split.start(blockIdx.x + 1);
+    const int64_t nj = (p.nblk + LIFT_WARPS - 1) / LIFT_WARPS;
+    int64_t have = -1;
+    for (int64_t u = u0; u < u1; ++u) {
+        const int64_t tile = u / nj, v0 = tile * C;
+        const int nc = (int)min((int64_t)C, p.nv - v0);
+        if (tile != have) {  // stage X(:, v0 .. v0 + C): row b at b * PITCH
+            __syncthreads();
+            have = tile;
+            if (p.x_es == 1) {
+                // lanes along b; VR vectors per thread make one 16-byte store
+                const int ss = (int)p.s;
+                for (int i = t; i < ss * LPE; i += LIFT_WARPS * 32) {
+                    const int q = i / ss, b = i - q * ss;
+                    V y{};
+                    T *ye = reinterpret_cast<T *>(&y);
+#pragma unroll
+                    for (int e = 0; e < VR; ++e)
+                        if (q * VR + e < nc) ye[e] = __ldg(p.X + b + (v0 + q * VR + e) * p.x_vs);
+                    *reinterpret_cast<V *>(xs + b * Cfg::PITCH + q * 16) = y;
+                }
+            } else {
+                for (int i = t; i < (int)p.s * C; i += LIFT_WARPS * 32) {
+                    const int b = i / C, c = i % C;
+                    *reinterpret_cast<T *>(xs + b * Cfg::PITCH + c * sizeof(T)) =
+                        c < nc ? __ldg(p.X + b * p.x_es + (v0 + c) * p.x_vs) : T(0);
+                }
+            }
+            __syncthreads();
+        }
+        const int64_t blk = (u - tile * nj) * LIFT_WARPS + wp;
+        if (blk >= p.nblk) continue;  // warp-uniform
+        const int64_t j0 = blk * 32;
+        const int cnt = (int)min((int64_t)32, p.L - j0);
+        // ---- the block's entries: bucket | sign << 15, lane = long index when nnz is known ----
+        if constexpr (NNZ > 0) {
+            if (lane < cnt) {
+                const int32_t *bp = p.bucket + (j0 + lane) * NNZ;
+                const uint8_t *np = p.negative + (j0 + lane) * NNZ;
+                int32_t b[NNZ];
+                uint32_t n[NNZ];
+                if constexpr (NNZ == 8) {
+                    const int4 b0 = __ldg(reinterpret_cast<const int4 *>(bp)), b1 = __ldg(reinterpret_cast<const int4 *>(bp) + 1);
+                    const uint2 m = __ldg(reinterpret_cast<const uint2 *>(np));
+                    const int32_t bb[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) {
+                        b[e] = bb[e];
+                        n[e] = ((e < 4 ? m.x : m.y) >> (8 * (e & 3))) & 1u;
+                    }
+                } else {
+#pragma unroll
+                    for (int e = 0; e < NNZ; ++e) {
+                        b[e] = __ldg(bp + e);
+                        n[e] = __ldg(np + e);
+                    }
+                }
+                uint32_t *wo = reinterpret_cast<uint32_t *>(words + lane * wpj);
+#pragma unroll
+                for (int e = 0; e < NNZ; e += 2) {
+                    uint32_t w = (uint32_t)b[e] | (n[e] << 15);
+                    if (e + 1 < NNZ) w |= ((uint32_t)b[(e + 1) % NNZ] << 16) | (n[(e + 1) % NNZ] << 31);
+                    wo[e / 2] = w;
+                }
+            }
+        } else {
+            for (int i = lane; i < cnt * nnz; i += 32) {
+                const int jl = i / nnz;
+                words[jl * wpj + i - jl * nnz] =
+                    (uint16_t)((uint32_t)__ldg(p.bucket + j0 * nnz + i) | ((uint32_t)__ldg(p.negative + j0 * nnz + i) << 15));
+            }
+        }
+        __syncwarp();
+        // ---- sums of JS long indices per step ----
+        const int l = lane % LPE, g = lane / LPE;
+        const unsigned char *xl = xs + l * 16;
+        auto entry = [&](V &a, uint32_t b, uint32_t sign) {
+            lift_add(a, *reinterpret_cast<const V *>(xl + b * Cfg::PITCH), sign);
+        };
+#pragma unroll 2
+        for (int q = 0; q < LPE; ++q) {
+            const int jl = q * JS + g;
+            V a{};
+            if (jl < cnt) {
+                const uint16_t *wj = words + jl * wpj;
+                auto pair = [&](uint32_t w) {
+                    entry(a, w & 0x7fffu, (w << 16) & 0x80000000u);
+                    entry(a, (w >> 16) & 0x7fffu, w & 0x80000000u);
+                };
+                if constexpr (NNZ == 8) {
+                    const uint4 w = *reinterpret_cast<const uint4 *>(wj);
+                    pair(w.x);
+                    pair(w.y);
+                    pair(w.z);
+                    pair(w.w);
+                } else {
+                    const uint32_t *w2 = reinterpret_cast<const uint32_t *>(wj);
+                    int e = 0;
+#pragma unroll
+                    for (; e + 2 <= nnz; e += 2) pair(w2[e >> 1]);
+                    if (e < nnz) {
+                        const uint32_t w = wj[e];
+                        entry(a, w & 0x7fffu, (w << 16) & 0x80000000u);
+                    }
+                }
+            }
+            *reinterpret_cast<V *>(out + jl * (LPE * 16) + lift_slot<T, LPE>(jl, l) * 16) = a;
+        }
+        __syncwarp();
+        // ---- write the 32 x C block ----
+        auto get = [&](int j, int c) {
+            return *reinterpret_cast<const T *>(out + j * (LPE * 16) + lift_slot<T, LPE>(j, c / VR) * 16 + (c % VR) * sizeof(T));
+        };
+        auto put = [&](int j, int c) {
+            T *yp = p.Y + (j0 + j) * p.y_es + (v0 + c) * p.y_vs;
+            T r = p.alpha * get(j, c);
+            if (!p.beta_zero) r += p.beta * *yp;
+            *yp = r;
+        };
+        if (p.y_es == 1) {
+            const bool vec = cnt == 32 && p.beta_zero && p.y_vs % VR == 0 && reinterpret_cast<uintptr_t>(p.Y) % 16 == 0;
+            if (vec) {
+                // 8 lanes along j, VR rows each, of 4 columns per pass
+                constexpr int RB = 32 / (8 * VR);
+#pragma unroll
+                for (int i = 0; i < RB * (C / 4); ++i) {
+                    const int c = (i / RB) * 4 + (lane >> 3), j = ((i % RB) * 8 + (lane & 7)) * VR;
+                    V y;
+                    T *ye = reinterpret_cast<T *>(&y);
+#pragma unroll
+                    for (int e = 0; e < VR; ++e) ye[e] = p.alpha * get(j + e, c);
+                    if (c < nc) *reinterpret_cast<V *>(p.Y + j0 + j + (v0 + c) * p.y_vs) = y;
+                }
+            } else {
+                for (int c = 0; c < nc; ++c)
+                    if (lane < cnt) put(lane, c);
+            }
+        } else {
+            for (int i = lane; i < cnt * C; i += 32)
+                if (i % C < nc) put(i / C, i % C);
+        }
+        __syncwarp();
+    }
+}
+
+// Lanes per entry whose staged rows fit next to the warps' blocks, 0 when none do.
+template <class T>
+static int lift_lanes(const rla_ctx *ctx, const rla_sketch *sk, size_t *smem) {
+    const int wpj = ((int)sk->nnz + 1) / 2 * 2;
+    if (sk->nnz > LIFT_MAX_NNZ || sk->s >= 32768) return 0;
+    for (int lpe = 8; lpe >= 2; lpe /= 2) {
+        *smem = (size_t)LIFT_WARPS * (32 * lpe * 16 + 32 * wpj * 2) + (size_t)sk->s * (lpe * 16 + 16);
+        if (*smem <= (size_t)ctx->smem_optin - 1024) return lpe;
+    }
+    return 0;
+}
+
+template <class T>
+int sparse_lift(rla_ctx *ctx, const rla_sketch *sk, const T *X, int64_t x_es, int64_t x_vs, int64_t nv, T *Y,
+                int64_t y_es, int64_t y_vs, T alpha, T beta, bool beta_zero, bool *taken) {
+    size_t smem = 0;
+    const int lpe = lift_lanes<T>(ctx, sk, &smem);
+    *taken = lpe != 0;
+    if (!lpe) return RLA_OK;
+    const int64_t C = lpe * (16 / (int64_t)sizeof(T)), nblk = ceil_div(sk->L, 32);
+    const int64_t units = ceil_div(nv, C) * ceil_div(nblk, LIFT_WARPS);
+    const int W = (int)std::min<int64_t>(ctx->sm_count, units);
+    LiftParams<T> p{X, x_es, x_vs, sk->L, nv, sk->s, sk->bucket, sk->negative, (int)sk->nnz, ((int)sk->nnz + 1) / 2 * 2,
+                    Y, y_es, y_vs, alpha, beta, beta_zero, nblk, Split::make(units, W)};
+    auto go = [&](auto kern) -> int {
+        RLA_CUDA_TRY(ctx, set_smem_max(kern));
+        kern<<<W, LIFT_WARPS * 32, smem, ctx->stream>>>(p);
+        return check_launch(ctx, "sparse_lift");
+    };
+    auto by_nnz = [&](auto lanes) -> int {
+        constexpr int N = decltype(lanes)::value;
+        switch (sk->nnz) {
+            case 1: return go(lift_kernel<T, N, 1>);
+            case 2: return go(lift_kernel<T, N, 2>);
+            case 4: return go(lift_kernel<T, N, 4>);
+            case 8: return go(lift_kernel<T, N, 8>);
+            default: return go(lift_kernel<T, N, 0>);
+        }
+    };
+    if (lpe == 8) return by_nnz(std::integral_constant<int, 8>());
+    if (lpe == 4) return by_nnz(std::integral_constant<int, 4>());
+    return by_nnz(std::integral_constant<int, 2>());
+}
+
+template int sparse_lift<float>(rla_ctx *, const rla_sketch *, const float *, int64_t, int64_t, int64_t, float *, int64_t,
+                                int64_t, float, float, bool, bool *);
+template int sparse_lift<double>(rla_ctx *, const rla_sketch *, const double *, int64_t, int64_t, int64_t, double *,
+                                 int64_t, int64_t, double, double, bool, bool *);
+
+}  // namespace rla
