@@ -67,6 +67,14 @@ int counters_get(rla_ctx *ctx, size_t n, int **out) {
     return RLA_OK;
 }
 
+// Whether this thread has raised the kernel's shared-memory limit on the device; `set` records it.
+bool smem_max_raised(const void *kern, int device, bool set) {
+    static thread_local std::vector<std::pair<const void *, int>> raised;
+    const std::pair<const void *, int> key(kern, device);
+    if (set) raised.push_back(key);
+    return set || std::find(raised.begin(), raised.end(), key) != raised.end();
+}
+
 }  // namespace rla
 
 using namespace rla;

@@ -82,12 +82,21 @@ int check_launch(rla_ctx *ctx, const char *what);
 // thread, so set_smem_max always raises it to the most the kernel can take (never to a
 // per-call size another thread could lower before its own launch).
 extern int g_smem_optin;
+// The two driver calls cost about 3 us of a 20 us call, so a thread remembers the (kernel, device)
+// pairs it has raised.
+bool smem_max_raised(const void *kern, int device, bool set);
 template <class K>
 inline cudaError_t set_smem_max(K kern) {
-    cudaFuncAttributes a;
-    cudaError_t e = cudaFuncGetAttributes(&a, reinterpret_cast<const void *>(kern));
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
-    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, g_smem_optin - (int)a.sharedSizeBytes);
+    if (smem_max_raised(reinterpret_cast<const void *>(kern), dev, false)) return cudaSuccess;
+    cudaFuncAttributes a;
+    e = cudaFuncGetAttributes(&a, reinterpret_cast<const void *>(kern));
+    if (e != cudaSuccess) return e;
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, g_smem_optin - (int)a.sharedSizeBytes);
+    if (e == cudaSuccess) smem_max_raised(reinterpret_cast<const void *>(kern), dev, true);
+    return e;
 }
 // Stream-ordered allocation from the context's pool (memory stays mapped between calls, so
 // repeated calls of the same size do not remap device memory).
@@ -304,7 +313,7 @@ struct rla_sketch {
     uint32_t *signbits = nullptr;  // [ceil(N/32)] bit r = 1 means +1
     uint4 *sign_tl = nullptr;      // fused compress kernel: per (chunk, thread) sign bits in register order (FP32: 64 as uint2, FP64: 128)
     int32_t *p2_ptr = nullptr;     // expand tables: per low-bit position, samples sorted
-    int32_t *p2_list = nullptr;
+    int32_t *p2_list = nullptr;    // [2s] samples by low position, then their rows in that order
     int64_t chunk = 0;             // WHT chunk length used by the expand tables
     // FJLT: compress matrix Kc (s x N) in CSR, and its transpose (N x s) in CSR
     int32_t *k_ptr = nullptr, *k_col = nullptr;

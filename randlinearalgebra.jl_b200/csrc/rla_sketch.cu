@@ -408,20 +408,21 @@ static int fjlt_transpose(rla_ctx *ctx, rla_sketch *sk) {
 // SRHT expand tables: samples grouped by their low log2(chunk) bits.
 static int srht_tables(rla_ctx *ctx, rla_sketch *sk) {
     int64_t s = sk->s;
-    sk->chunk = std::min<int64_t>(sk->N, 4096);
+    sk->chunk = std::min<int64_t>(sk->N, sk->p.dtype == RLA_F32 ? 1 << 14 : 1 << 13);  // chunk of wht_near_kernel
     int64_t ch = sk->chunk;
     std::vector<int32_t> rows(s);
     RLA_CUDA_TRY(ctx, cudaMemcpyAsync(rows.data(), sk->rows, sizeof(int32_t) * s, cudaMemcpyDeviceToHost, ctx->stream));
     RLA_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
-    std::vector<int32_t> ptr(ch + 1, 0), list(s);
+    std::vector<int32_t> ptr(ch + 1, 0), list(2 * s);  // list: samples, then their rows
     for (int64_t k = 0; k < s; ++k) ptr[(rows[k] & (ch - 1)) + 1]++;
     for (int64_t r = 0; r < ch; ++r) ptr[r + 1] += ptr[r];
     std::vector<int32_t> fill(ptr.begin(), ptr.end() - 1);
     for (int64_t k = 0; k < s; ++k) list[fill[rows[k] & (ch - 1)]++] = (int32_t)k;
-    if (!sk->p2_ptr) RLA_CUDA_TRY(ctx, cudaMalloc(&sk->p2_ptr, sizeof(int32_t) * (4096 + 1)));
-    if (!sk->p2_list) RLA_CUDA_TRY(ctx, cudaMalloc(&sk->p2_list, sizeof(int32_t) * s));
+    for (int64_t q = 0; q < s; ++q) list[s + q] = rows[list[q]];
+    if (!sk->p2_ptr) RLA_CUDA_TRY(ctx, cudaMalloc(&sk->p2_ptr, sizeof(int32_t) * (ch + 1)));
+    if (!sk->p2_list) RLA_CUDA_TRY(ctx, cudaMalloc(&sk->p2_list, sizeof(int32_t) * 2 * s));
     RLA_CUDA_TRY(ctx, cudaMemcpyAsync(sk->p2_ptr, ptr.data(), sizeof(int32_t) * (ch + 1), cudaMemcpyHostToDevice, ctx->stream));
-    RLA_CUDA_TRY(ctx, cudaMemcpyAsync(sk->p2_list, list.data(), sizeof(int32_t) * s, cudaMemcpyHostToDevice, ctx->stream));
+    RLA_CUDA_TRY(ctx, cudaMemcpyAsync(sk->p2_list, list.data(), sizeof(int32_t) * 2 * s, cudaMemcpyHostToDevice, ctx->stream));
     RLA_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
     return RLA_OK;
 }

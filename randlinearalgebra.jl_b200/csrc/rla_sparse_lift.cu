@@ -17,7 +17,7 @@
 
 namespace rla {
 
-constexpr int LIFT_WARPS = 16, LIFT_MAX_NNZ = 32;
+constexpr int LIFT_WARPS = 16, LIFT_MAX_NNZ = 32;  // most warps of a CTA
 
 template <class T, int LPE>
 struct LiftCfg {
@@ -40,7 +40,7 @@ struct LiftParams {
     T alpha, beta;
     int beta_zero;
     int64_t nblk;  // blocks of 32 long indices
-    Split split;   // over (tile, block of LIFT_WARPS * 32 long indices)
+    Split split;   // over (tile, a block of 32 long indices per warp)
 };
 
 __device__ __forceinline__ void lift_add(float4 &a, float4 x, uint32_t sign) {
@@ -72,12 +72,12 @@ __global__ void __launch_bounds__(LIFT_WARPS * 32, 1) lift_kernel(LiftParams<T> 
     constexpr int VR = Cfg::VR, C = Cfg::C, JS = Cfg::JS;
     const int nnz = NNZ ? NNZ : p.nnz, wpj = NNZ ? (NNZ + 1) / 2 * 2 : p.wpj;
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    const int t = threadIdx.x, lane = t & 31, wp = t >> 5;
+    const int t = threadIdx.x, lane = t & 31, wp = t >> 5, nt = blockDim.x, warps = nt >> 5;
     unsigned char *out = smem_raw + wp * Cfg::OUT;
-    uint16_t *words = reinterpret_cast<uint16_t *>(smem_raw + LIFT_WARPS * Cfg::OUT) + wp * 32 * wpj;
-    unsigned char *xs = smem_raw + LIFT_WARPS * (Cfg::OUT + 32 * wpj * 2);
+    uint16_t *words = reinterpret_cast<uint16_t *>(smem_raw + warps * Cfg::OUT) + wp * 32 * wpj;
+    unsigned char *xs = smem_raw + warps * (Cfg::OUT + 32 * wpj * 2);
     const int64_t u0 = p.split.start(blockIdx.x), u1 = p.split.start(blockIdx.x + 1);
-    const int64_t nj = (p.nblk + LIFT_WARPS - 1) / LIFT_WARPS;
+    const int64_t nj = (p.nblk + warps - 1) / warps;
     int64_t have = -1;
     for (int64_t u = u0; u < u1; ++u) {
         const int64_t tile = u / nj, v0 = tile * C;
@@ -88,7 +88,7 @@ __global__ void __launch_bounds__(LIFT_WARPS * 32, 1) lift_kernel(LiftParams<T> 
             if (p.x_es == 1) {
                 // lanes along b; VR vectors per thread make one 16-byte store
                 const int ss = (int)p.s;
-                for (int i = t; i < ss * LPE; i += LIFT_WARPS * 32) {
+                for (int i = t; i < ss * LPE; i += nt) {
                     const int q = i / ss, b = i - q * ss;
                     V y{};
                     T *ye = reinterpret_cast<T *>(&y);
@@ -98,7 +98,7 @@ __global__ void __launch_bounds__(LIFT_WARPS * 32, 1) lift_kernel(LiftParams<T> 
                     *reinterpret_cast<V *>(xs + b * Cfg::PITCH + q * 16) = y;
                 }
             } else {
-                for (int i = t; i < (int)p.s * C; i += LIFT_WARPS * 32) {
+                for (int i = t; i < (int)p.s * C; i += nt) {
                     const int b = i / C, c = i % C;
                     *reinterpret_cast<T *>(xs + b * Cfg::PITCH + c * sizeof(T)) =
                         c < nc ? __ldg(p.X + b * p.x_es + (v0 + c) * p.x_vs) : T(0);
@@ -106,7 +106,7 @@ __global__ void __launch_bounds__(LIFT_WARPS * 32, 1) lift_kernel(LiftParams<T> 
             }
             __syncthreads();
         }
-        const int64_t blk = (u - tile * nj) * LIFT_WARPS + wp;
+        const int64_t blk = (u - tile * nj) * warps + wp;
         if (blk >= p.nblk) continue;  // warp-uniform
         const int64_t j0 = blk * 32;
         const int cnt = (int)min((int64_t)32, p.L - j0);
@@ -241,13 +241,16 @@ int sparse_lift(rla_ctx *ctx, const rla_sketch *sk, const T *X, int64_t x_es, in
     *taken = lpe != 0;
     if (!lpe) return RLA_OK;
     const int64_t C = lpe * (16 / (int64_t)sizeof(T)), nblk = ceil_div(sk->L, 32);
-    const int64_t units = ceil_div(nv, C) * ceil_div(nblk, LIFT_WARPS);
+    // fewer warps per CTA while that spreads a small call over more SMs (every CTA stages X)
+    int warps = LIFT_WARPS;
+    while (warps > 4 && ceil_div(nv, C) * ceil_div(nblk, warps) < ctx->sm_count) warps /= 2;
+    const int64_t units = ceil_div(nv, C) * ceil_div(nblk, warps);
     const int W = (int)std::min<int64_t>(ctx->sm_count, units);
     LiftParams<T> p{X, x_es, x_vs, sk->L, nv, sk->s, sk->bucket, sk->negative, (int)sk->nnz, ((int)sk->nnz + 1) / 2 * 2,
                     Y, y_es, y_vs, alpha, beta, beta_zero, nblk, Split::make(units, W)};
     auto go = [&](auto kern) -> int {
         RLA_CUDA_TRY(ctx, set_smem_max(kern));
-        kern<<<W, LIFT_WARPS * 32, smem, ctx->stream>>>(p);
+        kern<<<W, warps * 32, smem, ctx->stream>>>(p);
         return check_launch(ctx, "sparse_lift");
     };
     auto by_nnz = [&](auto lanes) -> int {

@@ -145,6 +145,25 @@ __device__ __forceinline__ double2 get_vec(const Regs<double, 5> &r, int m) {
 __device__ __forceinline__ uint32_t sign_word(uint2 sg, int q) { return q < 32 ? sg.x : sg.y; }
 __device__ __forceinline__ uint32_t sign_word(uint32_t sg, int) { return sg; }
 
+// One butterfly between vectors m and n of a thread.
+__device__ __forceinline__ void wht_pair(Regs<float, 6> &r, int m, int n) {
+    const float2 m1 = make_float2(-1.f, -1.f);
+#pragma unroll
+    for (int o = 0; o < 2; ++o) {
+        const float2 a = r.d[2 * m + o], b = r.d[2 * n + o];
+        r.d[2 * m + o] = __fadd2_rn(a, b);
+        r.d[2 * n + o] = __ffma2_rn(b, m1, a);
+    }
+}
+__device__ __forceinline__ void wht_pair(Regs<double, 5> &r, int m, int n) {
+#pragma unroll
+    for (int o = 0; o < 2; ++o) {
+        const double a = r.d[2 * m + o], b = r.d[2 * n + o];
+        r.d[2 * m + o] = a + b;
+        r.d[2 * n + o] = a - b;
+    }
+}
+
 // Radix-2 butterflies over bits 0..3 of the index of a thread's 16 vectors (the elements of
 // a vector are carried through): packed FP32x2 adds and subtracts, or FP64 scalar ones.
 __device__ __forceinline__ void wht_vec16(Regs<float, 6> &r) {
@@ -175,6 +194,41 @@ __device__ __forceinline__ void wht_vec16(Regs<double, 5> &r) {
                     r.d[2 * (m | (1 << h)) + o] = a - b;
                 }
             }
+}
+
+// Butterflies over the VB bits inside a vector, and over the lowest `top` bits of the vector index.
+__device__ __forceinline__ void wht_inside(Regs<float, 6> &r) {
+    const float2 m1 = make_float2(-1.f, -1.f);
+#pragma unroll
+    for (int m = 0; m < 32; ++m) {
+        const float a = r.d[m].x, b = r.d[m].y;
+        r.d[m].x = a + b;
+        r.d[m].y = a - b;
+    }
+#pragma unroll
+    for (int m = 0; m < 32; m += 2) {
+        const float2 a = r.d[m], b = r.d[m + 1];
+        r.d[m] = __fadd2_rn(a, b);
+        r.d[m + 1] = __ffma2_rn(b, m1, a);
+    }
+}
+__device__ __forceinline__ void wht_inside(Regs<double, 5> &r) {
+#pragma unroll
+    for (int m = 0; m < 32; m += 2) {
+        const double a = r.d[m], b = r.d[m + 1];
+        r.d[m] = a + b;
+        r.d[m + 1] = a - b;
+    }
+}
+template <class R>
+__device__ __forceinline__ void wht_top(R &r, int top) {
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {
+        if (h >= top) break;
+#pragma unroll
+        for (int m = 0; m < 16; ++m)
+            if (!(m & (1 << h))) wht_pair(r, m, m | (1 << h));
+    }
 }
 
 // Pass-A loads of the chunk at cbase of column xv: register q = i | k<<VB (i < 2^VB, k < 16)
@@ -409,7 +463,7 @@ int build_srht_sign_table(rla_ctx *ctx, rla_sketch *sk) {
     return check_launch(ctx, "sign_table");
 }
 
-// Small padded sizes (N < 2^CH): one CTA per column, the whole padded column in
+// Small padded sizes (N < 2^(VB+8)): one CTA per column, the whole padded column in
 // shared memory, log2(N) butterfly stages.
 template <class T>
 __global__ void srht_small_kernel(const T *X, int64_t x_ld, int64_t L, int64_t N, int64_t nv,
@@ -490,67 +544,333 @@ __global__ void srht_expand_kernel(const T *X, int64_t x_es, int64_t x_vs, int64
     }
 }
 
-// ---- generic full transform for FJLT: W (N x nv, ld = N) in place --------------------
+// ------------------------------------------------------------------------------------
+// Transforms of whole padded columns (FJLT, SRHT expand, SRHT of short columns).
+//
+// The columns of a batch are one run of nv * N elements (N >= 2^(VB+8)); a CTA takes 2^CH of them:
+// a chunk of a column, or several short columns.  The butterflies are those of the fused kernel's
+// three register passes, with the top stages left out for short columns.  The source is the
+// operand itself (sign flip and padding while loading), the batch workspace, the transposed
+// sampling matrix of the FJLT or the samples of the SRHT; the result goes to the workspace, to
+// the output with its signs, or is sampled from shared memory.  Columns above 2^CH take
+// wht_far_kernel for the remaining bits.  Workspace batches hold at most 64 MB, so that the passes
+// between the first read and the last write stay in L2 (126 MB).
+//
+// Bound by the loads' latency in the near kernel (2 CTAs per SM, all of a thread's loads in flight
+// together) and by L2 in the rest.  FJLT 100003 -> 600 of 96 Float32 columns: 88 us a call
+// (near 30, far 10, gather 19), 324 us with a padding pass, scalar shared-memory stages and one
+// pass over the workspace per bit above 2^12; SRHT expand to 360737 x 61: 156 against 416 us, SRHT
+// 5003 -> 300 of 200 columns 28 against 85 us.
+// ------------------------------------------------------------------------------------
+enum WhtIn { WHT_IN_X, WHT_IN_W, WHT_IN_KT, WHT_IN_SAMPLES };
+enum WhtOut { WHT_OUT_W, WHT_OUT_Y, WHT_OUT_ROWS };
+
 template <class T>
-__global__ void wht_chunk_kernel(T *W, int64_t N, int64_t nv, int ch) {
+struct WhtParams {
+    const T *X;
+    int64_t x_es, x_vs;  // IN_X: x_es == 1
+    int x_vec;           // IN_X: every column starts on 16 bytes
+    int64_t L, N, nv;
+    int log_n, top;      // top: stages over bits [VB+8, VB+8+top) of the chunk
+    const uint32_t *signbits;
+    const int32_t *ptr, *idx;  // IN_KT: CSR of the transposed sampling matrix; IN_SAMPLES: idx = [samples | their rows] by low position
+    const T *val;
+    const int32_t *rows;       // IN_SAMPLES, OUT_ROWS
+    int64_t s;
+    T *W;
+    T *Y;
+    int64_t y_es, y_vs;
+    T alpha, beta;
+    int beta_zero;
+};
+
+// y = alpha * z (+ beta * y), z a 16-byte vector, signs from bits [r, r + 2^VB) of signbits.
+template <class T>
+__device__ __forceinline__ void wht_put(const WhtParams<T> &p, int64_t r, int64_t v, typename WhtCfg<T>::V z) {
+    constexpr int VW = 1 << WhtCfg<T>::VB;
+    const uint32_t sb = __ldg(p.signbits + (r >> 5)) >> (r & 31);
+    T *zp = reinterpret_cast<T *>(&z);
+    T *yp = p.Y + r * p.y_es + v * p.y_vs;
+#pragma unroll
+    for (int i = 0; i < VW; ++i) zp[i] = p.alpha * flip(zp[i], sb >> i);
+    if (p.beta_zero && p.y_es == 1 && r + VW <= p.L && (reinterpret_cast<uintptr_t>(yp) & 15u) == 0) {
+        *reinterpret_cast<typename WhtCfg<T>::V *>(yp) = z;
+        return;
+    }
+#pragma unroll
+    for (int i = 0; i < VW; ++i)
+        if (r + i < p.L) yp[i * p.y_es] = p.beta_zero ? zp[i] : zp[i] + p.beta * yp[i * p.y_es];
+}
+
+template <class T, int IN, int OUT>
+__global__ void __launch_bounds__(256, 2) wht_near_kernel(WhtParams<T> p) {
+    constexpr int VB = WhtCfg<T>::VB, CH = WhtCfg<T>::CH, VW = 1 << VB;
+    using V = typename WhtCfg<T>::V;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    T *Z = reinterpret_cast<T *>(smem_raw);
+    const int t = threadIdx.x, lane = t & 31, wp = t >> 5;
+    const int baseA = swzv<VB>(t << VB);
+    const int baseB = (t << (VB + 4)) | ((t & 7) << VB);
+    const int eC = ((lane & 15) << VB) | ((lane >> 4) << (VB + 8)) | (wp << (VB + 9));
+    const int64_t total = p.nv << p.log_n, nchunk = (total + (1 << CH) - 1) >> CH;
+    for (int64_t c = blockIdx.x; c < nchunk; c += gridDim.x) {
+        const int64_t base = c << CH;
+        Regs<T, VB + 4> r;
+        // the chunk starts at element e0 of column vc; short columns follow one another in it
+        const int64_t vc = base >> p.log_n, e0 = base & (p.N - 1);
+        const int in_chunk = (int)min(p.N - 1, (int64_t)(1 << CH) - 1);
+        if constexpr (IN == WHT_IN_SAMPLES) {
+            // samples in the order of their low position (zero elsewhere): the first of a run of
+            // samples with one low position adds the run
+#pragma unroll
+            for (int k = 0; k < 16; ++k) *reinterpret_cast<V *>(Z + baseA + (k << (VB + 8))) = V{};
+            __syncthreads();
+            const int ncol = (int)min((int64_t)((1 << CH) / (in_chunk + 1)), p.nv - vc), s = (int)p.s;
+            const uint32_t r1 = (uint32_t)(e0 >> CH);
+            for (int q = t; q < s * ncol; q += 256) {
+                const int cc = q / s, qq = q - cc * s;
+                uint32_t row = (uint32_t)__ldg(p.idx + s + qq);
+                const int lo = (int)(row & in_chunk);
+                if (qq > 0 && (int)((uint32_t)__ldg(p.idx + s + qq - 1) & in_chunk) == lo) continue;
+                T sum = T(0);
+                for (int n = qq;;) {
+                    const T x = __ldg(p.X + (int64_t)__ldg(p.idx + n) * p.x_es + (vc + cc) * p.x_vs);
+                    sum += flip(x, ~__popc((row >> CH) & r1));
+                    if (++n == s) break;
+                    row = (uint32_t)__ldg(p.idx + s + n);
+                    if ((int)(row & in_chunk) != lo) break;
+                }
+                Z[swzv<VB>((cc << p.log_n) + lo)] = sum;
+            }
+            __syncthreads();
+#pragma unroll
+            for (int k = 0; k < 16; ++k) set_vec(r, k, *reinterpret_cast<const V *>(Z + baseA + (k << (VB + 8))));
+        } else {
+#pragma unroll
+            for (int k = 0; k < 16; ++k) {
+                const int o = (t << VB) + (k << (VB + 8));
+                const int64_t v = vc + (o >> min(p.log_n, 31)), e = e0 + (o & in_chunk);
+                V q{};
+                T *qe = reinterpret_cast<T *>(&q);
+                if constexpr (IN == WHT_IN_X) {
+                    // loads without branches, so that all of a thread's are in flight together
+                    const T *x = p.X + e + v * p.x_vs;
+                    const int64_t left = v < p.nv ? p.L - e : 0;
+                    if (p.x_vec) {
+                        if (left >= VW) q = __ldg(reinterpret_cast<const V *>(x));
+#pragma unroll
+                        for (int i = 0; i < VW - 1; ++i)
+                            if (i < left && left < VW) qe[i] = __ldg(x + i);
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < VW; ++i)
+                            if (i < left) qe[i] = __ldg(x + i);
+                    }
+                } else if constexpr (IN == WHT_IN_W) {
+                    if (v < p.nv) q = *reinterpret_cast<const V *>(p.W + base + o);
+                } else if (v < p.nv) {  // IN_KT: rows e .. of the transposed matrix
+                    int a = __ldg(p.ptr + e);
+#pragma unroll
+                    for (int i = 0; i < VW; ++i) {
+                        const int b = __ldg(p.ptr + e + i + 1);
+                        T sum = T(0);
+                        for (int k2 = a; k2 < b; ++k2)
+                            sum += __ldg(p.val + k2) * __ldg(p.X + (int64_t)__ldg(p.idx + k2) * p.x_es + v * p.x_vs);
+                        qe[i] = sum;
+                        a = b;
+                    }
+                }
+                set_vec(r, k, q);
+            }
+            if constexpr (IN == WHT_IN_X) {
+#pragma unroll
+                for (int k = 0; k < 16; ++k) {
+                    const int64_t e = e0 + (((t << VB) + (k << (VB + 8))) & in_chunk);
+                    const uint32_t sb = __ldg(p.signbits + (e >> 5)) >> (e & 31);
+#pragma unroll
+                    for (int i = 0; i < VW; ++i) r.set(k * VW + i, flip(r.get(k * VW + i), sb >> i));
+                }
+            }
+        }
+        wht_inside(r);
+        wht_top(r, p.top);
+#pragma unroll
+        for (int k = 0; k < 16; ++k) *reinterpret_cast<V *>(Z + baseA + (k << (VB + 8))) = get_vec(r, k);
+        __syncthreads();
+#pragma unroll
+        for (int m = 0; m < 16; ++m)
+            set_vec(r, m, *reinterpret_cast<const V *>(Z + (baseB ^ ((m & 7) << VB)) + ((m >> 3) << (VB + 3))));
+        wht_vec16(r);
+#pragma unroll
+        for (int m = 0; m < 16; ++m)
+            *reinterpret_cast<V *>(Z + (baseB ^ ((m & 7) << VB)) + ((m >> 3) << (VB + 3))) = get_vec(r, m);
+        __syncthreads();
+#pragma unroll
+        for (int m = 0; m < 16; ++m)
+            set_vec(r, m, *reinterpret_cast<const V *>(Z + (eC ^ ((m & 7) << VB)) + (m << (VB + 4))));
+        wht_vec16(r);
+        if constexpr (OUT == WHT_OUT_ROWS) {
+#pragma unroll
+            for (int m = 0; m < 16; ++m)
+                *reinterpret_cast<V *>(Z + (eC ^ ((m & 7) << VB)) + (m << (VB + 4))) = get_vec(r, m);
+            __syncthreads();
+            const int64_t v0 = base >> p.log_n, ncol = min((int64_t)1 << (CH - p.log_n), p.nv - v0);
+            for (int64_t cc = 0; cc < ncol; ++cc)
+                for (int64_t i = t; i < p.s; i += 256) {
+                    T *yp = p.Y + i * p.y_es + (v0 + cc) * p.y_vs;
+                    T res = p.alpha * Z[swzv<VB>((int)(cc << p.log_n) + __ldg(p.rows + i))];
+                    if (!p.beta_zero) res += p.beta * *yp;
+                    *yp = res;
+                }
+        } else {
+#pragma unroll
+            for (int m = 0; m < 16; ++m) {
+                const int64_t f = base + (eC | (m << (VB + 4)));
+                if (f < total) {
+                    if constexpr (OUT == WHT_OUT_W) *reinterpret_cast<V *>(p.W + f) = get_vec(r, m);
+                    else wht_put(p, f & (p.N - 1), f >> p.log_n, get_vec(r, m));
+                }
+            }
+        }
+        __syncthreads();
+    }
+}
+
+// Butterflies over bits [b0, b0 + RB) of the workspace's columns: a thread holds one 16-byte vector
+// at 2^RB rows 2^b0 apart.
+template <class T, int RB, int OUT>
+__global__ void __launch_bounds__(256) wht_far_kernel(WhtParams<T> p, int b0) {
+    constexpr int VB = WhtCfg<T>::VB, NV = 1 << RB;
+    using V = typename WhtCfg<T>::V;
+    const int64_t per = p.N >> (VB + RB), total = per * p.nv;
+    for (int64_t q = blockIdx.x * 256ll + threadIdx.x; q < total; q += gridDim.x * 256ll) {
+        const int64_t v = q / per, g = q - v * per;
+        const int64_t lo = g & (((int64_t)1 << (b0 - VB)) - 1), hi = g >> (b0 - VB);
+        const int64_t e = (hi << (b0 + RB)) | (lo << VB);
+        T *w = p.W + (v << p.log_n) + e;
+        V x[NV];
+#pragma unroll
+        for (int i = 0; i < NV; ++i) x[i] = *reinterpret_cast<const V *>(w + ((int64_t)i << b0));
+#pragma unroll
+        for (int h = 0; h < RB; ++h)
+#pragma unroll
+            for (int i = 0; i < NV; ++i)
+                if (!(i & (1 << h))) {
+                    T *a = reinterpret_cast<T *>(&x[i]), *b = reinterpret_cast<T *>(&x[i | (1 << h)]);
+#pragma unroll
+                    for (int k = 0; k < (1 << VB); ++k) {
+                        const T s = a[k] + b[k], d = a[k] - b[k];
+                        a[k] = s;
+                        b[k] = d;
+                    }
+                }
+#pragma unroll
+        for (int i = 0; i < NV; ++i) {
+            if constexpr (OUT == WHT_OUT_W) *reinterpret_cast<V *>(w + ((int64_t)i << b0)) = x[i];
+            else wht_put(p, e + ((int64_t)i << b0), v, x[i]);
+        }
+    }
+}
+
+// Short columns (N < 2^(VB+8)) of the workspace in place, one CTA per column.
+template <class T>
+__global__ void wht_short_kernel(T *W, int64_t N, int64_t nv) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     T *z = reinterpret_cast<T *>(smem_raw);
-    const int64_t nchunks = N / ch;
-    for (int64_t blk = blockIdx.x; blk < nv * nchunks; blk += gridDim.x) {
-        T *w = W + (blk / nchunks) * N + (blk % nchunks) * ch;
-        for (int e = threadIdx.x; e < ch; e += blockDim.x) z[e] = w[e];
+    const int n = (int)N;
+    for (int64_t v = blockIdx.x; v < nv; v += gridDim.x) {
+        T *w = W + v * N;
+        for (int e = threadIdx.x; e < n; e += blockDim.x) z[e] = w[e];
         __syncthreads();
-        for (int h = 1; h < ch; h <<= 1) {
-            for (int q = threadIdx.x; q < ch / 2; q += blockDim.x) {
-                const int i = (q / h) * 2 * h + (q % h);
-                T a = z[i], b = z[i + h];
+        for (int h = 1; h < n; h <<= 1) {
+            for (int q = threadIdx.x; q < n / 2; q += blockDim.x) {
+                const int i = (q & ~(h - 1)) * 2 + (q & (h - 1));
+                const T a = z[i], b = z[i + h];
                 z[i] = a + b;
                 z[i + h] = a - b;
             }
             __syncthreads();
         }
-        for (int e = threadIdx.x; e < ch; e += blockDim.x) w[e] = z[e];
+        for (int e = threadIdx.x; e < n; e += blockDim.x) w[e] = z[e];
         __syncthreads();
     }
 }
 
-template <class T>
-__global__ void wht_stage_kernel(T *W, int64_t N, int64_t nv, int64_t h) {
-    const int64_t half = N / 2;
-    for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < half * nv; q += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t v = q / half, qq = q % half;
-        const int64_t i = (qq / h) * 2 * h + (qq % h);
-        T *w = W + v * N;
-        T a = w[i], b = w[i + h];
-        w[i] = a + b;
-        w[i + h] = a - b;
-    }
-}
-
-// W(r, v) = r < L ? d_r * X(r, v) : 0
+// W(r, v) = r < L ? d_r * X(r, v) : 0 for any strides of X, through 32 x 32 tiles.
 template <class T>
 __global__ void fjlt_pad_sign_kernel(const T *X, int64_t x_es, int64_t x_vs, int64_t L, int64_t N, int64_t nv,
                                      const uint32_t *signbits, T *W) {
-    for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < N * nv; q += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t v = q / N, r = q % N;
-        T x = r < L ? X[r * x_es + v * x_vs] : T(0);
-        W[q] = ((signbits[r >> 5] >> (r & 31)) & 1u) ? x : -x;
+    __shared__ T tile[32][33];
+    const int64_t r0 = (int64_t)blockIdx.x * 32, v0 = (int64_t)blockIdx.y * 32;
+    const bool along_v = x_vs == 1;
+    for (int yy = threadIdx.y; yy < 32; yy += blockDim.y) {
+        const int rr = along_v ? yy : (int)threadIdx.x, vv = along_v ? (int)threadIdx.x : yy;
+        const int64_t r = r0 + rr, v = v0 + vv;
+        tile[rr][vv] = (r < L && v < nv) ? X[r * x_es + v * x_vs] : T(0);
+    }
+    __syncthreads();
+    const int64_t r = r0 + threadIdx.x;
+    if (r >= N) return;
+    const uint32_t keep = signbits[r >> 5] >> (r & 31);
+    for (int yy = threadIdx.y; yy < 32; yy += blockDim.y)
+        if (v0 + yy < nv) W[r + (v0 + yy) * N] = flip(tile[threadIdx.x][yy], keep);
+}
+
+// Y(r, v) = alpha * d_r * W(r, v) + beta * Y(r, v), r < L, for any strides of Y.
+template <class T>
+__global__ void fjlt_expand_out_kernel(const T *W, int64_t N, int64_t L, int64_t nv, const uint32_t *signbits, T *Y,
+                                       int64_t y_es, int64_t y_vs, T alpha, T beta, int beta_zero) {
+    __shared__ T tile[32][33];
+    const int64_t r0 = (int64_t)blockIdx.x * 32, v0 = (int64_t)blockIdx.y * 32;
+    for (int yy = threadIdx.y; yy < 32; yy += blockDim.y) {
+        const int64_t r = r0 + threadIdx.x, v = v0 + yy;
+        tile[threadIdx.x][yy] = (r < N && v < nv) ? W[r + v * N] : T(0);
+    }
+    __syncthreads();
+    const bool along_v = y_vs == 1;
+    for (int yy = threadIdx.y; yy < 32; yy += blockDim.y) {
+        const int rr = along_v ? yy : (int)threadIdx.x, vv = along_v ? (int)threadIdx.x : yy;
+        const int64_t r = r0 + rr, v = v0 + vv;
+        if (r >= L || v >= nv) continue;
+        T *yp = Y + r * y_es + v * y_vs;
+        T res = alpha * flip(tile[rr][vv], signbits[r >> 5] >> (r & 31));
+        if (!beta_zero) res += beta * *yp;
+        *yp = res;
     }
 }
 
-// Y(i, v) = alpha * sum_k val_k * W(col_k, v) + beta * Y(i, v), rows i of a CSR matrix.
+// Y(i, v) = alpha * sum_k val_k * W(col_k, v) + beta * Y(i, v), rows i of a CSR matrix: 8 lanes share
+// a row's entries, for 4 vectors at a time (4 independent gathers per entry).
 template <class T>
-__global__ void csr_gather_kernel(const int32_t *ptr, const int32_t *col, const T *val, int64_t nrows, const T *W,
-                                  int64_t w_ld, int64_t nv, T *Y, int64_t y_es, int64_t y_vs, T alpha, T beta,
-                                  int beta_zero) {
-    for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < nrows * nv; q += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t v = q / nrows, i = q % nrows;
-        T acc = T(0);
-        for (int k = ptr[i]; k < ptr[i + 1]; ++k) acc += val[k] * W[(int64_t)col[k] + v * w_ld];
-        T *yp = Y + i * y_es + v * y_vs;
-        T res = alpha * acc;
-        if (!beta_zero) res += beta * *yp;
-        *yp = res;
+__global__ void __launch_bounds__(256) csr_gather_kernel(const int32_t *ptr, const int32_t *col, const T *val, int64_t nrows,
+                                                         const T *W, int64_t w_ld, int64_t nv, T *Y, int64_t y_es,
+                                                         int64_t y_vs, T alpha, T beta, int beta_zero) {
+    const int l8 = threadIdx.x & 7;
+    const int64_t nvg = (nv + 3) / 4, total = nrows * nvg;
+    for (int64_t g = (blockIdx.x * 256ll + threadIdx.x) >> 3; g < ((total + 3) & ~3ll); g += gridDim.x * 32ll) {
+        // neighbouring octets go along the contiguous dimension of Y; the last warp may be partial
+        const bool on = g < total;
+        const int64_t i = on ? (y_es == 1 ? g % nrows : g / nvg) : 0, v0 = on ? (y_es == 1 ? g / nrows : g % nvg) * 4 : 0;
+        T acc[4] = {T(0), T(0), T(0), T(0)};
+        const int b = on ? __ldg(ptr + i + 1) : 0;
+        for (int k = on ? __ldg(ptr + i) + l8 : 0; k < b; k += 8) {
+            const T a = __ldg(val + k);
+            const T *w = W + __ldg(col + k) + v0 * w_ld;
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (v0 + u < nv) acc[u] += a * w[u * w_ld];
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+#pragma unroll
+            for (int m = 4; m > 0; m >>= 1) acc[u] += __shfl_xor_sync(FULL, acc[u], m);
+            if (on && l8 == u && v0 + u < nv) {
+                T *yp = Y + i * y_es + (v0 + u) * y_vs;
+                T res = alpha * acc[u];
+                if (!beta_zero) res += beta * *yp;
+                *yp = res;
+            }
+        }
     }
 }
 
@@ -563,19 +883,6 @@ __global__ void csr_t_gather_kernel(const int32_t *ptr, const int32_t *rowi, con
         T acc = T(0);
         for (int k = ptr[r]; k < ptr[r + 1]; ++k) acc += val[k] * X[(int64_t)rowi[k] * x_es + v * x_vs];
         W[q] = acc;
-    }
-}
-
-template <class T>
-__global__ void fjlt_expand_out_kernel(const T *W, int64_t N, int64_t L, int64_t nv, const uint32_t *signbits, T *Y,
-                                       int64_t y_es, int64_t y_vs, T alpha, T beta, int beta_zero) {
-    for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < L * nv; q += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t v = q / L, r = q % L;
-        const T d = ((signbits[r >> 5] >> (r & 31)) & 1u) ? alpha : -alpha;
-        T *yp = Y + r * y_es + v * y_vs;
-        T res = d * W[r + v * N];
-        if (!beta_zero) res += beta * *yp;
-        *yp = res;
     }
 }
 
@@ -611,6 +918,96 @@ static int to_contiguous(rla_ctx *ctx, const T *X, int64_t x_es, int64_t x_vs, i
     return check_launch(ctx, "gather_columns");
 }
 
+// Columns per workspace batch (64 MB, see above).
+template <class T>
+static int64_t wht_batch(int64_t N, int64_t nv) {
+    return std::min<int64_t>(nv, std::max<int64_t>(1, (int64_t)(64 << 20) / (N * (int64_t)sizeof(T))));
+}
+
+template <class T>
+constexpr int64_t wht_near_min() {  // shortest column of wht_near_kernel
+    return (int64_t)1 << (WhtCfg<T>::VB + 8);
+}
+
+template <class T>
+static WhtParams<T> wht_params(const rla_sketch *sk, int64_t nv) {
+    WhtParams<T> p{};
+    p.L = sk->L;
+    p.N = sk->N;
+    p.nv = nv;
+    p.log_n = ilog2(sk->N);
+    p.top = std::min(4, p.log_n - (WhtCfg<T>::VB + 8));
+    p.signbits = sk->signbits;
+    p.rows = sk->rows;
+    p.s = sk->s;
+    return p;
+}
+
+template <class T, int IN, int OUT>
+static int launch_near(rla_ctx *ctx, const WhtParams<T> &p) {
+    constexpr int CH = WhtCfg<T>::CH;
+    auto kern = wht_near_kernel<T, IN, OUT>;
+    RLA_CUDA_TRY(ctx, set_smem_max(kern));
+    const int64_t nchunk = ceil_div(p.nv << p.log_n, (int64_t)1 << CH);
+    kern<<<(unsigned)std::min<int64_t>(nchunk, (int64_t)ctx->sm_count * 2), 256, sizeof(T) << CH, ctx->stream>>>(p);
+    return check_launch(ctx, "wht_near");
+}
+
+// The bits above 2^CH, four at most per pass; the last pass writes the output when out_y.
+template <class T>
+static int launch_far(rla_ctx *ctx, const WhtParams<T> &p, bool out_y) {
+    for (int b = WhtCfg<T>::CH; b < p.log_n;) {
+        const int left = p.log_n - b, passes = (left + 3) / 4, rb = (left + passes - 1) / passes;
+        const bool y = out_y && rb == left;
+        const int64_t work = (p.N >> (WhtCfg<T>::VB + rb)) * p.nv;
+        const unsigned grid = (unsigned)std::min<int64_t>(ceil_div(work, 256), (int64_t)ctx->sm_count * 16);
+        auto go = [&](auto ky, auto kw) {
+            if (y) ky<<<grid, 256, 0, ctx->stream>>>(p, b);
+            else kw<<<grid, 256, 0, ctx->stream>>>(p, b);
+        };
+        if (rb == 1) go(wht_far_kernel<T, 1, WHT_OUT_Y>, wht_far_kernel<T, 1, WHT_OUT_W>);
+        else if (rb == 2) go(wht_far_kernel<T, 2, WHT_OUT_Y>, wht_far_kernel<T, 2, WHT_OUT_W>);
+        else if (rb == 3) go(wht_far_kernel<T, 3, WHT_OUT_Y>, wht_far_kernel<T, 3, WHT_OUT_W>);
+        else go(wht_far_kernel<T, 4, WHT_OUT_Y>, wht_far_kernel<T, 4, WHT_OUT_W>);
+        RLA_TRY(check_launch(ctx, "wht_far"));
+        b += rb;
+    }
+    return RLA_OK;
+}
+
+static dim3 tiles32(int64_t len, int64_t nv) { return dim3(ceil_div_i(len, 32), ceil_div_i(nv, 32)); }
+
+template <class T>
+static int launch_out(rla_ctx *ctx, const WhtParams<T> &p) {
+    fjlt_expand_out_kernel<T><<<tiles32(p.L, p.nv), dim3(32, 8), 0, ctx->stream>>>(
+        p.W, p.N, p.L, p.nv, p.signbits, p.Y, p.y_es, p.y_vs, p.alpha, p.beta, p.beta_zero);
+    return check_launch(ctx, "wht_out");
+}
+
+// Columns shorter than a chunk: several per CTA, sampled from shared memory.
+template <class T>
+static int srht_short(rla_ctx *ctx, const rla_sketch *sk, const T *X, int64_t ldx, int64_t nv, T *Y, int64_t y_es,
+                      int64_t y_vs, T alpha, T beta, bool beta_zero) {
+    if (sk->N < wht_near_min<T>()) {
+        const int grid = (int)std::min<int64_t>(nv, (int64_t)ctx->sm_count * 8);
+        srht_small_kernel<T><<<grid, 256, (size_t)sk->N * sizeof(T), ctx->stream>>>(
+            X, ldx, sk->L, sk->N, nv, sk->signbits, sk->rows, sk->s, Y, y_es, y_vs, alpha, beta, beta_zero);
+        return check_launch(ctx, "srht_small");
+    }
+    WhtParams<T> p = wht_params<T>(sk, nv);
+    p.X = X;
+    p.x_es = 1;
+    p.x_vs = ldx;
+    p.x_vec = ldx % (1 << WhtCfg<T>::VB) == 0 && (uintptr_t)X % 16 == 0;
+    p.Y = Y;
+    p.y_es = y_es;
+    p.y_vs = y_vs;
+    p.alpha = alpha;
+    p.beta = beta;
+    p.beta_zero = beta_zero;
+    return launch_near<T, WHT_IN_X, WHT_OUT_ROWS>(ctx, p);
+}
+
 template <class T>
 int srht_compress(rla_ctx *ctx, const rla_sketch *sk, const T *X, int64_t x_es, int64_t x_vs, int64_t nv, T *Y,
                   int64_t y_es, int64_t y_vs, double alpha, double beta) {
@@ -644,14 +1041,7 @@ int srht_compress(rla_ctx *ctx, const rla_sketch *sk, const T *X, int64_t x_es, 
         Xc = (const T *)scratch;
         ldx = L;
     }
-    if (N < ((int64_t)1 << CH)) {
-        const size_t smem = (size_t)N * es;
-        set_smem_max(srht_small_kernel<T>);
-        const int grid = (int)std::min<int64_t>(nv, (int64_t)ctx->sm_count * 8);
-        srht_small_kernel<T><<<grid, 256, smem, ctx->stream>>>(Xc, ldx, L, N, nv, sk->signbits, sk->rows, s, Y, y_es,
-                                                               y_vs, a, (T)beta, beta_zero);
-        return check_launch(ctx, "srht_small");
-    }
+    if (N < ((int64_t)1 << CH)) return srht_short<T>(ctx, sk, Xc, ldx, nv, Y, y_es, y_vs, a, (T)beta, beta_zero);
     int *cnt = nullptr;
     RLA_TRY(counters_get(ctx, (size_t)nv, &cnt));
     const bool vec = (ldx % (int64_t)(1 << VB) == 0) && ((uintptr_t)Xc % 16 == 0);
@@ -668,33 +1058,45 @@ int srht_compress(rla_ctx *ctx, const rla_sketch *sk, const T *X, int64_t x_es, 
     return RLA_OK;
 }
 
+// A strided output is written through the workspace (32 x 32 tiles); batches keep grid.y in range.
 template <class T>
 int srht_expand(rla_ctx *ctx, const rla_sketch *sk, const T *X, int64_t x_es, int64_t x_vs, int64_t nv, T *Y,
                 int64_t y_es, int64_t y_vs, double alpha, double beta) {
     if (nv == 0) return RLA_OK;
-    const int ch = (int)sk->chunk;
-    const int log_ch = ilog2(ch);
-    const int64_t nblk = nv * (sk->N >> log_ch);
-    const int grid = (int)std::min<int64_t>(nblk, (int64_t)ctx->sm_count * 16);
-    const size_t smem = (size_t)ch * sizeof(T);
-    srht_expand_kernel<T><<<grid, 256, smem, ctx->stream>>>(X, x_es, x_vs, sk->L, sk->N, nv, sk->signbits, sk->rows,
-                                                            sk->p2_ptr, sk->p2_list, ch, log_ch, Y, y_es, y_vs,
-                                                            (T)(alpha * sk->scale), (T)beta, beta == 0.0);
-    return check_launch(ctx, "srht_expand");
-}
-
-template <class T>
-static int wht_full(rla_ctx *ctx, T *W, int64_t N, int64_t nv) {
-    const int ch = (int)std::min<int64_t>(N, 4096);
-    const int64_t nblk = nv * (N / ch);
-    wht_chunk_kernel<T><<<(int)std::min<int64_t>(nblk, (int64_t)ctx->sm_count * 16), 256, ch * sizeof(T), ctx->stream>>>(
-        W, N, nv, ch);
-    RLA_TRY(check_launch(ctx, "wht_chunk"));
-    for (int64_t h = ch; h < N; h <<= 1) {
-        const int64_t work = (N / 2) * nv;
-        wht_stage_kernel<T><<<(int)std::min<int64_t>(ceil_div(work, 256), (int64_t)ctx->sm_count * 32), 256, 0,
-                              ctx->stream>>>(W, N, nv, h);
-        RLA_TRY(check_launch(ctx, "wht_stage"));
+    const T a = (T)(alpha * sk->scale);
+    if (sk->N < wht_near_min<T>()) {
+        const int ch = (int)sk->chunk;
+        const int log_ch = ilog2(ch);
+        const int64_t nblk = nv * (sk->N >> log_ch);
+        const int grid = (int)std::min<int64_t>(nblk, (int64_t)ctx->sm_count * 16);
+        const size_t smem = (size_t)ch * sizeof(T);
+        srht_expand_kernel<T><<<grid, 256, smem, ctx->stream>>>(X, x_es, x_vs, sk->L, sk->N, nv, sk->signbits, sk->rows,
+                                                                sk->p2_ptr, sk->p2_list, ch, log_ch, Y, y_es, y_vs, a,
+                                                                (T)beta, beta == 0.0);
+        return check_launch(ctx, "srht_expand");
+    }
+    WhtParams<T> p = wht_params<T>(sk, nv);
+    p.X = X;
+    p.x_es = x_es;
+    p.x_vs = x_vs;
+    p.idx = sk->p2_list;
+    p.Y = Y;
+    p.y_es = y_es;
+    p.y_vs = y_vs;
+    p.alpha = a;
+    p.beta = (T)beta;
+    p.beta_zero = beta == 0.0;
+    if (y_es == 1) return launch_near<T, WHT_IN_SAMPLES, WHT_OUT_Y>(ctx, p);
+    const int64_t nb = std::min<int64_t>(wht_batch<T>(sk->N, nv), 65535 * 32);
+    void *w;
+    RLA_TRY(scratch_get(ctx, (size_t)(sk->N * nb) * sizeof(T), &w));
+    p.W = (T *)w;
+    for (int64_t v = 0; v < nv; v += nb) {
+        p.nv = std::min(nb, nv - v);
+        p.X = X + v * x_vs;
+        p.Y = Y + v * y_vs;
+        RLA_TRY((launch_near<T, WHT_IN_SAMPLES, WHT_OUT_W>(ctx, p)));
+        RLA_TRY(launch_out(ctx, p));
     }
     return RLA_OK;
 }
@@ -703,38 +1105,85 @@ template <class T>
 int fjlt_compress(rla_ctx *ctx, const rla_sketch *sk, const T *X, int64_t x_es, int64_t x_vs, int64_t nv, T *Y,
                   int64_t y_es, int64_t y_vs, double alpha, double beta) {
     if (nv == 0) return RLA_OK;
-    const int64_t N = sk->N;
+    const int64_t N = sk->N, nb = std::min<int64_t>(wht_batch<T>(N, nv), 65535 * 32);
     void *w;
-    RLA_TRY(scratch_get(ctx, (size_t)N * nv * sizeof(T), &w));
-    T *Wb = (T *)w;
-    const int grid = (int)std::min<int64_t>(ceil_div(N * nv, 256), (int64_t)ctx->sm_count * 32);
-    fjlt_pad_sign_kernel<T><<<grid, 256, 0, ctx->stream>>>(X, x_es, x_vs, sk->L, N, nv, sk->signbits, Wb);
-    RLA_TRY(check_launch(ctx, "fjlt_pad_sign"));
-    RLA_TRY(wht_full(ctx, Wb, N, nv));
-    const int grid2 = (int)std::min<int64_t>(ceil_div(sk->s * nv, 256), (int64_t)ctx->sm_count * 32);
-    csr_gather_kernel<T><<<std::max(grid2, 1), 256, 0, ctx->stream>>>(sk->k_ptr, sk->k_col, (const T *)sk->k_val, sk->s,
-                                                                     Wb, N, nv, Y, y_es, y_vs, (T)(alpha * sk->scale),
-                                                                     (T)beta, beta == 0.0);
-    return check_launch(ctx, "fjlt_csr_gather");
+    RLA_TRY(scratch_get(ctx, (size_t)(N * nb) * sizeof(T), &w));
+    WhtParams<T> p = wht_params<T>(sk, nv);
+    p.x_es = x_es;
+    p.x_vs = x_vs;
+    p.W = (T *)w;
+    const bool near = N >= wht_near_min<T>();
+    for (int64_t v = 0; v < nv; v += nb) {
+        p.nv = std::min(nb, nv - v);
+        p.X = X + v * x_vs;
+        p.x_vec = x_vs % (1 << WhtCfg<T>::VB) == 0 && (uintptr_t)X % 16 == 0;
+        if (near && x_es == 1) {
+            RLA_TRY((launch_near<T, WHT_IN_X, WHT_OUT_W>(ctx, p)));
+        } else {
+            fjlt_pad_sign_kernel<T><<<tiles32(N, p.nv), dim3(32, 8), 0, ctx->stream>>>(p.X, x_es, x_vs, sk->L, N, p.nv,
+                                                                                      sk->signbits, p.W);
+            RLA_TRY(check_launch(ctx, "fjlt_pad_sign"));
+            if (near) {
+                RLA_TRY((launch_near<T, WHT_IN_W, WHT_OUT_W>(ctx, p)));
+            } else {
+                wht_short_kernel<T><<<(unsigned)std::min<int64_t>(p.nv, (int64_t)ctx->sm_count * 16), 256, N * sizeof(T),
+                                      ctx->stream>>>(p.W, N, p.nv);
+                RLA_TRY(check_launch(ctx, "wht_short"));
+            }
+        }
+        RLA_TRY(launch_far(ctx, p, false));
+        const int64_t octets = sk->s * ceil_div(p.nv, 4);
+        csr_gather_kernel<T><<<(unsigned)std::min<int64_t>(ceil_div(octets, 32), (int64_t)ctx->sm_count * 32), 256, 0,
+                               ctx->stream>>>(sk->k_ptr, sk->k_col, (const T *)sk->k_val, sk->s, p.W, N, p.nv,
+                                              Y + v * y_vs, y_es, y_vs, (T)(alpha * sk->scale), (T)beta, beta == 0.0);
+        RLA_TRY(check_launch(ctx, "fjlt_csr_gather"));
+    }
+    return RLA_OK;
 }
 
 template <class T>
 int fjlt_expand(rla_ctx *ctx, const rla_sketch *sk, const T *X, int64_t x_es, int64_t x_vs, int64_t nv, T *Y,
                 int64_t y_es, int64_t y_vs, double alpha, double beta) {
     if (nv == 0) return RLA_OK;
-    const int64_t N = sk->N;
+    const int64_t N = sk->N, nb = std::min<int64_t>(wht_batch<T>(N, nv), 65535 * 32);
     void *w;
-    RLA_TRY(scratch_get(ctx, (size_t)N * nv * sizeof(T), &w));
-    T *Wb = (T *)w;
-    const int grid = (int)std::min<int64_t>(ceil_div(N * nv, 256), (int64_t)ctx->sm_count * 32);
-    csr_t_gather_kernel<T><<<grid, 256, 0, ctx->stream>>>(sk->kt_ptr, sk->kt_row, (const T *)sk->kt_val, N, X, x_es,
-                                                          x_vs, nv, Wb);
-    RLA_TRY(check_launch(ctx, "fjlt_csr_t_gather"));
-    RLA_TRY(wht_full(ctx, Wb, N, nv));
-    const int grid2 = (int)std::min<int64_t>(ceil_div(sk->L * nv, 256), (int64_t)ctx->sm_count * 32);
-    fjlt_expand_out_kernel<T><<<grid2, 256, 0, ctx->stream>>>(Wb, N, sk->L, nv, sk->signbits, Y, y_es, y_vs,
-                                                              (T)(alpha * sk->scale), (T)beta, beta == 0.0);
-    return check_launch(ctx, "fjlt_expand_out");
+    RLA_TRY(scratch_get(ctx, (size_t)(N * nb) * sizeof(T), &w));
+    WhtParams<T> p = wht_params<T>(sk, nv);
+    p.x_es = x_es;
+    p.x_vs = x_vs;
+    p.ptr = sk->kt_ptr;
+    p.idx = sk->kt_row;
+    p.val = (const T *)sk->kt_val;
+    p.W = (T *)w;
+    p.y_es = y_es;
+    p.y_vs = y_vs;
+    p.alpha = (T)(alpha * sk->scale);
+    p.beta = (T)beta;
+    p.beta_zero = beta == 0.0;
+    for (int64_t v = 0; v < nv; v += nb) {
+        p.nv = std::min(nb, nv - v);
+        p.X = X + v * x_vs;
+        p.Y = Y + v * y_vs;
+        if (N < wht_near_min<T>()) {
+            const int grid = (int)std::min<int64_t>(ceil_div(N * p.nv, 256), (int64_t)ctx->sm_count * 32);
+            csr_t_gather_kernel<T><<<grid, 256, 0, ctx->stream>>>(p.ptr, p.idx, p.val, N, p.X, x_es, x_vs, p.nv, p.W);
+            RLA_TRY(check_launch(ctx, "fjlt_csr_t_gather"));
+            wht_short_kernel<T><<<(unsigned)std::min<int64_t>(p.nv, (int64_t)ctx->sm_count * 16), 256, N * sizeof(T),
+                                  ctx->stream>>>(p.W, N, p.nv);
+            RLA_TRY(check_launch(ctx, "wht_short"));
+            RLA_TRY(launch_out(ctx, p));
+            continue;
+        }
+        const bool far = p.log_n > WhtCfg<T>::CH, direct = y_es == 1;
+        if (!far && direct) {
+            RLA_TRY((launch_near<T, WHT_IN_KT, WHT_OUT_Y>(ctx, p)));
+            continue;
+        }
+        RLA_TRY((launch_near<T, WHT_IN_KT, WHT_OUT_W>(ctx, p)));
+        RLA_TRY(launch_far(ctx, p, direct));
+        if (!direct) RLA_TRY(launch_out(ctx, p));
+    }
+    return RLA_OK;
 }
 
 // ------------------------------------------------------------------------------------
@@ -783,14 +1232,7 @@ static int srht_noalloc_t(rla_ctx *ctx, const rla_sketch *sk, const T *X, int64_
     const int64_t L = sk->L, N = sk->N, s = sk->s;
     const T a = (T)(alpha * sk->scale);
     const bool beta_zero = beta == 0.0;
-    if (N < ((int64_t)1 << CH)) {
-        const size_t smem = (size_t)N * es;
-        set_smem_max(srht_small_kernel<T>);
-        const int grid = (int)std::min<int64_t>(nv, (int64_t)ctx->sm_count * 8);
-        srht_small_kernel<T><<<grid, 256, smem, ctx->stream>>>(X, ldx, L, N, nv, sk->signbits, sk->rows, s, Y, 1, ldy,
-                                                               a, (T)beta, beta_zero);
-        return check_launch(ctx, "srht_small(noalloc)");
-    }
+    if (N < ((int64_t)1 << CH)) return srht_short<T>(ctx, sk, X, ldx, nv, Y, 1, ldy, a, (T)beta, beta_zero);
     const int s_win = (int)std::min<int64_t>(s, srht_window<T>());
     const int64_t cpv = N >> CH, total = cpv * nv;
     int64_t W = std::min<int64_t>((int64_t)ctx->sm_count * 2, total);
