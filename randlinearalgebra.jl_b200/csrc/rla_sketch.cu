@@ -172,6 +172,10 @@ __global__ void __launch_bounds__(1024) sched_scan_kernel(const int32_t *nr, int
 // are distinct, and empty entries point at the lane's dummy slot.  flags[batch] is the
 // number of extra rounds, or TILE_SLOW when the batch needs run-time resolution (its words
 // then all point at bins).
+// More than MAX_DEFER of 512 elements repeat a bucket below about 2000 buckets, and the batch is
+// resolved at run time (1048576 x 256 Float32 to 1000: 3054 us): those sketches take the tile
+// kernel of rla_sparse_tile.cu.
+constexpr int CS_TILE_MAX_S = 2080;
 constexpr int CS_SCHED_WARPS = 4, CS_BATCH = 512, CS_XROUNDS = 2;
 
 __global__ void __launch_bounds__(CS_SCHED_WARPS * 32) cs_sched_kernel(const int32_t *bucket, const uint8_t *negative,
@@ -428,10 +432,12 @@ static int srht_tables(rla_ctx *ctx, rla_sketch *sk) {
 }
 
 static int build_meta(rla_ctx *ctx, rla_sketch *sk) {
-    // SparseSign: the tile kernel takes every layout.  CountSketch: it takes the strided vectors of
-    // a Right sketch (A*S on column-major A); contiguous ones keep the batch schedule below.
-    if (sk->nnz > 1 || sk->p.card == RLA_RIGHT) RLA_TRY(tile_plan_build(ctx, sk));
-    if (sk->bl_ok && sk->nnz > 1) return RLA_OK;
+    // SparseSign, and CountSketch with few buckets: the tile kernel takes every layout.  Other
+    // CountSketches: it takes the strided vectors of a Right sketch (A*S on column-major A);
+    // contiguous ones keep the batch schedule below.
+    const bool all = sk->nnz > 1 || sk->s <= CS_TILE_MAX_S;
+    if (all || sk->p.card == RLA_RIGHT) RLA_TRY(tile_plan_build(ctx, sk));
+    if (sk->bl_ok && all) return RLA_OK;
     if (sk->s > (1 << 22)) return RLA_OK;  // compression dimension beyond the packed form: strided/expand paths only
     if (!sk->meta)
         RLA_CUDA_TRY(ctx, cudaMalloc(&sk->meta, sizeof(uint32_t) * (size_t)ceil_div(sk->L, 128) * 128 * sk->nnz));

@@ -7,8 +7,8 @@
 // entry with 16-byte accesses: reading row j and adding to the bins of bucket b are then one
 // conflict-free wavefront each whatever j and b are, and a warp instruction serves four entries.
 // The entries of a chunk of R long indices are kept sorted by bucket (built when the sketch is
-// drawn) and cut into groups of four entries of one bucket, the last group of a bucket filled up
-// with a row of zeros: a step of the kernel adds one group per octet to its bucket, with no
+// drawn) and cut into groups of four entries of one bucket (of one, when buckets are sparse), the
+// last group of a bucket filled up with a row of zeros: a step of the kernel adds one group per octet to its bucket, with no
 // branches.  With e = R * nnz / s entries per bucket and chunk and g = ceil(e/4) groups,
 //   wavefronts per bucket and chunk = g * (4 rows + 2 bins + 1/4 words).
 // Measured (unprofiled call): 150001 -> 1332 (nnz 8) of 333 Float32 columns 257 us, 603 us with one
@@ -87,6 +87,7 @@ __device__ __forceinline__ uint32_t tile_off(int j, int c) {
 // ------------------------------------------------------------------------------------
 struct BlGeom {
     int nwin, sw, G, spw;  // windows, buckets per window, copies, keys (bucket copies) per warp
+    int gs;                // entries per group, 4 or 1
     int64_t nchunk, cap;   // cap: words reserved per chunk, a multiple of 16
 };
 
@@ -99,8 +100,11 @@ static bool bl_geometry(const rla_sketch *sk, BlGeom *g) {
         while (g->G < 16 && g->sw * g->G < 256 && (int64_t)BL_R * sk->nnz >= 8 * (int64_t)g->sw * g->G) g->G *= 2;
     g->spw = ceil_div_i((int64_t)g->sw * g->G, BL_WARPS);
     g->nchunk = ceil_div(sk->L, BL_R);
+    // Groups of four fill up with zero rows when buckets are sparse: at e = 2 they take as many
+    // wavefronts per entry (3.2) as single entries, each with its own bin update.
+    g->gs = (int64_t)BL_R * sk->nnz >= 2 * sk->s * g->G ? 4 : 1;
     const int64_t ne = (int64_t)BL_R * sk->nnz, keys = (int64_t)g->nwin * BL_WARPS * g->spw;
-    g->cap = (ne + 3 * std::min(ne, keys) + 15 * BL_WARPS * g->nwin + 15) / 16 * 16 + BL_SLACK;
+    g->cap = (ne + (g->gs - 1) * std::min(ne, keys) + 15 * BL_WARPS * g->nwin + 15) / 16 * 16 + BL_SLACK;
     return true;
 }
 
@@ -146,9 +150,10 @@ __global__ void __launch_bounds__(BL_BUILD_WARPS * 32) bl_build_kernel(const int
             __syncwarp();
             if (pass == 1 && valid) {
                 const uint32_t neg = (uint32_t)negative[base + i];
-                const int r = before + rank, k = koff[key] + r / 4, part = lpart[list];
+                const int r = before + rank, k = koff[key] + r / g.gs, part = lpart[list];
                 const int o = k / part, q = k - o * part;
-                out[lstart[list] + ((q * 4 + o) << 2) + (r & 3)] =
+                const int gpw = 4 / g.gs;  // groups per 16-byte word of an octet
+                out[lstart[list] + (((q / gpw) * 4 + o) << 2) + (q % gpw) * g.gs + r % g.gs] =
                     tile_off<T>(jl, 0) | ((uint32_t)(vlb * (BL_PITCH / 16)) << BL_BIN_SHIFT) | (neg << 31);
             }
         }
@@ -168,12 +173,12 @@ __global__ void __launch_bounds__(BL_BUILD_WARPS * 32) bl_build_kernel(const int
         for (int l = t; l < nlist; l += nt) {
             int run = 0, most = 0;
             for (int k = l * g.spw; k < (l + 1) * g.spw; ++k) {
-                const int ng = (tot[k] + 3) / 4;
+                const int ng = (tot[k] + g.gs - 1) / g.gs;
                 koff[k] = (uint16_t)run;
                 run += ng;
                 most = max(most, ng);
             }
-            const int part = (run + 3) / 4, slow = most > part;
+            const int gpw = 4 / g.gs, part = ((run + 3) / 4 + gpw - 1) / gpw * gpw, slow = most > part;
             lpart[l] = part;
             lslow[l] = slow;
         }
@@ -182,13 +187,13 @@ __global__ void __launch_bounds__(BL_BUILD_WARPS * 32) bl_build_kernel(const int
             int run = 0;
             for (int l = 0; l < nlist; ++l) {
                 lstart[l] = run;
-                run += 16 * lpart[l];
+                run += 4 * g.gs * lpart[l];
             }
         }
         __syncthreads();
         for (int l = t; l < nlist; l += nt)
-            lists[chunk * nlist + l] = make_int2(lstart[l] / 16, lpart[l] | (lslow[l] ? BL_SLOW : 0));
-        const int all = lstart[nlist - 1] + 16 * lpart[nlist - 1];
+            lists[chunk * nlist + l] = make_int2(lstart[l] / 16, lpart[l] * g.gs / 4 | (lslow[l] ? BL_SLOW : 0));
+        const int all = lstart[nlist - 1] + 4 * g.gs * lpart[nlist - 1];
         const uint32_t fill = BL_ZERO_ROW | ((uint32_t)(g.sw * g.G * (BL_PITCH / 16)) << BL_BIN_SHIFT);
         for (int i = t; i < all + BL_SLACK; i += nt) out[i] = fill;
         __syncthreads();
@@ -233,6 +238,19 @@ struct TileParams {
     Split split;  // over (tile, window, chunk), chunk fastest
 };
 
+// y +- x, 16 bytes per lane
+__device__ __forceinline__ float4 octet_add(float4 y, float4 x, uint32_t w) {
+    const float s = __uint_as_float((w & 0x80000000u) | 0x3f800000u);
+    const float2 s2 = make_float2(s, s);
+    const float2 lo = __ffma2_rn(make_float2(x.x, x.y), s2, make_float2(y.x, y.y));
+    const float2 hi = __ffma2_rn(make_float2(x.z, x.w), s2, make_float2(y.z, y.w));
+    return make_float4(lo.x, lo.y, hi.x, hi.y);
+}
+__device__ __forceinline__ double2 octet_add(double2 y, double2 x, uint32_t w) {
+    const long long m = (long long)(w & 0x80000000u) << 32;
+    return make_double2(y.x + __longlong_as_double(__double_as_longlong(x.x) ^ m),
+                        y.y + __longlong_as_double(__double_as_longlong(x.y) ^ m));
+}
 // +-x0 +-x1 +-x2 +-x3 + y, 16 bytes per lane
 __device__ __forceinline__ float4 octet_sum(float4 x0, float4 x1, float4 x2, float4 x3, uint4 w, float4 y) {
     auto sg = [](uint32_t u) {
@@ -289,7 +307,7 @@ __device__ __forceinline__ double ld_ahead(const double *a) {
 // with 16-byte aligned rows, strided vectors at any alignment.
 enum { TILE_CONTIG = 0, TILE_SHIFT = 1, TILE_ROWS = 2, TILE_ROWS_ANY = 3 };
 
-template <class T, int MODE>
+template <class T, int MODE, int GS>
 __global__ void __launch_bounds__(BL_WARPS * 32, 1) tile_compress_kernel(TileParams<T> p) {
     using V = typename TileVec<T>::type;
     constexpr int VR = TileCfg<T>::VR, C = TileCfg<T>::C, PE = BL_PITCH / (int)sizeof(T);
@@ -445,14 +463,31 @@ __global__ void __launch_bounds__(BL_WARPS * 32, 1) tile_compress_kernel(TilePar
                 for (int i = 0; i < BL_AHEAD; ++i) {
                     if (q + i >= nq) break;
                     const uint4 wc = w[i], wn = w[(i + 1) % BL_AHEAD];
-                    V *bp = bins_of(wc.x);
-                    V y = *bp;
-                    y = octet_sum(x0, x1, x2, x3, wc, y);
-                    x0 = row(wn.x);
-                    x1 = row(wn.y);
-                    x2 = row(wn.z);
-                    x3 = row(wn.w);
-                    *bp = y;
+                    if constexpr (GS == 4) {
+                        V *bp = bins_of(wc.x);
+                        V y = *bp;
+                        y = octet_sum(x0, x1, x2, x3, wc, y);
+                        x0 = row(wn.x);
+                        x1 = row(wn.y);
+                        x2 = row(wn.z);
+                        x3 = row(wn.w);
+                        *bp = y;
+                    } else {
+                        auto one = [&](V &x, uint32_t u, uint32_t un) {
+                            V *bp = bins_of(u);
+                            V y = *bp;
+                            y = octet_add(y, x, u);
+                            x = row(un);
+                            *bp = y;
+                        };
+                        one(x0, wc.x, wn.x);
+                        __syncwarp();
+                        one(x1, wc.y, wn.y);
+                        __syncwarp();
+                        one(x2, wc.z, wn.z);
+                        __syncwarp();
+                        one(x3, wc.w, wn.w);
+                    }
                     w[i] = __ldg(lp + 4 * i);
                     __syncwarp();  // orders these bin updates before the next step's
                 }
@@ -462,8 +497,17 @@ __global__ void __launch_bounds__(BL_WARPS * 32, 1) tile_compress_kernel(TilePar
                 const uint4 w = __ldg(lp);
                 for (int o = 0; o < 4; ++o) {
                     if ((lane >> 3) == o) {
-                        V *bp = bins_of(w.x);
-                        *bp = octet_sum(row(w.x), row(w.y), row(w.z), row(w.w), w, *bp);
+                        if constexpr (GS == 4) {
+                            V *bp = bins_of(w.x);
+                            *bp = octet_sum(row(w.x), row(w.y), row(w.z), row(w.w), w, *bp);
+                        } else {
+                            const uint32_t ws[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) {
+                                V *bp = bins_of(ws[i]);
+                                *bp = octet_add(*bp, row(ws[i]), ws[i]);
+                            }
+                        }
                     }
                     __syncwarp();
                 }
@@ -565,8 +609,12 @@ int tile_compress(rla_ctx *ctx, const rla_sketch *sk, const T *X, int64_t x_es, 
         kern<<<W, BL_WARPS * 32, smem, ctx->stream>>>(p);
         return check_launch(ctx, "tile_compress");
     };
-    if (contig) RLA_TRY(vec ? go(tile_compress_kernel<T, TILE_CONTIG>) : go(tile_compress_kernel<T, TILE_SHIFT>));
-    else RLA_TRY(vec ? go(tile_compress_kernel<T, TILE_ROWS>) : go(tile_compress_kernel<T, TILE_ROWS_ANY>));
+    auto by_mode = [&](auto gs) -> int {
+        constexpr int GS = decltype(gs)::value;
+        if (contig) return vec ? go(tile_compress_kernel<T, TILE_CONTIG, GS>) : go(tile_compress_kernel<T, TILE_SHIFT, GS>);
+        return vec ? go(tile_compress_kernel<T, TILE_ROWS, GS>) : go(tile_compress_kernel<T, TILE_ROWS_ANY, GS>);
+    };
+    RLA_TRY(g.gs == 4 ? by_mode(std::integral_constant<int, 4>()) : by_mode(std::integral_constant<int, 1>()));
     if (!shared) return RLA_OK;
     tile_reduce_kernel<T><<<dim3((unsigned)groups, ceil_div_i(g.sw, 32)), 256, 0, ctx->stream>>>(p);
     return check_launch(ctx, "tile_reduce");

@@ -89,3 +89,39 @@ def test_loaded_draws_with_repeated_buckets(rla, orc, dev):
     np.add.at(dense, (idx, np.repeat(np.arange(L), nnz)), vals)
     out = (S @ column_major(A, 0, dev)).cpu().numpy()
     assert rel_err(out, dense @ A) < TOL[np.float64]
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+def test_count_sketch_few_buckets(rla, orc, dev, dtype):
+    """CountSketch up to 2080 buckets: groups of four entries (dense buckets) and single ones."""
+    for L, s, nv, pad in [(1, 1, 1, 0), (639, 300, 33, 1), (5000, 319, 40, 0), (5000, 321, 40, 1), (20001, 1040, 31, 0),
+                          (20001, 1041, 33, 1), (7000, 2080, 17, 0), (3000, 2, 5, 1)]:
+        rng = np.random.default_rng([L, s])
+        A = rng.standard_normal((L, nv)).astype(dtype)
+        S = rla.complete_compressor(rla.CountSketch(compression_dim=s, type=dtype), A, seed=7)
+        ref = np.zeros((s, nv), order="F")
+        orc.mul_SA(ref, oracle_recipe(orc, S), A.astype(np.float64))
+        C = column_major(np.zeros((s, nv), dtype), pad, dev)
+        rla.mul_(C, S, column_major(A, pad, dev))
+        assert rel_err(C.cpu().numpy(), ref) < TOL[dtype], (L, s, nv)
+
+
+@pytest.mark.parametrize("nnz", [1, 8])
+@pytest.mark.parametrize("s", [40, 900])
+@pytest.mark.parametrize("used", [1, 3])
+def test_all_entries_in_few_buckets(rla, dev, nnz, s, used):
+    """Loaded draws that put every entry into one or three buckets: runs longer than an octet's
+    share, which the octets of a warp add one after another."""
+    rng = np.random.default_rng([nnz, s, used])
+    L, nv = 1500, 34
+    A = rng.standard_normal((L, nv))
+    comp = (rla.CountSketch(compression_dim=s, type=np.float64) if nnz == 1
+            else rla.SparseSign(compression_dim=s, nnz=nnz, type=np.float64))
+    S = rla.complete_compressor(comp, A, seed=2)
+    idx = 16 * rng.integers(0, used, L * nnz)
+    vals = np.where(rng.integers(0, 2, L * nnz) == 1, 1.0, -1.0) * (1.0 if nnz == 1 else 1.0 / np.sqrt(nnz))
+    S.load_draws(idx=idx, vals=vals)
+    dense = np.zeros((s, L))
+    np.add.at(dense, (idx, np.repeat(np.arange(L), nnz)), vals)
+    out = (S @ column_major(A, 0, dev)).cpu().numpy()
+    assert rel_err(out, dense @ A) < TOL[np.float64]
