@@ -67,6 +67,27 @@ int counters_get(rla_ctx *ctx, size_t n, int **out) {
     return RLA_OK;
 }
 
+bool scratch_ready(rla_ctx *ctx, size_t bytes) {
+    if (ctx->scratch.bytes >= ((bytes + 255) & ~size_t(255))) return true;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    return cudaStreamIsCapturing(ctx->stream, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone;
+}
+
+cudaError_t ctx_pool_create(rla_ctx *ctx) {
+    cudaMemPoolProps pp = {};
+    pp.allocType = cudaMemAllocationTypePinned;
+    pp.location.type = cudaMemLocationTypeDevice;
+    pp.location.id = ctx->device;
+    const cudaError_t e = cudaMemPoolCreate(&ctx->pool, &pp);
+    if (e != cudaSuccess) {
+        ctx->pool = nullptr;
+        return e;
+    }
+    uint64_t keep = UINT64_MAX;
+    cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    return cudaSuccess;
+}
+
 // Whether this thread has raised the kernel's shared-memory limit on the device; `set` records it.
 bool smem_max_raised(const void *kern, int device, bool set) {
     static thread_local std::vector<std::pair<const void *, int>> raised;
@@ -112,29 +133,20 @@ int rla_ctx_create(int device, void *stream, rla_ctx **out) {
         delete ctx;
         return RLA_E_CUDA;
     }
-    cudaDeviceProp prop;
-    if (cudaGetDeviceProperties(&prop, device) != cudaSuccess) {
+    // single attributes: cudaGetDeviceProperties takes milliseconds
+    int major = 0, sms = 0, optin = 0;
+    if (cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, device) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
+        cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device) != cudaSuccess) {
         delete ctx;
         return RLA_E_CUDA;
     }
-    if (prop.major < 10) {
+    if (major < 10) {
         delete ctx;
         return RLA_E_UNSUPPORTED;  // sm_100a kernels only
     }
-    {
-        cudaMemPoolProps pp = {};
-        pp.allocType = cudaMemAllocationTypePinned;
-        pp.location.type = cudaMemLocationTypeDevice;
-        pp.location.id = device;
-        if (cudaMemPoolCreate(&ctx->pool, &pp) != cudaSuccess) {
-            delete ctx;
-            return RLA_E_CUDA;
-        }
-        uint64_t keep = UINT64_MAX;
-        cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &keep);
-    }
-    ctx->sm_count = prop.multiProcessorCount;
-    ctx->smem_optin = (int)prop.sharedMemPerBlockOptin;
+    ctx->sm_count = sms;
+    ctx->smem_optin = optin;
     g_smem_optin = ctx->smem_optin;
     if (stream) {
         ctx->stream = (cudaStream_t)stream;
@@ -146,6 +158,7 @@ int rla_ctx_create(int device, void *stream, rla_ctx **out) {
         }
         ctx->owns_stream = true;
     }
+    pool_contexts(device, 1);
     *out = ctx;
     return RLA_OK;
 }
@@ -164,6 +177,7 @@ int rla_ctx_destroy(rla_ctx *ctx) {
         }
     if (ctx->owns_stream) cudaStreamDestroy(ctx->stream);
     if (ctx->pool) cudaMemPoolDestroy(ctx->pool);
+    pool_contexts(ctx->device, -1);
     delete ctx;
     return RLA_OK;
 }

@@ -98,10 +98,35 @@ inline cudaError_t set_smem_max(K kern) {
     if (e == cudaSuccess) smem_max_raised(reinterpret_cast<const void *>(kern), dev, true);
     return e;
 }
+// Memory of objects that outlive a call (sketches, solvers), from a pool of the device that is
+// shared by its contexts and keeps at most 256 MB of freed memory mapped (given back with the
+// last context): a cudaMalloc / cudaFree pair of a few MB takes 100-300 us, a solve on a new
+// problem makes twenty.  Allocated in the order of ctx->stream: other streams may use it once that
+// stream has been waited for.  dev_free: after the work that uses the memory has completed.
+cudaError_t dev_alloc(rla_ctx *ctx, void **p, size_t bytes);
+void dev_free(void *p);
+// Counts the device's contexts; the last one gives the pool's free memory back.
+void pool_contexts(int device, int change);
+template <class P>
+inline cudaError_t dev_alloc_t(rla_ctx *ctx, P **p, size_t bytes) {
+    return dev_alloc(ctx, reinterpret_cast<void **>(p), bytes);
+}
+// A pinned host slot of 64 bytes for a solver's status (cudaMallocHost takes as long as a solver's
+// iteration): 64 slots of one page, allocated on the first use; above, single allocations.
+cudaError_t pinned_slot(double **p);
+void pinned_slot_free(double *p);
+// False while ctx->stream captures a graph and the scratch would have to grow for `bytes`.
+bool scratch_ready(rla_ctx *ctx, size_t bytes);
+// The context's pool, made on its first use (a solver's private context needs none).
+cudaError_t ctx_pool_create(rla_ctx *ctx);
 // Stream-ordered allocation from the context's pool (memory stays mapped between calls, so
 // repeated calls of the same size do not remap device memory).
 template <class P>
 inline cudaError_t pool_malloc_s(rla_ctx *ctx, P **p, size_t bytes, cudaStream_t s) {
+    if (!ctx->pool) {
+        const cudaError_t e = ctx_pool_create(ctx);
+        if (e != cudaSuccess) return e;
+    }
     return cudaMallocFromPoolAsync(reinterpret_cast<void **>(p), bytes, ctx->pool, s);
 }
 

@@ -526,8 +526,8 @@ static int ihs_step_t(rla_ctx *ctx, rla_ihs *h, const T *A, int64_t lda, const T
 static void ihs_free(rla_ihs *h) {
     void *p[] = {h->SA, h->u, h->G, h->d, h->gd, h->g_part, h->e_part, h->stat, h->bad};
     for (void *q : p)
-        if (q) cudaFree(q);
-    if (h->hstat) cudaFreeHost(h->hstat);
+        dev_free(q);
+    pinned_slot_free(h->hstat);
     if (h->ev_apply) cudaEventDestroy(h->ev_apply);
     if (h->ev_draw) cudaEventDestroy(h->ev_draw);
     if (h->side) rla_ctx_destroy(h->side);
@@ -607,7 +607,7 @@ int rla_ihs_create(rla_ctx *ctx, rla_sketch *compressor, int dtype, int64_t m, i
     const int64_t eparts = std::max<int64_t>(h->nblk, ceil_div(m, 256));
     cudaError_t e = cudaSuccess;
     auto grab = [&](void **p, size_t bytes) {
-        if (e == cudaSuccess) e = cudaMalloc(p, std::max<size_t>(bytes, 16));
+        if (e == cudaSuccess) e = dev_alloc(ctx, p, bytes);
     };
     grab(&h->SA, (size_t)es * s * n);
     grab(&h->u, (size_t)es * n);
@@ -618,12 +618,13 @@ int rla_ihs_create(rla_ctx *ctx, rla_sketch *compressor, int dtype, int64_t m, i
     grab((void **)&h->e_part, sizeof(double) * eparts);
     grab((void **)&h->stat, sizeof(double) * 4);
     grab((void **)&h->bad, sizeof(int));
-    if (e == cudaSuccess) e = cudaMallocHost((void **)&h->hstat, sizeof(double) * 4);
+    if (e == cudaSuccess) e = pinned_slot(&h->hstat);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h->ev_apply, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h->ev_draw, cudaEventDisableTiming);
     if (e == cudaSuccess && rla_ctx_create(ctx->device, nullptr, &h->side) != RLA_OK) e = cudaErrorUnknown;
     if (e == cudaSuccess) e = cudaMemsetAsync(h->bad, 0, sizeof(int), ctx->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(h->u, 0, (size_t)es * n, ctx->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);  // the solver may be run on any stream
     if (e != cudaSuccess) {
         ihs_free(h);
         delete h;

@@ -1,0 +1,82 @@
+// rla_pool.cu -- memory of objects that outlive a call: a bounded device pool shared by the
+// contexts of a device, and pinned status slots.
+#include <mutex>
+
+#include "rla_internal.cuh"
+
+namespace rla {
+
+struct DevicePool {
+    cudaMemPool_t pool = nullptr;
+    int contexts = 0;
+};
+static std::mutex g_pool_mu;
+static DevicePool g_pool[64];
+
+cudaError_t dev_alloc(rla_ctx *ctx, void **p, size_t bytes) {
+    bytes = std::max<size_t>(bytes, 16);
+    cudaMemPool_t pool = nullptr;
+    if (ctx->device < 64) {
+        std::lock_guard<std::mutex> lock(g_pool_mu);
+        DevicePool &d = g_pool[ctx->device];
+        if (!d.pool) {
+            cudaMemPoolProps pp = {};
+            pp.allocType = cudaMemAllocationTypePinned;
+            pp.location.type = cudaMemLocationTypeDevice;
+            pp.location.id = ctx->device;
+            uint64_t keep = 256ull << 20;
+            if (cudaMemPoolCreate(&d.pool, &pp) == cudaSuccess)
+                cudaMemPoolSetAttribute(d.pool, cudaMemPoolAttrReleaseThreshold, &keep);
+            else
+                d.pool = nullptr;
+        }
+        pool = d.pool;
+    }
+    if (!pool) return cudaMalloc(p, bytes);
+    return cudaMallocFromPoolAsync(p, bytes, pool, ctx->stream);
+}
+
+void dev_free(void *p) {
+    if (p) cudaFreeAsync(p, nullptr);
+}
+
+static std::mutex g_slot_mu;
+static char *g_slots = nullptr;
+static uint64_t g_slots_used = 0;
+
+cudaError_t pinned_slot(double **p) {
+    std::lock_guard<std::mutex> lock(g_slot_mu);
+    if (!g_slots) {
+        const cudaError_t e = cudaHostAlloc((void **)&g_slots, 64 * 64, cudaHostAllocPortable);
+        if (e != cudaSuccess) {
+            g_slots = nullptr;
+            return e;
+        }
+    }
+    for (int i = 0; i < 64; ++i)
+        if (!((g_slots_used >> i) & 1u)) {
+            g_slots_used |= 1ull << i;
+            *p = (double *)(g_slots + 64 * i);
+            return cudaSuccess;
+        }
+    return cudaHostAlloc((void **)p, 64, cudaHostAllocPortable);
+}
+
+void pinned_slot_free(double *p) {
+    if (!p) return;
+    std::lock_guard<std::mutex> lock(g_slot_mu);
+    const ptrdiff_t off = (char *)p - g_slots;
+    if (g_slots && off >= 0 && off < 64 * 64) g_slots_used &= ~(1ull << (off / 64));
+    else cudaFreeHost(p);
+}
+
+// The device's last context gives the pool's free memory back.
+void pool_contexts(int device, int change) {
+    if (device >= 64) return;
+    std::lock_guard<std::mutex> lock(g_pool_mu);
+    DevicePool &d = g_pool[device];
+    d.contexts += change;
+    if (d.contexts == 0 && d.pool) cudaMemPoolTrimTo(d.pool, 0);
+}
+
+}  // namespace rla

@@ -147,8 +147,8 @@ namespace rla {
 static void proj_free(rla_proj *h) {
     void *p[] = {h->Y, h->Sb, h->uT, h->G, h->d, h->c, h->y, h->part, h->vec, h->stat, h->bad, h->skip};
     for (void *q : p)
-        if (q) cudaFree(q);
-    if (h->hstat) cudaFreeHost(h->hstat);
+        dev_free(q);
+    pinned_slot_free(h->hstat);
     if (h->ev_apply) cudaEventDestroy(h->ev_apply);
     if (h->ev_draw) cudaEventDestroy(h->ev_draw);
     if (h->side) rla_ctx_destroy(h->side);
@@ -299,7 +299,7 @@ int rla_proj_create(rla_ctx *ctx, rla_sketch *compressor, int kind, int dtype, i
     const size_t es = dtype == RLA_F32 ? 4 : 8;
     cudaError_t e = cudaSuccess;
     auto grab = [&](void **p, size_t bytes) {
-        if (e == cudaSuccess) e = cudaMalloc(p, std::max<size_t>(bytes, 16));
+        if (e == cudaSuccess) e = dev_alloc(ctx, p, bytes);
     };
     grab(&h->Y, es * (size_t)s * (kind == RLA_PROJ_KACZMARZ ? n : m));
     grab(&h->Sb, es * (size_t)s);
@@ -313,9 +313,10 @@ int rla_proj_create(rla_ctx *ctx, rla_sketch *compressor, int kind, int dtype, i
     grab((void **)&h->stat, sizeof(double) * 2);
     grab((void **)&h->bad, sizeof(int));
     grab((void **)&h->skip, sizeof(int));
-    if (e == cudaSuccess) e = cudaMallocHost((void **)&h->hstat, sizeof(double) * 2);
+    if (e == cudaSuccess) e = pinned_slot(&h->hstat);
     if (e == cudaSuccess) e = cudaMemsetAsync(h->bad, 0, sizeof(int), ctx->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(h->skip, 0, sizeof(int), ctx->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);  // the solver may be run on any stream
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h->ev_apply, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h->ev_draw, cudaEventDisableTiming);
     if (e == cudaSuccess && rla_ctx_create(ctx->device, nullptr, &h->side) != RLA_OK) e = cudaErrorUnknown;

@@ -826,11 +826,11 @@ int rla_sampling_create(rla_ctx *ctx, int card, int dtype, int64_t compression_d
     sk->s_replace = replace != 0;
     sk->s_beta = beta;
     sk->scale = 1.0;
-    cudaError_t e = cudaMalloc((void **)&sk->sidx, sizeof(int64_t) * sk->s);
-    if (e == cudaSuccess) e = cudaMalloc((void **)&sk->splan, sizeof(int64_t) * (3 * sk->s + 2));
-    if (e == cudaSuccess) e = cudaMalloc((void **)&sk->s_err, sizeof(int64_t));
+    cudaError_t e = dev_alloc_t(ctx, &sk->sidx, sizeof(int64_t) * sk->s);
+    if (e == cudaSuccess) e = dev_alloc_t(ctx, &sk->splan, sizeof(int64_t) * (3 * sk->s + 2));
+    if (e == cudaSuccess) e = dev_alloc_t(ctx, &sk->s_err, sizeof(int64_t));
     if (e == cudaSuccess) e = cudaMemsetAsync(sk->s_err, 0, sizeof(int64_t), ctx->stream);
-    if (e == cudaSuccess && distribution == RLA_DIST_L2NORM) e = cudaMalloc((void **)&sk->sweights, sizeof(double) * sk->L);
+    if (e == cudaSuccess && distribution == RLA_DIST_L2NORM) e = dev_alloc_t(ctx, &sk->sweights, sizeof(double) * sk->L);
     if (e == cudaSuccess) e = cudaMemsetAsync(sk->sidx, 0, sizeof(int64_t) * sk->s, ctx->stream);
     int rc = e == cudaSuccess ? RLA_OK : set_error(ctx, RLA_E_OOM, "%s", cudaGetErrorString(e));
     // Uniform draws at once; L2Norm and Agmon draw in rla_sampling_update (they need A)

@@ -423,8 +423,8 @@ static int srht_tables(rla_ctx *ctx, rla_sketch *sk) {
     std::vector<int32_t> fill(ptr.begin(), ptr.end() - 1);
     for (int64_t k = 0; k < s; ++k) list[fill[rows[k] & (ch - 1)]++] = (int32_t)k;
     for (int64_t q = 0; q < s; ++q) list[s + q] = rows[list[q]];
-    if (!sk->p2_ptr) RLA_CUDA_TRY(ctx, cudaMalloc(&sk->p2_ptr, sizeof(int32_t) * (ch + 1)));
-    if (!sk->p2_list) RLA_CUDA_TRY(ctx, cudaMalloc(&sk->p2_list, sizeof(int32_t) * 2 * s));
+    if (!sk->p2_ptr) RLA_CUDA_TRY(ctx, dev_alloc_t(ctx, &sk->p2_ptr, sizeof(int32_t) * (ch + 1)));
+    if (!sk->p2_list) RLA_CUDA_TRY(ctx, dev_alloc_t(ctx, &sk->p2_list, sizeof(int32_t) * 2 * s));
     RLA_CUDA_TRY(ctx, cudaMemcpyAsync(sk->p2_ptr, ptr.data(), sizeof(int32_t) * (ch + 1), cudaMemcpyHostToDevice, ctx->stream));
     RLA_CUDA_TRY(ctx, cudaMemcpyAsync(sk->p2_list, list.data(), sizeof(int32_t) * 2 * s, cudaMemcpyHostToDevice, ctx->stream));
     RLA_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
@@ -440,14 +440,14 @@ static int build_meta(rla_ctx *ctx, rla_sketch *sk) {
     if (sk->bl_ok && all) return RLA_OK;
     if (sk->s > (1 << 22)) return RLA_OK;  // compression dimension beyond the packed form: strided/expand paths only
     if (!sk->meta)
-        RLA_CUDA_TRY(ctx, cudaMalloc(&sk->meta, sizeof(uint32_t) * (size_t)ceil_div(sk->L, 128) * 128 * sk->nnz));
+        RLA_CUDA_TRY(ctx, dev_alloc_t(ctx, &sk->meta, sizeof(uint32_t) * (size_t)ceil_div(sk->L, 128) * 128 * sk->nnz));
     sk->batch_mode = (sk->nnz == 1 && sk->s <= 65536) ? 1 : 0;
     if (sk->batch_mode) {
         const int64_t nb = ceil_div(sk->L, CS_BATCH);
         const size_t bm_bytes = (size_t)CS_SCHED_WARPS * ceil_div(sk->s, 32) * 4;
-        if (!sk->tile_flags) RLA_CUDA_TRY(ctx, cudaMalloc(&sk->tile_flags, sizeof(uint32_t) * nb));
+        if (!sk->tile_flags) RLA_CUDA_TRY(ctx, dev_alloc_t(ctx, &sk->tile_flags, sizeof(uint32_t) * nb));
         if (!sk->extra) {
-            RLA_CUDA_TRY(ctx, cudaMalloc(&sk->extra, sizeof(uint32_t) * 64 * nb));
+            RLA_CUDA_TRY(ctx, dev_alloc_t(ctx, &sk->extra, sizeof(uint32_t) * 64 * nb));
             sk->extra_rounds_cap = 2 * nb;
         }
         if (bm_bytes > 48 * 1024)
@@ -473,10 +473,10 @@ static int build_meta(rla_ctx *ctx, rla_sketch *sk) {
         if (sk->extra_rounds_cap < cap) {
             if (sk->extra) RLA_CUDA_TRY(ctx, cudaFree(sk->extra));
             sk->extra = nullptr;
-            RLA_CUDA_TRY(ctx, cudaMalloc(&sk->extra, sizeof(uint32_t) * 32 * cap));
+            RLA_CUDA_TRY(ctx, dev_alloc_t(ctx, &sk->extra, sizeof(uint32_t) * 32 * cap));
             sk->extra_rounds_cap = cap;
         }
-        if (!sk->tile_flags) RLA_CUDA_TRY(ctx, cudaMalloc(&sk->tile_flags, sizeof(uint32_t) * std::max<int64_t>(ntile, 1)));
+        if (!sk->tile_flags) RLA_CUDA_TRY(ctx, dev_alloc_t(ctx, &sk->tile_flags, sizeof(uint32_t) * std::max<int64_t>(ntile, 1)));
         sched_scan_kernel<<<1, 1024, 0, ctx->stream>>>(nr, ntile, base);
         RLA_TRY(check_launch(ctx, "sched_scan"));
         sparse_sched_kernel<1><<<blocks, SCHED_WARPS * 32, 0, ctx->stream>>>(
@@ -501,9 +501,9 @@ static int build_meta(rla_ctx *ctx, rla_sketch *sk) {
         if (sk->extra) RLA_CUDA_TRY(ctx, cudaFree(sk->extra));
         sk->extra = nullptr;
         sk->extra_rounds_cap = std::max<int64_t>(tot, 1) + tot / 4;
-        RLA_CUDA_TRY(ctx, cudaMalloc(&sk->extra, sizeof(uint32_t) * 32 * sk->extra_rounds_cap));
+        RLA_CUDA_TRY(ctx, dev_alloc_t(ctx, &sk->extra, sizeof(uint32_t) * 32 * sk->extra_rounds_cap));
     }
-    if (!sk->tile_flags) RLA_CUDA_TRY(ctx, cudaMalloc(&sk->tile_flags, sizeof(uint32_t) * std::max<int64_t>(ntile, 1)));
+    if (!sk->tile_flags) RLA_CUDA_TRY(ctx, dev_alloc_t(ctx, &sk->tile_flags, sizeof(uint32_t) * std::max<int64_t>(ntile, 1)));
     RLA_CUDA_TRY(ctx, cudaMemcpyAsync(base, hb.data(), sizeof(int64_t) * ntile, cudaMemcpyHostToDevice, ctx->stream));
     sparse_sched_kernel<1><<<blocks, SCHED_WARPS * 32, 0, ctx->stream>>>(sk->bucket, sk->negative, sk->L, (int)sk->nnz,
                                                                          sk->meta, nr, base, sk->tile_flags, sk->extra);
@@ -586,8 +586,7 @@ static void free_sketch_buffers(rla_sketch *sk) {
     void *ptrs[] = {sk->bucket, sk->negative, sk->meta, sk->rows, sk->signbits, sk->sign_tl, sk->tile_flags, sk->extra, sk->p2_ptr, sk->p2_list,
                     sk->k_ptr, sk->k_col, sk->k_val, sk->kt_ptr, sk->kt_row, sk->kt_val, sk->dense,
                     sk->sidx, sk->splan, sk->sweights, sk->s_err, sk->tp_ptr, sk->tp_idx, sk->bl_words, sk->bl_lists};
-    for (void *p : ptrs)
-        if (p) cudaFree(p);
+    for (void *p : ptrs) dev_free(p);
 }
 
 }  // namespace rla
@@ -638,8 +637,8 @@ int rla_sketch_create(rla_ctx *ctx, const rla_sketch_params *pp, rla_sketch **ou
     int rc = RLA_OK;
     auto alloc = [&](void **ptr, size_t bytes) {
         if (rc != RLA_OK) return;
-        cudaError_t e = cudaMalloc(ptr, std::max<size_t>(bytes, 16));
-        if (e != cudaSuccess) rc = set_error(ctx, RLA_E_OOM, "cudaMalloc(%zu) failed: %s", bytes, cudaGetErrorString(e));
+        cudaError_t e = dev_alloc(ctx, ptr, bytes);
+        if (e != cudaSuccess) rc = set_error(ctx, RLA_E_OOM, "allocating %zu bytes failed: %s", bytes, cudaGetErrorString(e));
     };
     switch (p.kind) {
         case RLA_SPARSE_SIGN:
@@ -873,9 +872,9 @@ int rla_sketch_set_draws(rla_ctx *ctx, rla_sketch *sk, const int64_t *idx, const
             if (sk->k_val) cudaFree(sk->k_val);
             sk->k_ptr = sk->k_col = nullptr;
             sk->k_val = nullptr;
-            RLA_CUDA_TRY(ctx, cudaMalloc(&sk->k_ptr, (sk->s + 1) * 4));
-            RLA_CUDA_TRY(ctx, cudaMalloc(&sk->k_col, std::max<int64_t>(k_nnz, 1) * 4));
-            RLA_CUDA_TRY(ctx, cudaMalloc(&sk->k_val, std::max<int64_t>(k_nnz, 1) * es));
+            RLA_CUDA_TRY(ctx, dev_alloc_t(ctx, &sk->k_ptr, (sk->s + 1) * 4));
+            RLA_CUDA_TRY(ctx, dev_alloc_t(ctx, &sk->k_col, std::max<int64_t>(k_nnz, 1) * 4));
+            RLA_CUDA_TRY(ctx, dev_alloc_t(ctx, &sk->k_val, std::max<int64_t>(k_nnz, 1) * es));
             RLA_CUDA_TRY(ctx, cudaMemcpy(sk->k_ptr, cp.data(), (sk->s + 1) * 4, cudaMemcpyHostToDevice));
             if (k_nnz) {
                 RLA_CUDA_TRY(ctx, cudaMemcpy(sk->k_col, cc.data(), k_nnz * 4, cudaMemcpyHostToDevice));

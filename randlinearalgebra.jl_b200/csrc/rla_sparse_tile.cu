@@ -205,8 +205,8 @@ int tile_plan_build(rla_ctx *ctx, rla_sketch *sk) {
     sk->bl_ok = false;
     if (!bl_geometry(sk, &g)) return RLA_OK;
     const int nlist = g.nwin * BL_WARPS, K = nlist * g.spw;
-    if (!sk->bl_words) RLA_CUDA_TRY(ctx, cudaMalloc(&sk->bl_words, sizeof(uint32_t) * (size_t)(g.nchunk * g.cap)));
-    if (!sk->bl_lists) RLA_CUDA_TRY(ctx, cudaMalloc(&sk->bl_lists, sizeof(int2) * (size_t)(g.nchunk * nlist)));
+    if (!sk->bl_words) RLA_CUDA_TRY(ctx, dev_alloc_t(ctx, &sk->bl_words, sizeof(uint32_t) * (size_t)(g.nchunk * g.cap)));
+    if (!sk->bl_lists) RLA_CUDA_TRY(ctx, dev_alloc_t(ctx, &sk->bl_lists, sizeof(int2) * (size_t)(g.nchunk * nlist)));
     const size_t smem = sizeof(uint16_t) * (size_t)K * (BL_BUILD_WARPS + 2);
     auto go = [&](auto kern) -> int {
         RLA_CUDA_TRY(ctx, set_smem_max(kern));
@@ -236,6 +236,7 @@ struct TileParams {
     int beta_zero;
     T *partials;  // [slot][sw][C]
     Split split;  // over (tile, window, chunk), chunk fastest
+    int64_t unit;  // chunks per split unit: 1, or all of a (tile, window) when no partial sums are kept
 };
 
 // y +- x, 16 bytes per lane
@@ -317,7 +318,7 @@ __global__ void __launch_bounds__(BL_WARPS * 32, 1) tile_compress_kernel(TilePar
     const int t = threadIdx.x, lane = t & 31, wp = t >> 5, l8 = lane & 7;
     const uint32_t lane16 = (uint32_t)l8 << 4;
     const int64_t nchunk = p.g.nchunk;
-    const int64_t u0 = p.split.start(blockIdx.x), u1 = p.split.start(blockIdx.x + 1);
+    const int64_t u0 = p.split.start(blockIdx.x) * p.unit, u1 = p.split.start(blockIdx.x + 1) * p.unit;
     if (u0 >= u1) return;
     auto zero_bins = [&]() {
         for (int i = t; i < (p.g.sw * p.g.G + 1) * (BL_PITCH / 16); i += BL_WARPS * 32) reinterpret_cast<V *>(bin_raw)[i] = V{};
@@ -594,13 +595,17 @@ int tile_compress(rla_ctx *ctx, const rla_sketch *sk, const T *X, int64_t x_es, 
     BlGeom g;
     if (!sk->bl_ok || !bl_geometry(sk, &g)) return set_error(ctx, RLA_E_UNSUPPORTED, "no bucket lists for this sketch");
     const int64_t groups = ceil_div(nv, C) * g.nwin, units = groups * g.nchunk;
-    const int W = (int)std::min<int64_t>(ctx->sm_count, units);
+    int W = (int)std::min<int64_t>(ctx->sm_count, units);
     void *part = nullptr;
-    const bool shared = W > 1 && g.nchunk > 1;
-    if (shared) RLA_TRY(scratch_get(ctx, (size_t)(2 * W) * g.sw * C * sizeof(T), &part));
+    const size_t part_bytes = (size_t)(2 * W) * g.sw * C * sizeof(T);
+    // no partial sums when each CTA has whole (tile, window)s, also in a graph capture that finds
+    // the scratch too small
+    const bool shared = W > 1 && g.nchunk > 1 && scratch_ready(ctx, part_bytes);
+    if (shared) RLA_TRY(scratch_get(ctx, part_bytes, &part));
+    else W = (int)std::min<int64_t>(ctx->sm_count, groups);
     const bool contig = x_es == 1;
     TileParams<T> p{X, contig ? x_vs : x_es, sk->L, nv, sk->s, sk->bl_words, sk->bl_lists, g, Y, y_es, y_vs,
-                    alpha, beta, beta_zero, (T *)part, Split::make(units, W)};
+                    alpha, beta, beta_zero, (T *)part, Split::make(shared ? units : groups, W), shared ? 1 : g.nchunk};
     const size_t smem = (size_t)BL_TILE_BYTES + (size_t)(g.sw * g.G + 1) * BL_PITCH;
     const bool aligned = (nv == 1 && contig) || p.x_ld % VR == 0;
     const bool vec = aligned && (uintptr_t)X % 16 == 0;

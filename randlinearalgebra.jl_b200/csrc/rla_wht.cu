@@ -452,7 +452,7 @@ int build_srht_sign_table(rla_ctx *ctx, rla_sketch *sk) {
     if (sk->N < ((int64_t)1 << CH)) return RLA_OK;
     const int64_t nchunks = sk->N >> CH;
     const size_t bytes = (f32 ? sizeof(WhtCfg<float>::SignW) : sizeof(WhtCfg<double>::SignW)) * nchunks * NT;
-    if (!sk->sign_tl) RLA_CUDA_TRY(ctx, cudaMalloc(&sk->sign_tl, bytes));
+    if (!sk->sign_tl) RLA_CUDA_TRY(ctx, dev_alloc_t(ctx, &sk->sign_tl, bytes));
     const int64_t n = nchunks * NT;
     if (f32)
         sign_table_kernel<float><<<ceil_div_i(n, 256), 256, 0, ctx->stream>>>(
@@ -1086,8 +1086,9 @@ int srht_expand(rla_ctx *ctx, const rla_sketch *sk, const T *X, int64_t x_es, in
     p.alpha = a;
     p.beta = (T)beta;
     p.beta_zero = beta == 0.0;
-    if (y_es == 1) return launch_near<T, WHT_IN_SAMPLES, WHT_OUT_Y>(ctx, p);
     const int64_t nb = std::min<int64_t>(wht_batch<T>(sk->N, nv), 65535 * 32);
+    if (y_es == 1 || !scratch_ready(ctx, (size_t)(sk->N * nb) * sizeof(T)))
+        return launch_near<T, WHT_IN_SAMPLES, WHT_OUT_Y>(ctx, p);
     void *w;
     RLA_TRY(scratch_get(ctx, (size_t)(sk->N * nb) * sizeof(T), &w));
     p.W = (T *)w;
