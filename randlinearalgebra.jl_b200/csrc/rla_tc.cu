@@ -28,6 +28,7 @@
 #include "rla_internal.cuh"
 #include "rla_kernels.cuh"
 #include "rla_tc.cuh"
+#include "rla_tc_ptx.cuh"
 
 namespace rla {
 
@@ -35,16 +36,6 @@ namespace rla {
 // FP32 -> NT BF16 terms; element (r, c) of X at X[r + c*ldx], outputs at [r + c*ldo]
 // (or, transposed, at [c + r*ldo])
 // ------------------------------------------------------------------------------------
-template <int NT>
-__device__ __forceinline__ void split_terms(float v, bf16 (&t)[NT]) {
-    float rem = v;
-#pragma unroll
-    for (int q = 0; q < NT; ++q) {
-        t[q] = __float2bfloat16_rn(rem);
-        rem -= __bfloat162float(t[q]);
-    }
-}
-
 template <int NT>
 __global__ void split_terms_kernel(const float *__restrict__ X, int64_t rows, int64_t cols, int64_t ldx, bf16 *o0,
                                    bf16 *o1, bf16 *o2, int64_t ldo, int vec) {
@@ -144,112 +135,9 @@ int split_bf16(rla_ctx *ctx, const float *X, int64_t rows, int64_t cols, int64_t
 }
 
 // ------------------------------------------------------------------------------------
-// PTX wrappers (sm_100a)
-// ------------------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-__device__ __forceinline__ uint64_t global_ns() {
-    uint64_t t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-// Wait for the phase of parity `parity` to complete; gives up after limit_ns (and 2^26
-// polls) or once another CTA has recorded a failure, records the failure in *status and
-// returns false.
-__device__ __noinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int *status, uint64_t limit_ns) {
-    if (mbar_try(bar, parity)) return true;
-    const uint64_t t0 = global_ns();
-    for (uint32_t it = 0; it < (1u << 26) && limit_ns > 0; ++it) {
-        if (mbar_try(bar, parity)) return true;
-        if ((it & 63u) == 0u && (global_ns() - t0 > limit_ns || *(volatile int *)status != 0)) break;
-    }
-    atomicExch(status, 1);
-    return false;
-}
-
-// Drain wait before a CTA releases its shared memory or tensor memory: waits for copies or
-// MMAs already issued, whatever the pipeline limit, for at most 2 s (and 2^26 polls).
-constexpr uint64_t TC_DRAIN_NS = 2000000000ull;
-__device__ __noinline__ bool mbar_drain(uint32_t bar, uint32_t parity, int *status) {
-    const uint64_t t0 = global_ns();
-    for (uint32_t it = 0; it < (1u << 26); ++it) {
-        if (mbar_try(bar, parity)) return true;
-        if ((it & 63u) == 0u && global_ns() - t0 > TC_DRAIN_NS) break;
-    }
-    atomicExch(status, 2);
-    return false;
-}
-
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map, uint32_t bar, int x, int y) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(dst),
-        "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(x), "r"(y)
-        : "memory");
-}
-
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-
-__device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accum) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accum)
-        : "memory");
-}
-__device__ __forceinline__ void mma_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
-        "%15}, [%16];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-        : "r"(taddr));
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
-
-// Shared-memory matrix descriptor, 64-byte swizzle (Blackwell descriptor version 1).
-__device__ __forceinline__ uint64_t sdesc_sw64(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
-    uint64_t d = (uint64_t)((saddr >> 4) & 0x3FFFu);
-    d |= (uint64_t)((lbo >> 4) & 0x3FFFu) << 16;
-    d |= (uint64_t)((sbo >> 4) & 0x3FFFu) << 32;
-    d |= (uint64_t)1 << 46;
-    d |= (uint64_t)4 << 61;
-    return d;
-}
-
-// Instruction descriptor of kind::f16 with BF16 inputs and an FP32 accumulator.
-__host__ __device__ constexpr uint32_t idesc_bf16(int M, int N, int a_mn_major, int b_mn_major) {
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)a_mn_major << 15) | ((uint32_t)b_mn_major << 16) |
-           ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
-}
-
-// ------------------------------------------------------------------------------------
 // GEMM kernel
 // ------------------------------------------------------------------------------------
-constexpr int TC_BM = 128, TC_BK = 32, TC_THREADS = 128;
-constexpr uint32_t TC_A_BYTES = TC_BM * TC_BK * 2;  // 8 KB per operand term
+constexpr int TC_THREADS = 128;
 
 // Tensor maps of the NT BF16 terms of both operands.
 template <int NT>
@@ -853,7 +741,7 @@ static PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
 
 // 2-D BF16 map over a column-major array: inner dimension `inner` (contiguous), outer
 // dimension `outer` with stride ld elements; 64-byte swizzle, zero fill outside.
-static int make_map(rla_ctx *ctx, CUtensorMap *map, const bf16 *ptr, int64_t inner, int64_t outer, int64_t ld,
+int tc_make_map(rla_ctx *ctx, CUtensorMap *map, const bf16 *ptr, int64_t inner, int64_t outer, int64_t ld,
                     uint32_t box_inner, uint32_t box_outer) {
     auto fn = encode_fn();
     if (!fn) return set_error(ctx, RLA_E_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
@@ -952,11 +840,11 @@ int tc_gemm_split(rla_ctx *ctx, int64_t M, int64_t N, int64_t K, const bf16 *con
         TcMaps<NT> maps;
         const uint32_t box_n = (uint32_t)(NT == 2 ? pl.main_cols : pl.BN / pl.nch);
         for (int t = 0; t < NT; ++t) {
-            if (a_kmajor) RLA_TRY(make_map(ctx, &maps.a[t], A[t], K, M, lda, TC_BK, TC_BM));
-            else RLA_TRY(make_map(ctx, &maps.a[t], A[t], M, K, lda, 32, TC_BK));
-            if (box_n) RLA_TRY(make_map(ctx, &maps.b[t], B[t] + n0 * ldb, K, nb, ldb, TC_BK, box_n));
+            if (a_kmajor) RLA_TRY(tc_make_map(ctx, &maps.a[t], A[t], K, M, lda, TC_BK, TC_BM));
+            else RLA_TRY(tc_make_map(ctx, &maps.a[t], A[t], M, K, lda, 32, TC_BK));
+            if (box_n) RLA_TRY(tc_make_map(ctx, &maps.b[t], B[t] + n0 * ldb, K, nb, ldb, TC_BK, box_n));
             if (NT == 2 && pl.rem_cols)
-                RLA_TRY(make_map(ctx, &maps.b_rem[t], B[t] + n0 * ldb, K, nb, ldb, TC_BK, (uint32_t)pl.rem_cols));
+                RLA_TRY(tc_make_map(ctx, &maps.b_rem[t], B[t] + n0 * ldb, K, nb, ldb, TC_BK, (uint32_t)pl.rem_cols));
         }
         TC *Cn = C + n0 * ldc;
         const bool direct = pl.splits == 1 && std::is_same<TC, float>::value && alpha == 1.0 && beta == 0.0;
@@ -1038,9 +926,9 @@ int tc_group_build(rla_ctx *ctx, const std::vector<TcGroupSpec> &specs, TcGroup 
             return set_error(ctx, RLA_E_UNSUPPORTED, "grouped tensor-core product: shape %lld x %lld x %lld",
                              (long long)sp.M, (long long)sp.N, (long long)sp.K);
         for (int t = 0; t < NT; ++t) {
-            if (sp.a_kmajor) RLA_TRY(make_map(ctx, &it.a[t], sp.a[t], sp.K, sp.M, sp.lda, TC_BK, TC_BM));
-            else RLA_TRY(make_map(ctx, &it.a[t], sp.a[t], sp.M, sp.K, sp.lda, 32, TC_BK));
-            RLA_TRY(make_map(ctx, &it.b[t], sp.b[t], sp.K, sp.N, sp.ldb, TC_BK, TC64_BN));
+            if (sp.a_kmajor) RLA_TRY(tc_make_map(ctx, &it.a[t], sp.a[t], sp.K, sp.M, sp.lda, TC_BK, TC_BM));
+            else RLA_TRY(tc_make_map(ctx, &it.a[t], sp.a[t], sp.M, sp.K, sp.lda, 32, TC_BK));
+            RLA_TRY(tc_make_map(ctx, &it.b[t], sp.b[t], sp.K, sp.N, sp.ldb, TC_BK, TC64_BN));
         }
         it.M = (int)sp.M;
         it.N = (int)sp.N;
@@ -1159,9 +1047,9 @@ int tc_gemm_f64acc(rla_ctx *ctx, int64_t M, int64_t N, int64_t K, const bf16 *co
     splits = ceil_div(nkb, kbps);
     TcMaps<NT> maps;
     for (int t = 0; t < NT; ++t) {
-        if (a_kmajor) RLA_TRY(make_map(ctx, &maps.a[t], A[t], K, M, lda, TC_BK, TC_BM));
-        else RLA_TRY(make_map(ctx, &maps.a[t], A[t], M, K, lda, 32, TC_BK));
-        RLA_TRY(make_map(ctx, &maps.b[t], B[t], K, N, ldb, TC_BK, TC64_BN));
+        if (a_kmajor) RLA_TRY(tc_make_map(ctx, &maps.a[t], A[t], K, M, lda, TC_BK, TC_BM));
+        else RLA_TRY(tc_make_map(ctx, &maps.a[t], A[t], M, K, lda, 32, TC_BK));
+        RLA_TRY(tc_make_map(ctx, &maps.b[t], B[t], K, N, ldb, TC_BK, TC64_BN));
     }
     const int64_t ldo = M, sstride = M * N;
     void *ws = nullptr;
@@ -1187,7 +1075,7 @@ int tc_gemm_f64acc(rla_ctx *ctx, int64_t M, int64_t N, int64_t K, const bf16 *co
 // A or A' (both layouts are read by TMA); op(B) must be K-major for the MMA, so B' (tb = 1)
 // is transposed while it is split.  The split copies come from the context's memory pool.
 template <class TC>
-int gemm_f32_tc(rla_ctx *ctx, int64_t M, int64_t N, int64_t K, const float *A, int64_t lda, int ta, const float *B,
+int gemm_f32_tc_presplit(rla_ctx *ctx, int64_t M, int64_t N, int64_t K, const float *A, int64_t lda, int ta, const float *B,
                 int64_t ldb, int tb, TC *C, int64_t ldc, double alpha, double beta) {
     if (M <= 0 || N <= 0) return RLA_OK;
     if (K <= 0) return gemm<float, float, TC, double>(ctx, M, N, K, A, lda, ta, B, ldb, tb, C, ldc, alpha, beta);
@@ -1209,10 +1097,14 @@ int gemm_f32_tc(rla_ctx *ctx, int64_t M, int64_t N, int64_t K, const float *A, i
     return rc;
 }
 
-template int gemm_f32_tc<float>(rla_ctx *, int64_t, int64_t, int64_t, const float *, int64_t, int, const float *,
-                                int64_t, int, float *, int64_t, double, double);
-template int gemm_f32_tc<double>(rla_ctx *, int64_t, int64_t, int64_t, const float *, int64_t, int, const float *,
-                                 int64_t, int, double *, int64_t, double, double);
+template int gemm_f32_tc_presplit<float>(rla_ctx *, int64_t, int64_t, int64_t, const float *, int64_t, int, const float *,
+                                        int64_t, int, float *, int64_t, double, double);
+template int gemm_f32_tc_presplit<double>(rla_ctx *, int64_t, int64_t, int64_t, const float *, int64_t, int, const float *,
+                                         int64_t, int, double *, int64_t, double, double);
+template int tc_gemm_f64acc<float>(rla_ctx *, int64_t, int64_t, int64_t, const bf16 *const *, int64_t, int, const bf16 *const *,
+                                   int64_t, float *, int64_t, double, double);
+template int tc_gemm_f64acc<double>(rla_ctx *, int64_t, int64_t, int64_t, const bf16 *const *, int64_t, int,
+                                    const bf16 *const *, int64_t, double *, int64_t, double, double);
 
 }  // namespace rla
 

@@ -56,6 +56,11 @@ template <class TC>
 int gemm_f32_tc(rla_ctx *ctx, int64_t M, int64_t N, int64_t K, const float *A, int64_t lda, int ta, const float *B,
                 int64_t ldb, int tb, TC *C, int64_t ldc, double alpha, double beta);
 
+// The same product with both operands split into BF16 terms in memory beforehand.
+template <class TC>
+int gemm_f32_tc_presplit(rla_ctx *ctx, int64_t M, int64_t N, int64_t K, const float *A, int64_t lda, int ta, const float *B,
+                         int64_t ldb, int tb, TC *C, int64_t ldc, double alpha, double beta);
+
 // C = alpha * op(A) * B + beta * C from three BF16 terms per operand (K-major B), FP64
 // accumulation across chunks of four k-blocks.  Asynchronous.
 template <class TC>

@@ -1,0 +1,401 @@
+// rla_tc_conv.cu -- FP32-accurate tensor-core products whose large operand is split into BF16 terms
+// inside the kernel.
+//
+// C = alpha * op(A) * B + beta * C with NT BF16 terms per operand (t0 = bf16(x), t1 = bf16(x - t0),
+// ...) and FP64 accumulation across chunks of four k-blocks, the products and their order as in
+// tc_gemm_f64acc_kernel (rla_tc.cu).  There the terms of A come from HBM: splitting reads 4 bytes
+// and writes 2 NT per element, and the product reads the 2 NT again.  Here four converter warps
+// copy A's Float32 tile ahead with cp.async (4 k-blocks of 16 KB in flight), turn it into the
+// terms and store them where TMA would have put them (64-byte swizzle), so A is read once, at any
+// alignment.  B, the small operand, is split beforehand and loaded by TMA.
+//
+// Warps: 0 TMA producer of B, 1 MMA issuer, 2 TMEM allocator, 4..11 chunk drain / epilogue (lane
+// quarter by warp mod 4, 32 of the 64 columns each), 12..15 converters.  A tile is 128 x 64.
+// Bound by the converters' chain per k-block (copy, convert, store, proxy fence, arrive; four warps):
+// the tensor pipe is 17 % and the ALU pipe 24 % busy at 65536 x 1024 x 128.
+#include "rla_internal.cuh"
+#include "rla_kernels.cuh"
+#include "rla_tc.cuh"
+#include "rla_tc_ptx.cuh"
+
+namespace rla {
+
+constexpr int CV_THREADS = 512, CV_BN = 64, CV_CHUNK = 4, CV_RAW = 4, CV_EPI_WARPS = 8;
+constexpr uint32_t CV_RAW_BYTES = TC_BM * TC_BK * 4;  // 16 KB per k-block of A
+constexpr uint32_t CV_B_BYTES = CV_BN * TC_BK * 2;
+constexpr uint32_t cv_tmem_cols(int NT) { return NT >= 3 ? 512u : (NT == 2 ? 256u : 128u); }
+constexpr uint32_t cv_stage_bytes(int NT) { return NT * (TC_A_BYTES + CV_B_BYTES); }
+
+struct ConvArgs {
+    const float *A;  // a_kmajor: element (m, k) at A[k + m*lda]; else at A[m + k*lda]
+    int64_t lda;
+    int a_vec;       // every 8-element group of A starts on 16 bytes
+    int M, N, K;
+    void *out, *out2;  // element (m, n) at out[m*rs + n*cs]; out2 (optional) likewise
+    int64_t rs, cs;
+    int out_f64;
+    double alpha, beta;  // beta: read and scaled when beta_on
+    int beta_on;
+    int stages;
+    int *status;
+    uint64_t wait_ns;
+};
+
+__device__ __forceinline__ void cp_async_zfill(uint32_t dst, const void *src, int bytes) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void cp_async4_zfill(uint32_t dst, const void *src, int bytes) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+
+// Converter thread t of 128: four groups of 8 elements of each k-block, in the order in which
+// consecutive lanes read consecutive memory.  A group's raw values stay private to the thread,
+// so waiting for its own copies is enough.
+template <int NT, int AK>
+__device__ __forceinline__ void conv_warps(const ConvArgs &p, int t, uint32_t base, uint32_t raw, unsigned char *raw_gen,
+                                           unsigned char *stage_gen, int m0, int kb0, int nkb, uint32_t empty0,
+                                           uint32_t afull0) {
+    const int lane = t & 31, c = t & 3;
+    auto issue = [&](int kb) {
+        if (kb < nkb) {
+            const int k0 = (kb0 + kb) * TC_BK;
+            const uint32_t slot = raw + (uint32_t)(kb % CV_RAW) * CV_RAW_BYTES + (uint32_t)t * 16u;
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int m = AK ? m0 + u * 32 + (t >> 2) : m0 + 32 * u + 8 * c;
+                const int k = AK ? k0 + 8 * c : k0 + (t >> 2);
+                const int valid = AK ? (m < p.M ? min(8, p.K - k) : 0) : (k < p.K ? min(8, p.M - m) : 0);
+                const float *src = valid > 0 ? p.A + (AK ? k + (int64_t)m * p.lda : m + (int64_t)k * p.lda) : p.A;
+                const uint32_t d = slot + (uint32_t)u * 4096u;
+                if (p.a_vec) {
+                    cp_async_zfill(d, src, 4 * max(0, min(4, valid)));
+                    cp_async_zfill(d + 2048u, valid > 4 ? src + 4 : src, 4 * max(0, valid - 4));
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 8; ++i)
+                        cp_async4_zfill(d + (uint32_t)(i >> 2) * 2048u + (uint32_t)(i & 3) * 4u, i < valid ? src + i : src,
+                                        i < valid ? 4 : 0);
+                }
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+#pragma unroll
+    for (int i = 0; i < CV_RAW - 1; ++i) issue(i);
+    for (int kb = 0; kb < nkb; ++kb) {
+        issue(kb + CV_RAW - 1);
+        const int s = kb % p.stages;
+        const uint32_t ph = (uint32_t)(kb / p.stages) & 1u;
+        if (!__all_sync(FULL, mbar_wait(empty0 + 8u * (uint32_t)s, ph ^ 1u, p.status, p.wait_ns))) break;
+        asm volatile("cp.async.wait_group %0;" ::"n"(CV_RAW - 1) : "memory");
+        const unsigned char *slot = raw_gen + (size_t)(kb % CV_RAW) * CV_RAW_BYTES + t * 16;
+        unsigned char *st = stage_gen + (size_t)s * cv_stage_bytes(NT);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const float4 a = *reinterpret_cast<const float4 *>(slot + u * 4096);
+            const float4 b = *reinterpret_cast<const float4 *>(slot + u * 4096 + 2048);
+            const float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+            uint4 o[NT];
+            split_terms8<NT>(v, o);
+            const int row = AK ? u * 32 + (t >> 2) : t >> 2;  // 64-byte row of the tile (of box u when not K-major)
+            const uint32_t off = (AK ? 0u : (uint32_t)u * 2048u) + (uint32_t)row * 64u + (uint32_t)((c ^ ((row >> 1) & 3)) << 4);
+#pragma unroll
+            for (int q = 0; q < NT; ++q)
+                *reinterpret_cast<uint4 *>(st + (size_t)q * TC_A_BYTES + off) = o[q];
+        }
+        // the MMAs read the tile through the async proxy
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(afull0 + 8u * (uint32_t)s) : "memory");
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+}
+
+// The 128 x 64 tile (m0, n0) over k-blocks kb0 .. kb0 + nkb - 1.
+template <int NT>
+__device__ __forceinline__ void conv_cta(const CUtensorMap *mb, const ConvArgs &p, int a_kmajor, int m0, int n0, int kb0,
+                                         int nkb) {
+    extern __shared__ unsigned char smem_raw[];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t raw0 = smem_u32(smem_raw);
+    const uint32_t base = (raw0 + 1023u) & ~1023u;
+    unsigned char *gen = smem_raw + (base - raw0);
+    const uint32_t ring = base + (uint32_t)p.stages * cv_stage_bytes(NT);
+    const uint32_t bars = ring + CV_RAW * CV_RAW_BYTES;
+    const uint32_t afull0 = bars, bfull0 = bars + 64u, empty0 = bars + 128u;  // up to 8 stages each
+    auto accf_bar = [&](int x) { return bars + 192u + 8u * (uint32_t)x; };
+    auto acce_bar = [&](int x) { return bars + 208u + 8u * (uint32_t)x; };
+    const uint32_t done_bar = bars + 224u, tmem_slot = bars + 232u;
+    volatile uint32_t *tmem_slot_ptr = reinterpret_cast<volatile uint32_t *>(gen + (tmem_slot - base));
+    const int nchunks = (nkb + CV_CHUNK - 1) / CV_CHUNK;
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < p.stages; ++s) {
+            mbar_init(afull0 + 8u * s, 4);
+            mbar_init(bfull0 + 8u * s, 1);
+            mbar_init(empty0 + 8u * s, 1);
+        }
+        for (int x = 0; x < 2; ++x) {
+            mbar_init(accf_bar(x), 1);
+            mbar_init(acce_bar(x), CV_EPI_WARPS);
+        }
+        mbar_init(done_bar, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+#pragma unroll
+        for (int q = 0; q < NT; ++q)
+            asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(mb + q)) : "memory");
+    }
+    if (warp == 2) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tmem_slot),
+                     "r"(cv_tmem_cols(NT))
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *tmem_slot_ptr;
+
+    if (warp == 0) {
+        if (lane == 0) {
+            int issued = 0;
+            for (int kb = 0; kb < nkb; ++kb) {
+                const int s = kb % p.stages;
+                const uint32_t ph = (uint32_t)(kb / p.stages) & 1u;
+                if (!mbar_wait(empty0 + 8u * s, ph ^ 1u, p.status, p.wait_ns)) break;
+                issued = kb + 1;
+                const uint32_t b0 = base + (uint32_t)s * cv_stage_bytes(NT) + NT * TC_A_BYTES;
+                mbar_arrive_expect_tx(bfull0 + 8u * s, NT * CV_B_BYTES);
+#pragma unroll
+                for (int t = 0; t < NT; ++t)
+                    tma_load_2d(b0 + (uint32_t)t * CV_B_BYTES, mb + t, bfull0 + 8u * s, (kb0 + kb) * TC_BK, n0);
+            }
+            for (int kb = max(0, issued - p.stages); kb < issued; ++kb)
+                mbar_drain(bfull0 + 8u * (kb % p.stages), (uint32_t)(kb / p.stages) & 1u, p.status);
+        }
+        __syncwarp();
+    } else if (warp == 1) {
+        if (lane == 0) {
+            // chunk c accumulates into TMEM columns (c & 1) * 64 NT; A_t x [B_0 | .. | B_(NT-1-t)] is
+            // one MMA, column group u collects the products with B_u
+            const uint32_t a_mn = a_kmajor ? 0 : 1;
+            const uint32_t idesc_n[3] = {idesc_bf16(TC_BM, CV_BN * NT, a_mn, 0),
+                                         idesc_bf16(TC_BM, CV_BN * (NT >= 2 ? NT - 1 : 1), a_mn, 0),
+                                         idesc_bf16(TC_BM, CV_BN * (NT >= 3 ? NT - 2 : 1), a_mn, 0)};
+            for (int kb = 0; kb < nkb; ++kb) {
+                const int c = kb / CV_CHUNK, x = c & 1;
+                const bool first = kb % CV_CHUNK == 0;
+                if (first) {
+                    if (!mbar_wait(acce_bar(x), ((uint32_t)(c >> 1) & 1u) ^ 1u, p.status, p.wait_ns)) break;
+                    tc_fence_after();
+                }
+                const int s = kb % p.stages;
+                const uint32_t ph = (uint32_t)(kb / p.stages) & 1u;
+                if (!mbar_wait(bfull0 + 8u * s, ph, p.status, p.wait_ns)) break;
+                if (!mbar_wait(afull0 + 8u * s, ph, p.status, p.wait_ns)) break;
+                tc_fence_after();
+                const uint32_t st = base + (uint32_t)s * cv_stage_bytes(NT);
+                const uint32_t d = tmem + (uint32_t)x * CV_BN * NT;
+#pragma unroll
+                for (int kk = 0; kk < TC_BK / 16; ++kk) {
+                    const uint64_t db = sdesc_sw64(st + NT * TC_A_BYTES + kk * 32u, 16u, 512u);  // from B_0 on
+#pragma unroll
+                    for (int t = 0; t < NT; ++t) {
+                        const uint32_t a_t = st + (uint32_t)t * TC_A_BYTES;
+                        const uint64_t da = a_kmajor ? sdesc_sw64(a_t + kk * 32u, 16u, 512u)
+                                                     : sdesc_sw64(a_t + kk * 1024u, 2048u, 512u);
+                        mma_bf16(d, da, db, idesc_n[t], (first && kk == 0 && t == 0) ? 0u : 1u);
+                    }
+                }
+                mma_commit(empty0 + 8u * s);
+                if (kb % CV_CHUNK == CV_CHUNK - 1 || kb == nkb - 1) mma_commit(accf_bar(x));
+            }
+            mma_commit(done_bar);
+        }
+        __syncwarp();
+    } else if (warp >= 4 && warp < 4 + CV_EPI_WARPS) {
+        // ---- chunk drain: FP64 sums of 32 rows (TMEM lane quarter) and 32 columns ----
+        const int q = warp & 3, h = (warp - 4) >> 2;
+        double acc[CV_BN / 2];
+#pragma unroll
+        for (int j = 0; j < CV_BN / 2; ++j) acc[j] = 0.0;
+        bool ok = true;
+        for (int c = 0; c < nchunks; ++c) {
+            const int x = c & 1;
+            ok = __all_sync(FULL, mbar_wait(accf_bar(x), (uint32_t)(c >> 1) & 1u, p.status, p.wait_ns));
+            if (!ok) break;
+            tc_fence_after();
+#pragma unroll
+            for (int c0 = 0; c0 < CV_BN / 2; c0 += 16) {
+#pragma unroll
+                for (int u = 0; u < NT; ++u) {
+                    uint32_t r[16];
+                    tmem_ld16(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(x * CV_BN * NT + u * CV_BN + h * (CV_BN / 2) + c0), r);
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) acc[c0 + j] += (double)__uint_as_float(r[j]);
+                }
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(acce_bar(x)) : "memory");
+        }
+        const int row = m0 + q * 32 + lane, col0 = n0 + h * (CV_BN / 2);
+        if (row < p.M) {
+#pragma unroll
+            for (int j = 0; j < CV_BN / 2; ++j) {
+                if (col0 + j >= p.N) break;
+                const int64_t o = row * p.rs + (int64_t)(col0 + j) * p.cs;
+                double v = ok ? p.alpha * acc[j] : 0.0;
+                if (p.out_f64) {
+                    double *y = (double *)p.out + o;
+                    if (p.beta_on) v += p.beta * *y;
+                    *y = v;
+                    if (p.out2) ((double *)p.out2)[o] = v;
+                } else {
+                    float *y = (float *)p.out + o;
+                    if (p.beta_on) v += p.beta * (double)*y;
+                    *y = (float)v;
+                    if (p.out2) ((float *)p.out2)[o] = (float)v;
+                }
+            }
+        }
+    } else if (warp >= 4 + CV_EPI_WARPS) {
+        const int t = threadIdx.x - 32 * (4 + CV_EPI_WARPS);
+        unsigned char *ring_gen = gen + (ring - base);
+        if (a_kmajor) conv_warps<NT, 1>(p, t, base, ring, ring_gen, gen, m0, kb0, nkb, empty0, afull0);
+        else conv_warps<NT, 0>(p, t, base, ring, ring_gen, gen, m0, kb0, nkb, empty0, afull0);
+    }
+    // every MMA issued (done_bar is committed on every path) has finished before the
+    // accumulators are released
+    if (threadIdx.x == 64) mbar_drain(done_bar, 0u, p.status);
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 2)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(cv_tmem_cols(NT)) : "memory");
+}
+
+template <int NT>
+struct ConvMaps {
+    CUtensorMap b[NT];
+};
+
+// CTA (tile, split): tiles with the N index fastest, so that the CTAs that share rows of A run
+// together; split z writes its FP64 partial tile at out + z * stride.
+template <int NT>
+__global__ void __launch_bounds__(CV_THREADS, 1)
+conv_gemm_kernel(const __grid_constant__ ConvMaps<NT> maps, ConvArgs p, int a_kmajor, int ntl, int nkb, int kbps,
+                 int64_t stride) {
+    const int tile = blockIdx.x, kb0 = blockIdx.y * kbps;
+    if (blockIdx.y) p.out = (double *)p.out + (int64_t)blockIdx.y * stride;
+    conv_cta<NT>(maps.b, p, a_kmajor, (tile / ntl) * TC_BM, (tile % ntl) * CV_BN, kb0, max(0, min(nkb - kb0, kbps)));
+}
+
+// C(m, n) (at C[m*rs + n*cs]) = alpha * sum_s P[s](m, n) + beta * C(m, n), P(m, n) at [m + n*M], splits
+// added in order, through 32 x 32 tiles so that both sides are read and written along memory.
+template <class TC>
+__global__ void __launch_bounds__(256) conv_reduce_kernel(const double *P, int splits, int64_t stride, int64_t M, int64_t N,
+                                                          TC *C, int64_t rs, int64_t cs, double alpha, double beta,
+                                                          int beta_on) {
+    __shared__ double tile[32][33];
+    const int64_t tn = (N + 31) / 32, m0 = blockIdx.x / tn * 32, n0 = blockIdx.x % tn * 32;
+    const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const int64_t m = m0 + x, n = n0 + y + 8 * q;
+        double a = 0.0;
+        if (m < M && n < N)
+            for (int s = 0; s < splits; ++s) a += P[s * stride + m + n * M];
+        tile[x][y + 8 * q] = a;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const int i = rs == 1 ? x : y + 8 * q, j = rs == 1 ? y + 8 * q : x;
+        if (m0 + i >= M || n0 + j >= N) continue;
+        TC *c = C + (m0 + i) * rs + (n0 + j) * cs;
+        double v = alpha * tile[i][j];
+        if (beta_on) v += beta * (double)*c;
+        *c = (TC)v;
+    }
+}
+
+// C (M x N, ld ldc, TC) = alpha * op(A) * op(B) + beta * C for Float32 A and B (an FP32-accurate
+// product).  The operand with more elements is converted in the kernel; when that is B, the
+// transposed product is computed and written with its strides exchanged.  The other one is split
+// beforehand into K-major terms in the context's memory pool.  Gaussian A * Omega, A 65536 x 1024,
+// Omega 1024 x 128: 304 us a call, 394 us with both operands split in memory.
+template <class TC>
+int gemm_f32_tc(rla_ctx *ctx, int64_t M, int64_t N, int64_t K, const float *A, int64_t lda, int ta, const float *B,
+                int64_t ldb, int tb, TC *C, int64_t ldc, double alpha, double beta) {
+    constexpr int NT = 3;
+    if (M <= 0 || N <= 0) return RLA_OK;
+    if (K <= 0) return gemm<float, float, TC, double>(ctx, M, N, K, A, lda, ta, B, ldb, tb, C, ldc, alpha, beta);
+    if (M >= (1ll << 31) || K >= (1ll << 31) || N >= (1ll << 31))
+        return set_error(ctx, RLA_E_UNSUPPORTED, "tensor-core GEMM: dimension above 2^31");
+    // every tile of 64 columns converts its 128 rows of A again: above four of them splitting A once in
+    // memory is faster (16000 x 512 to 1000 rows: 389 us converting, 363 us split before), unless K is
+    // so short that the FP64 partial tiles of the other kernel cost more (25756 x 4057, K = 131: 1170
+    // against 1426 us)
+    if (std::min(M, N) > 4 * CV_BN && K > 256)
+        return gemm_f32_tc_presplit<TC>(ctx, M, N, K, A, lda, ta, B, ldb, tb, C, ldc, alpha, beta);
+    int64_t rs = 1, cs = ldc;
+    if (N > M) {  // C' = op(B)' op(A)'
+        std::swap(M, N);
+        std::swap(A, B);
+        std::swap(lda, ldb);
+        const int t = ta;
+        ta = !tb;
+        tb = !t;
+        std::swap(rs, cs);
+    }
+    const int64_t mt = ceil_div(M, TC_BM), ntl = ceil_div(N, CV_BN), nkb = ceil_div(K, TC_BK);
+    if (mt * ntl >= (1ll << 31)) return set_error(ctx, RLA_E_UNSUPPORTED, "tensor-core GEMM: grid too large");
+    int *status = nullptr;
+    RLA_TRY(tc_status_get(ctx, &status));
+    const int64_t budget = ctx->smem_optin - 1024 - 256 - (int64_t)CV_RAW * CV_RAW_BYTES;
+    const int stages = (int)std::min<int64_t>(4, budget / cv_stage_bytes(NT));
+    const size_t smem = 1024 + 256 + (size_t)stages * cv_stage_bytes(NT) + CV_RAW * CV_RAW_BYTES;
+    // split K until the grid covers the GPU, keeping whole chunks per split
+    const int64_t tiles = mt * ntl;
+    int64_t splits = 1;
+    if (tiles < ctx->sm_count)
+        splits = std::min<int64_t>(ceil_div(ctx->sm_count, tiles), std::max<int64_t>(1, nkb / (2 * CV_CHUNK)));
+    const int64_t kbps = ceil_div(ceil_div(nkb, splits), CV_CHUNK) * CV_CHUNK;
+    splits = ceil_div(nkb, kbps);
+    void *ws = nullptr;
+    if (splits > 1) RLA_TRY(scratch_get(ctx, sizeof(double) * (size_t)(M * N * splits), &ws));
+    const int64_t ldb2 = ceil_div(K, 8) * 8;
+    const size_t nb = (size_t)ldb2 * N;
+    bf16 *buf = nullptr;
+    RLA_CUDA_TRY(ctx, pool_malloc_s(ctx, (void **)&buf, sizeof(bf16) * 3 * nb + 256, ctx->stream));
+    bf16 *b3[3] = {buf, buf + nb, buf + 2 * nb};
+    int rc = tb ? split_terms_launch<NT>(ctx, B, N, K, ldb, 1, b3, ldb2) : split_terms_launch<NT>(ctx, B, K, N, ldb, 0, b3, ldb2);
+    ConvMaps<NT> maps;
+    for (int t = 0; t < NT && rc == RLA_OK; ++t) rc = tc_make_map(ctx, &maps.b[t], b3[t], K, N, ldb2, TC_BK, CV_BN);
+    auto launch = [&]() -> int {
+        const bool part = splits > 1;
+        ConvArgs p{A, lda, lda % 4 == 0 && (uintptr_t)A % 16 == 0, (int)M, (int)N, (int)K,
+                   part ? ws : (void *)C, nullptr, part ? 1 : rs, part ? M : cs, part || sizeof(TC) == 8,
+                   part ? 1.0 : alpha, beta, !part && beta != 0.0, stages, status, ctx->wait_ns};
+        RLA_CUDA_TRY(ctx, set_smem_max(conv_gemm_kernel<NT>));
+        cudaEvent_t e0 = timing_begin(ctx);
+        conv_gemm_kernel<NT><<<dim3((unsigned)tiles, (unsigned)splits), CV_THREADS, smem, ctx->stream>>>(
+            maps, p, ta, (int)ntl, (int)nkb, (int)kbps, M * N);
+        RLA_TRY(check_launch(ctx, "conv_gemm"));
+        timing_end(ctx, 0, e0);
+        if (!part) return RLA_OK;
+        conv_reduce_kernel<TC><<<(unsigned)(ceil_div(M, 32) * ceil_div(N, 32)), 256, 0, ctx->stream>>>(
+            (const double *)ws, (int)splits, M * N, M, N, C, rs, cs, alpha, beta, beta != 0.0);
+        return check_launch(ctx, "conv_reduce");
+    };
+    if (rc == RLA_OK) rc = launch();
+    cudaFreeAsync(buf, ctx->stream);
+    return rc;
+}
+
+template int gemm_f32_tc<float>(rla_ctx *, int64_t, int64_t, int64_t, const float *, int64_t, int, const float *,
+                                int64_t, int, float *, int64_t, double, double);
+template int gemm_f32_tc<double>(rla_ctx *, int64_t, int64_t, int64_t, const float *, int64_t, int, const float *,
+                                 int64_t, int, double *, int64_t, double, double);
+
+}  // namespace rla
