@@ -626,6 +626,7 @@ int rla_ihs_create(rla_ctx *ctx, rla_sketch *compressor, int dtype, int64_t m, i
     if (e == cudaSuccess) e = cudaMemsetAsync(h->u, 0, (size_t)es * n, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);  // the solver may be run on any stream
     if (e != cudaSuccess) {
+        cudaStreamSynchronize(ctx->stream);  // memsets may be queued on the buffers
         ihs_free(h);
         delete h;
         return set_error(ctx, e == cudaErrorMemoryAllocation ? RLA_E_OOM : RLA_E_CUDA, "%s", cudaGetErrorString(e));

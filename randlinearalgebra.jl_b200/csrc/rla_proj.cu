@@ -321,6 +321,7 @@ int rla_proj_create(rla_ctx *ctx, rla_sketch *compressor, int kind, int dtype, i
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h->ev_draw, cudaEventDisableTiming);
     if (e == cudaSuccess && rla_ctx_create(ctx->device, nullptr, &h->side) != RLA_OK) e = cudaErrorUnknown;
     if (e != cudaSuccess) {
+        cudaStreamSynchronize(ctx->stream);  // memsets may be queued on the buffers
         proj_free(h);
         delete h;
         return set_error(ctx, e == cudaErrorMemoryAllocation ? RLA_E_OOM : RLA_E_CUDA, "%s", cudaGetErrorString(e));

@@ -683,6 +683,7 @@ int rla_sketch_create(rla_ctx *ctx, const rla_sketch_params *pp, rla_sketch **ou
     }
     if (rc == RLA_OK) rc = draw(ctx, sk);
     if (rc != RLA_OK) {
+        cudaStreamSynchronize(ctx->stream);  // kernels of the draw may be queued on the buffers
         free_sketch_buffers(sk);
         delete sk;
         return rc;

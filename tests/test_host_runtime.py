@@ -1,0 +1,82 @@
+"""Order of the library's host calls, on a fake CUDA runtime (fake_cuda.py; CPU only): device memory
+that outlives a call comes from a pool shared by all contexts of a device, so it may be given back
+only when no queued work can still touch it."""
+import ctypes
+
+import pytest
+
+from fake_cuda import F32, LEFT, RIGHT, fake, i64, vp  # noqa: F401 (fixture)
+
+IHS, KACZMARZ, COLUMN = "ihs", 0, 1
+
+
+def freed_while_queued(log):
+    """Releases that are not ordered behind work queued before them: freed on the legacy stream (or
+    with cudaFree, which does not wait for pool memory) with no wait for the stream since that work."""
+    pending, bad = set(), []
+    for line in log:
+        call, *rest = line.split()
+        stream = next((r[7:] for r in rest if r.startswith("stream=")), None)
+        if call == "launch" or call in ("cudaMemsetAsync", "cudaMemcpyAsync"):
+            pending.add(stream)
+        elif call == "cudaStreamSynchronize":
+            pending.discard(stream)
+        elif call == "cudaDeviceSynchronize":
+            pending.clear()
+        elif call == "cudaFree" or (call == "cudaFreeAsync" and stream == "(nil)"):
+            if pending:
+                bad.append(line)
+    return bad
+
+
+def test_check_sees_a_planted_release():
+    log = ["launch k grid=1 stream=0x10", "cudaFreeAsync 0x5 stream=(nil)"]
+    assert freed_while_queued(log) == log[1:]
+    assert freed_while_queued([log[0], "cudaStreamSynchronize stream=0x10", log[1]]) == []
+    assert freed_while_queued([log[0], "cudaStreamSynchronize stream=0x20", log[1]]) == log[1:]
+    assert freed_while_queued([log[0], "cudaFreeAsync 0x5 stream=0x10"]) == []
+
+
+@pytest.mark.parametrize("kind,nnz", [("sparse_sign", 8), ("count_sketch", 1), ("srht", 1), ("fjlt", 1), ("gaussian", 1)])
+@pytest.mark.parametrize("call", ["cudaMallocFromPoolAsync", "cudaMallocAsync", "launch"])
+def test_failed_sketch_creation_waits_for_its_draws(fake, kind, nnz, call):
+    """Whatever call of the creation fails, the buffers go back after the work queued on them."""
+    ctx = fake.context()
+    failed = 0
+    for ok in range(12):
+        fake.reset()
+        fake.fail_after(call, ok)
+        rc, sk = fake.create(ctx, kind, 40, 3000, nnz=nnz, card=RIGHT)
+        if rc:
+            failed += 1
+            assert freed_while_queued(fake.log()) == [], (call, ok)
+        else:
+            fake.lib.rla_sketch_destroy(sk)
+    assert failed or call == "cudaMallocAsync"
+    fake.lib.rla_ctx_destroy(ctx)
+
+
+@pytest.mark.parametrize("solver", [IHS, KACZMARZ, COLUMN])
+@pytest.mark.parametrize("call", ["cudaMallocFromPoolAsync", "cudaMemsetAsync", "cudaEventCreateWithFlags",
+                                  "cudaStreamCreateWithFlags"])
+def test_failed_solver_creation_waits_for_its_memsets(fake, solver, call):
+    ctx = fake.context()
+    sk = fake.sketch(ctx, "sparse_sign", 64, 500 if solver != COLUMN else 20, nnz=4, card=LEFT if solver != COLUMN else RIGHT)
+    failed = 0
+    for ok in range(14):
+        fake.reset()
+        fake.fail_after(call, ok)
+        h = vp()
+        if solver == IHS:
+            rc = fake.lib.rla_ihs_create(ctx, sk, F32, i64(500), i64(20), ctypes.c_double(1.0), ctypes.byref(h))
+        else:
+            rc = fake.lib.rla_proj_create(ctx, sk, solver, F32, i64(500), i64(20), ctypes.c_double(1.0),
+                                          ctypes.byref(h))
+        if rc:
+            failed += 1
+            assert freed_while_queued(fake.log()) == [], (call, ok)
+        else:
+            (fake.lib.rla_ihs_destroy if solver == IHS else fake.lib.rla_proj_destroy)(h)
+    assert failed
+    fake.lib.rla_sketch_destroy(sk)
+    fake.lib.rla_ctx_destroy(ctx)
