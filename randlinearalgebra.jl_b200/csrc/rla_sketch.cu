@@ -470,9 +470,7 @@ static int build_meta(rla_ctx *ctx, rla_sketch *sk) {
         // the schedule never needs more than SS_MAX_XROUNDS rounds per tile: size `extra` for
         // that once and scan the counts on the device, so a redraw waits on nothing
         const int64_t cap = std::max<int64_t>(ntile * SS_MAX_XROUNDS, 1);
-        if (sk->extra_rounds_cap < cap) {
-            if (sk->extra) RLA_CUDA_TRY(ctx, cudaFree(sk->extra));
-            sk->extra = nullptr;
+        if (!sk->extra) {
             RLA_CUDA_TRY(ctx, dev_alloc_t(ctx, &sk->extra, sizeof(uint32_t) * 32 * cap));
             sk->extra_rounds_cap = cap;
         }
@@ -498,10 +496,13 @@ static int build_meta(rla_ctx *ctx, rla_sketch *sk) {
     // a tile flag holds the tile's first extra round in bits 8..30
     if (tot >= (int64_t(1) << 23)) return set_error(ctx, RLA_E_UNSUPPORTED, "too many deferred rounds");
     if (tot > sk->extra_rounds_cap) {
-        if (sk->extra) RLA_CUDA_TRY(ctx, cudaFree(sk->extra));
+        // in stream order (cudaFree would return pool memory without waiting for its readers)
+        if (sk->extra) RLA_CUDA_TRY(ctx, cudaFreeAsync(sk->extra, ctx->stream));
         sk->extra = nullptr;
-        sk->extra_rounds_cap = std::max<int64_t>(tot, 1) + tot / 4;
-        RLA_CUDA_TRY(ctx, dev_alloc_t(ctx, &sk->extra, sizeof(uint32_t) * 32 * sk->extra_rounds_cap));
+        sk->extra_rounds_cap = 0;
+        const int64_t cap = std::max<int64_t>(tot, 1) + tot / 4;
+        RLA_CUDA_TRY(ctx, dev_alloc_t(ctx, &sk->extra, sizeof(uint32_t) * 32 * cap));
+        sk->extra_rounds_cap = cap;
     }
     if (!sk->tile_flags) RLA_CUDA_TRY(ctx, dev_alloc_t(ctx, &sk->tile_flags, sizeof(uint32_t) * std::max<int64_t>(ntile, 1)));
     RLA_CUDA_TRY(ctx, cudaMemcpyAsync(base, hb.data(), sizeof(int64_t) * ntile, cudaMemcpyHostToDevice, ctx->stream));
@@ -868,19 +869,22 @@ int rla_sketch_set_draws(rla_ctx *ctx, rla_sketch *sk, const int64_t *idx, const
                         memcpy(cv.data() + d * es, (const char *)vals + k * es, es);
                     }
             }
-            if (sk->k_ptr) cudaFree(sk->k_ptr);
-            if (sk->k_col) cudaFree(sk->k_col);
-            if (sk->k_val) cudaFree(sk->k_val);
+            // released, allocated and filled in the order of ctx->stream, once nothing on the device
+            // reads the old matrix (cudaFree would return pool memory without waiting)
+            RLA_CUDA_TRY(ctx, cudaDeviceSynchronize());
+            for (void *p : {(void *)sk->k_ptr, (void *)sk->k_col, (void *)sk->k_val})
+                if (p) cudaFreeAsync(p, ctx->stream);
             sk->k_ptr = sk->k_col = nullptr;
             sk->k_val = nullptr;
             RLA_CUDA_TRY(ctx, dev_alloc_t(ctx, &sk->k_ptr, (sk->s + 1) * 4));
             RLA_CUDA_TRY(ctx, dev_alloc_t(ctx, &sk->k_col, std::max<int64_t>(k_nnz, 1) * 4));
             RLA_CUDA_TRY(ctx, dev_alloc_t(ctx, &sk->k_val, std::max<int64_t>(k_nnz, 1) * es));
-            RLA_CUDA_TRY(ctx, cudaMemcpy(sk->k_ptr, cp.data(), (sk->s + 1) * 4, cudaMemcpyHostToDevice));
+            RLA_CUDA_TRY(ctx, cudaMemcpyAsync(sk->k_ptr, cp.data(), (sk->s + 1) * 4, cudaMemcpyHostToDevice, ctx->stream));
             if (k_nnz) {
-                RLA_CUDA_TRY(ctx, cudaMemcpy(sk->k_col, cc.data(), k_nnz * 4, cudaMemcpyHostToDevice));
-                RLA_CUDA_TRY(ctx, cudaMemcpy(sk->k_val, cv.data(), k_nnz * es, cudaMemcpyHostToDevice));
+                RLA_CUDA_TRY(ctx, cudaMemcpyAsync(sk->k_col, cc.data(), k_nnz * 4, cudaMemcpyHostToDevice, ctx->stream));
+                RLA_CUDA_TRY(ctx, cudaMemcpyAsync(sk->k_val, cv.data(), k_nnz * es, cudaMemcpyHostToDevice, ctx->stream));
             }
+            RLA_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));  // the host arrays go out of scope
             sk->k_nnz = k_nnz;
             if (sk->p.dtype == RLA_F32) RLA_TRY(fjlt_transpose<float>(ctx, sk));
             else RLA_TRY(fjlt_transpose<double>(ctx, sk));

@@ -5,7 +5,7 @@ import ctypes
 
 import pytest
 
-from fake_cuda import F32, LEFT, RIGHT, fake, i64, vp  # noqa: F401 (fixture)
+from fake_cuda import F32, F64, LEFT, RIGHT, fake, i64, vp  # noqa: F401 (fixture)
 
 IHS, KACZMARZ, COLUMN = "ihs", 0, 1
 
@@ -78,5 +78,51 @@ def test_failed_solver_creation_waits_for_its_memsets(fake, solver, call):
         else:
             (fake.lib.rla_ihs_destroy if solver == IHS else fake.lib.rla_proj_destroy)(h)
     assert failed
+    fake.lib.rla_sketch_destroy(sk)
+    fake.lib.rla_ctx_destroy(ctx)
+
+
+def pool_rule_violations(log):
+    """Uses of pool memory that its order does not cover: filled by the legacy stream (cudaMemcpy) before
+    the stream it was allocated on has been waited for, or released with cudaFree, which returns
+    pool memory without waiting for the device."""
+    fresh, pool, bad = {}, set(), []
+    for line in log:
+        call, *rest = line.split()
+        stream = next((r[7:] for r in rest if r.startswith("stream=")), None)
+        if call == "cudaMallocFromPoolAsync":
+            fresh[rest[0]] = stream
+            pool.add(rest[0])
+        elif call == "cudaStreamSynchronize":
+            fresh = {p: s for p, s in fresh.items() if s != stream}
+        elif call == "cudaDeviceSynchronize":
+            fresh = {}
+        elif call == "cudaMemcpy" and rest[0] in fresh:
+            bad.append(line)
+        elif call == "cudaFree" and rest[0] in pool:
+            bad.append(line)
+    return bad
+
+
+@pytest.mark.parametrize("card", [LEFT, RIGHT])
+@pytest.mark.parametrize("dtype", [F32, F64])
+def test_loaded_fjlt_draws_follow_the_pool_order(fake, card, dtype):
+    """The matrix of loaded FJLT draws is allocated, filled and released in the order of the context's
+    stream; loading twice replaces what the first load allocated."""
+    ctx = fake.context()
+    s, L, N = 5, 50, 64
+    sk = fake.sketch(ctx, "fjlt", s, L, card=card, dtype=dtype)
+    ncol, nrow = (N, s) if card == LEFT else (s, N)
+    nnz = ncol
+    kptr = (ctypes.c_int64 * (ncol + 1))(*range(ncol + 1))
+    idx = (ctypes.c_int64 * nnz)(*[i % nrow for i in range(nnz)])
+    vals = ((ctypes.c_float if dtype == F32 else ctypes.c_double) * nnz)(*[1.0] * nnz)
+    signs = (ctypes.c_uint8 * N)()
+    fake.reset()
+    for _ in range(2):
+        rc = fake.lib.rla_sketch_set_draws(ctx, sk, idx, vals, signs, kptr, i64(nnz))
+        assert rc == 0, fake.lib.rla_ctx_last_error(ctx)
+    assert any(ln.startswith("cudaMallocFromPoolAsync") for ln in fake.log())
+    assert pool_rule_violations(fake.log()) == []
     fake.lib.rla_sketch_destroy(sk)
     fake.lib.rla_ctx_destroy(ctx)
