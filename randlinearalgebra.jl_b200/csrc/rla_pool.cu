@@ -1,5 +1,6 @@
 // rla_pool.cu -- memory of objects that outlive a call: a bounded device pool shared by the
 // contexts of a device, and pinned status slots.
+#include <map>
 #include <mutex>
 
 #include "rla_internal.cuh"
@@ -11,12 +12,12 @@ struct DevicePool {
     int contexts = 0;
 };
 static std::mutex g_pool_mu;
-static DevicePool g_pool[64];
+static std::map<int, DevicePool> &g_pool = *new std::map<int, DevicePool>;  // by device; lives as long as the process
 
 cudaError_t dev_alloc(rla_ctx *ctx, void **p, size_t bytes) {
     bytes = std::max<size_t>(bytes, 16);
     cudaMemPool_t pool = nullptr;
-    if (ctx->device < 64) {
+    {
         std::lock_guard<std::mutex> lock(g_pool_mu);
         DevicePool &d = g_pool[ctx->device];
         if (!d.pool) {
@@ -25,14 +26,15 @@ cudaError_t dev_alloc(rla_ctx *ctx, void **p, size_t bytes) {
             pp.location.type = cudaMemLocationTypeDevice;
             pp.location.id = ctx->device;
             uint64_t keep = 256ull << 20;
-            if (cudaMemPoolCreate(&d.pool, &pp) == cudaSuccess)
-                cudaMemPoolSetAttribute(d.pool, cudaMemPoolAttrReleaseThreshold, &keep);
-            else
+            const cudaError_t e = cudaMemPoolCreate(&d.pool, &pp);
+            if (e != cudaSuccess) {  // no other allocator: dev_free knows pool memory only
                 d.pool = nullptr;
+                return e;
+            }
+            cudaMemPoolSetAttribute(d.pool, cudaMemPoolAttrReleaseThreshold, &keep);
         }
         pool = d.pool;
     }
-    if (!pool) return cudaMalloc(p, bytes);
     return cudaMallocFromPoolAsync(p, bytes, pool, ctx->stream);
 }
 
@@ -72,7 +74,6 @@ void pinned_slot_free(double *p) {
 
 // The device's last context gives the pool's free memory back.
 void pool_contexts(int device, int change) {
-    if (device >= 64) return;
     std::lock_guard<std::mutex> lock(g_pool_mu);
     DevicePool &d = g_pool[device];
     d.contexts += change;

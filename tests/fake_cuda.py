@@ -4,6 +4,7 @@ import ctypes
 import importlib.util
 import os
 import re
+import shutil
 import subprocess
 from concurrent.futures import ThreadPoolExecutor
 
@@ -41,7 +42,7 @@ def build(folder):
             f.write('void %s(void) { fprintf(stderr, "fake runtime: %s\\n"); abort(); }\n' % (n, n))
     lib = os.path.join(folder, "librla_fake.so")
     subprocess.run(["g++", "-shared", "-fPIC", "-Wl,-Bsymbolic", "-o", lib, *objs, fake, "-x", "c", stubs], check=True)
-    return ctypes.CDLL(lib)
+    return lib
 
 
 class Params(ctypes.Structure):
@@ -51,10 +52,15 @@ class Params(ctypes.Structure):
 
 
 class Fake:
-    def __init__(self, folder):
-        self.lib = build(str(folder))
+    def __init__(self, path):
+        self.path = path
+        self.lib = ctypes.CDLL(path)
         self.lib.fake_log.restype = ctypes.c_char_p
         self.lib.rla_ctx_last_error.restype = ctypes.c_char_p
+
+    def fresh(self, folder):
+        """Another instance of the library, with none of this one's state."""
+        return Fake(shutil.copy(self.path, os.path.join(str(folder), "librla_fake_fresh.so")))
 
     def reset(self):
         self.lib.fake_reset()
@@ -108,7 +114,7 @@ _fake = []
 @pytest.fixture
 def fake(tmp_path_factory):
     if not _fake:
-        _fake.append(Fake(tmp_path_factory.mktemp("fake_cuda")))
+        _fake.append(Fake(build(str(tmp_path_factory.mktemp("fake_cuda")))))
     _fake[0].reset()
     yield _fake[0]
     _fake[0].reset()

@@ -126,3 +126,31 @@ def test_loaded_fjlt_draws_follow_the_pool_order(fake, card, dtype):
     assert pool_rule_violations(fake.log()) == []
     fake.lib.rla_sketch_destroy(sk)
     fake.lib.rla_ctx_destroy(ctx)
+
+
+def mismatched_releases(log):
+    """Allocations that are released by the call of another allocator, or never."""
+    open_, bad = {}, []
+    for line in log:
+        call, *rest = line.split()
+        if call in ("cudaMalloc", "cudaMallocAsync", "cudaMallocFromPoolAsync"):
+            open_[rest[0]] = call
+        elif call in ("cudaFree", "cudaFreeAsync"):
+            if open_.pop(rest[0]) == "cudaMalloc" and call == "cudaFreeAsync":
+                bad.append(line)
+    return bad + sorted(open_)
+
+
+@pytest.mark.parametrize("pool", [True, False])
+def test_buffers_are_released_by_their_own_allocator(fake, pool, tmp_path):
+    """Also on a device whose pool cannot be made: the creation then fails, without a buffer that a
+    release in stream order does not know."""
+    fake = fake.fresh(tmp_path)
+    ctx = fake.context()
+    if not pool:
+        fake.fail_after("cudaMemPoolCreate", 0)
+    rc, sk = fake.create(ctx, "sparse_sign", 40, 3000, nnz=8)
+    assert (rc == 0) == pool
+    fake.lib.rla_sketch_destroy(sk)
+    fake.lib.rla_ctx_destroy(ctx)
+    assert mismatched_releases(fake.log()) == []
