@@ -16,6 +16,11 @@ static std::map<int, DevicePool> &g_pool = *new std::map<int, DevicePool>;  // b
 
 cudaError_t dev_alloc(rla_ctx *ctx, void **p, size_t bytes) {
     bytes = std::max<size_t>(bytes, 16);
+    // an allocation that became part of a captured graph would be mapped only while the graph runs
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    const cudaError_t ec = cudaStreamIsCapturing(ctx->stream, &cap);
+    if (ec != cudaSuccess) return ec;
+    if (cap != cudaStreamCaptureStatusNone) return cudaErrorStreamCaptureUnsupported;
     cudaMemPool_t pool = nullptr;
     {
         std::lock_guard<std::mutex> lock(g_pool_mu);

@@ -78,10 +78,8 @@ static int sparse_t_plan(rla_ctx *ctx, rla_sketch *sk) {
     if (sk->tp_ptr && sk->tp_version == sk->draw_count) return RLA_OK;
     const int64_t n = sk->L * sk->nnz, s = sk->s;
     if (n >= (1ll << 31)) return set_error(ctx, RLA_E_UNSUPPORTED, "sparse operand: more than 2^31 sketch entries");
-    if (!sk->tp_ptr) {
-        RLA_CUDA_TRY(ctx, dev_alloc_t(ctx, &sk->tp_ptr, sizeof(int64_t) * (s + 1)));
-        RLA_CUDA_TRY(ctx, dev_alloc_t(ctx, &sk->tp_idx, sizeof(int32_t) * std::max<int64_t>(n, 1)));
-    }
+    if (!sk->tp_ptr) RLA_CUDA_TRY(ctx, dev_alloc_t(ctx, &sk->tp_ptr, sizeof(int64_t) * (s + 1)));
+    if (!sk->tp_idx) RLA_CUDA_TRY(ctx, dev_alloc_t(ctx, &sk->tp_idx, sizeof(int32_t) * std::max<int64_t>(n, 1)));
     int end_bit = 1;
     while (end_bit < 31 && ((int64_t)1 << end_bit) < s) ++end_bit;
     int32_t *keys_out = nullptr, *vals_in = nullptr;

@@ -208,6 +208,7 @@ cudaError_t cudaDeviceGetAttribute(int *v, cudaDeviceAttr a, int) {
 }
 cudaError_t cudaFuncGetAttributes(cudaFuncAttributes *a, const void *) {
     memset(a, 0, sizeof *a);
+    a->ptxVersion = a->binaryVersion = 100;
     return cudaSuccess;
 }
 cudaError_t cudaFuncSetAttribute(const void *, cudaFuncAttribute, int) { return cudaSuccess; }

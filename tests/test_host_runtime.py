@@ -154,3 +154,25 @@ def test_buffers_are_released_by_their_own_allocator(fake, pool, tmp_path):
     fake.lib.rla_sketch_destroy(sk)
     fake.lib.rla_ctx_destroy(ctx)
     assert mismatched_releases(fake.log()) == []
+
+
+def test_nothing_is_allocated_into_a_capture(fake):
+    """Memory that an object keeps must not become part of a graph that is being captured (it would
+    be mapped only while the graph runs): the call is refused and leaves the object as it was."""
+    ctx = fake.context()
+    s, m, n = 40, 3000, 7
+    sk = fake.sketch(ctx, "sparse_sign", s, m, nnz=4)
+    # the scratch of the later call, so that the capture finds it large enough
+    mul = fake.lib.rla_sketch_mul_sparse_t
+    mul.argtypes = [vp, vp, i64, i64, vp, i64, i64, i64, i64, vp, vp, vp, ctypes.c_double, ctypes.c_double]
+    call = lambda k: mul(ctx, k, s, n, 1 << 40, s, m, n, 5, 1 << 41, 1 << 42, 1 << 43, 1.0, 0.0)
+    other = fake.sketch(ctx, "sparse_sign", s, m, nnz=4)
+    assert call(other) == 0, fake.lib.rla_ctx_last_error(ctx)
+    fake.reset()
+    fake.capturing(True)
+    assert call(sk) != 0
+    assert not any("cudaMallocFromPoolAsync" in ln for ln in fake.log())
+    fake.capturing(False)
+    fake.reset()
+    assert call(sk) == 0
+    assert any("iota" in k for k in fake.launches())  # the plan is built by the call that runs
