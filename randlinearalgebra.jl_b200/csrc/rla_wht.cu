@@ -1087,7 +1087,10 @@ int srht_expand(rla_ctx *ctx, const rla_sketch *sk, const T *X, int64_t x_es, in
     p.beta = (T)beta;
     p.beta_zero = beta == 0.0;
     const int64_t nb = std::min<int64_t>(wht_batch<T>(sk->N, nv), 65535 * 32);
-    if (y_es == 1 || !scratch_ready(ctx, (size_t)(sk->N * nb) * sizeof(T)))
+    // not in a graph capture: the graph would keep the scratch after a later call had grown it
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    RLA_CUDA_TRY(ctx, cudaStreamIsCapturing(ctx->stream, &cap));
+    if (y_es == 1 || cap != cudaStreamCaptureStatusNone)
         return launch_near<T, WHT_IN_SAMPLES, WHT_OUT_Y>(ctx, p);
     void *w;
     RLA_TRY(scratch_get(ctx, (size_t)(sk->N * nb) * sizeof(T), &w));

@@ -176,3 +176,18 @@ def test_nothing_is_allocated_into_a_capture(fake):
     fake.reset()
     assert call(sk) == 0
     assert any("iota" in k for k in fake.launches())  # the plan is built by the call that runs
+
+
+def test_srht_expand_keeps_no_scratch_in_a_capture(fake):
+    """S' * Y into a row-major result goes through the context's scratch, but not in a graph capture:
+    the graph would keep the buffer after a later call had grown (and released) it."""
+    ctx = fake.context()
+    s, L, nv = 40, 3000, 64
+    sk = fake.sketch(ctx, "srht", s, L)
+    staged = lambda: [k for k in fake.launches() if "fjlt_expand_out" in k]
+    assert fake.mul(ctx, sk, (s, L, nv), LEFT, adjoint=True, row_c=True) == 0
+    assert staged()  # and the scratch is now large enough
+    fake.reset()
+    fake.capturing(True)
+    assert fake.mul(ctx, sk, (s, L, nv), LEFT, adjoint=True, row_c=True, wait=False) == 0
+    assert fake.launches() and not staged()
