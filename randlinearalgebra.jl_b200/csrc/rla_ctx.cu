@@ -67,12 +67,6 @@ int counters_get(rla_ctx *ctx, size_t n, int **out) {
     return RLA_OK;
 }
 
-bool scratch_ready(rla_ctx *ctx, size_t bytes) {
-    if (ctx->scratch.bytes >= ((bytes + 255) & ~size_t(255))) return true;
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    return cudaStreamIsCapturing(ctx->stream, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone;
-}
-
 cudaError_t ctx_pool_create(rla_ctx *ctx) {
     cudaMemPoolProps pp = {};
     pp.allocType = cudaMemAllocationTypePinned;

@@ -115,8 +115,6 @@ inline cudaError_t dev_alloc_t(rla_ctx *ctx, P **p, size_t bytes) {
 // iteration): 64 slots of one page, allocated on the first use; above, single allocations.
 cudaError_t pinned_slot(double **p);
 void pinned_slot_free(double *p);
-// False while ctx->stream captures a graph and the scratch would have to grow for `bytes`.
-bool scratch_ready(rla_ctx *ctx, size_t bytes);
 // The context's pool, made on its first use (a solver's private context needs none).
 cudaError_t ctx_pool_create(rla_ctx *ctx);
 // Stream-ordered allocation from the context's pool (memory stays mapped between calls, so

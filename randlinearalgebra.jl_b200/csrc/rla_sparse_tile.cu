@@ -599,8 +599,12 @@ int tile_compress(rla_ctx *ctx, const rla_sketch *sk, const T *X, int64_t x_es, 
     void *part = nullptr;
     const size_t part_bytes = (size_t)(2 * W) * g.sw * C * sizeof(T);
     // no partial sums when each CTA has whole (tile, window)s, also in a graph capture that finds
-    // the scratch too small
-    const bool shared = W > 1 && g.nchunk > 1 && scratch_ready(ctx, part_bytes);
+    // the scratch too small, or has four rounds of them (a captured scratch must not be grown later)
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    RLA_CUDA_TRY(ctx, cudaStreamIsCapturing(ctx->stream, &cap));
+    const bool whole = cap != cudaStreamCaptureStatusNone &&
+                       (ctx->scratch.bytes < part_bytes || groups >= 4 * (int64_t)ctx->sm_count);
+    const bool shared = W > 1 && g.nchunk > 1 && !whole;
     if (shared) RLA_TRY(scratch_get(ctx, part_bytes, &part));
     else W = (int)std::min<int64_t>(ctx->sm_count, groups);
     const bool contig = x_es == 1;

@@ -191,3 +191,19 @@ def test_srht_expand_keeps_no_scratch_in_a_capture(fake):
     fake.capturing(True)
     assert fake.mul(ctx, sk, (s, L, nv), LEFT, adjoint=True, row_c=True, wait=False) == 0
     assert fake.launches() and not staged()
+
+
+def test_wide_strided_compress_keeps_no_scratch_in_a_capture(fake):
+    """A * S with so many rows that their tiles fill the device many times over needs no partial sums:
+    a graph capture takes none from the scratch, whose growth would release them."""
+    ctx = fake.context()
+    s, L, nv = 40, 3000, 80000
+    sk = fake.sketch(ctx, "sparse_sign", s, L, card=RIGHT, nnz=4)
+    wide = fake.sketch(ctx, "srht", 4000, 5000)
+    assert fake.mul(ctx, wide, (4000, 5000, 5000), LEFT, row_a=True) == 0  # a large scratch
+    for capturing in (False, True):
+        fake.reset()
+        fake.capturing(capturing)
+        assert fake.mul(ctx, sk, (s, L, nv), RIGHT, wait=False) == 0
+        k = fake.launches()
+        assert any("tile_compress" in x for x in k) and any("tile_reduce" in x for x in k) == (not capturing)
