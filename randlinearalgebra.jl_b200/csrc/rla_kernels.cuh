@@ -44,7 +44,7 @@ int tile_compress(rla_ctx *ctx, const rla_sketch *sk, const T *X, int64_t x_es, 
                   int64_t y_es, int64_t y_vs, T alpha, T beta, bool beta_zero);
 
 // SparseSign / CountSketch expand on tiles of vectors (rla_sparse_lift.cu); *taken = false when
-// the compression dimension does not fit its staged tile.
+// the compression dimension does not fit its staged tile, or the call is too small for it.
 template <class T>
 int sparse_lift(rla_ctx *ctx, const rla_sketch *sk, const T *X, int64_t x_es, int64_t x_vs, int64_t nv, T *Y,
                 int64_t y_es, int64_t y_vs, T alpha, T beta, bool beta_zero, bool *taken);

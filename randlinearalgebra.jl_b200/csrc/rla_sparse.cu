@@ -811,12 +811,8 @@ template <class T>
 int sparse_expand(rla_ctx *ctx, const rla_sketch *sk, const T *X, int64_t x_es, int64_t x_vs, int64_t nv, T *Y,
                   int64_t y_es, int64_t y_vs, double alpha, double beta) {
     if (nv == 0) return RLA_OK;
-    // Staging the short operand and turning the blocks costs about 4 us; the kernel below does
-    // half a million (entry, vector) pairs per us (5549 x 23, nnz 4: 21.6 us a call, 24.0 staged).
-    bool taken = false;
-    if (sk->L * sk->nnz >= ((int64_t)1 << 21) / nv)
-        RLA_TRY(sparse_lift<T>(ctx, sk, X, x_es, x_vs, nv, Y, y_es, y_vs, (T)(alpha * sk->scale), (T)beta, beta == 0.0,
-                               &taken));
+    bool taken = false;  // false: fewer vectors or outputs than pay for staging the short operand
+    RLA_TRY(sparse_lift<T>(ctx, sk, X, x_es, x_vs, nv, Y, y_es, y_vs, (T)(alpha * sk->scale), (T)beta, beta == 0.0, &taken));
     if (taken) return RLA_OK;
     const int64_t L = sk->L;
     const int out_contig = y_es == 1;

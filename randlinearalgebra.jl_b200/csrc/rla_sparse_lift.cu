@@ -10,8 +10,9 @@
 // traffic alone would take 32 us): 131072 x 200 Float64, s = 1000, nnz = 8 in 122 us, 436 us with
 // a thread per output element.  The entry loop is unrolled for the usual nnz (154 us without).
 //
-// LPE = 8 / 4 / 2 lanes per entry (rows of 128 / 64 / 32 bytes) for s up to 1158 / 2084 / 3473:
-// the widest row that fits; above, the thread-per-element kernel of rla_sparse.cu.
+// LPE = 8 / 4 / 2 lanes per entry (rows of 128 / 64 / 32 bytes) for s up to 1095 / 2380 / 4309 at
+// nnz = 8 (1137 / 2457 / 4437 at nnz <= 2): the widest row that fits; above, and for calls too small
+// to pay for the staging (lift_pays), the thread-per-element kernel of rla_sparse.cu.
 #include "rla_internal.cuh"
 #include "rla_kernels.cuh"
 
@@ -233,13 +234,41 @@ static int lift_lanes(const rla_ctx *ctx, const rla_sketch *sk, size_t *smem) {
     return 0;
 }
 
+// Whether staging pays, against a thread per output element (rla_sparse.cu).  Times of a call in
+// us, that kernel / this one, Float32 unless named:
+//  * Column-major results.  That kernel takes about (2 + nnz) ps more per output; staging costs
+//    about 8 us at s = 1000 (8 lanes), twice that from a row-major short operand: 30000 x 16,
+//    nnz 8, s = 1000: 33 / 38; 131072 x 32, nnz 1: 42 / 36.  A tile of 32 (Float64: 16) vectors
+//    that is mostly empty costs as much as a full one: 2^20 long indices of nnz 8, 1 vector
+//    38 / 73, 4 vectors 81 / 72; nnz 1, 4 vectors 41 / 48, 8 vectors 57 / 49; nnz 3 (no unrolled
+//    loop) 8 vectors 67 / 73, 16 vectors 110 / 81.
+//  * Row-major results.  That kernel's blocks hold 128 vectors whatever their number is, so this
+//    one pays from two vectors on when there are enough long indices per staged row: 2^20 x 2,
+//    nnz 8: 300 / 95; 30000 x 32, nnz 8, s = 1000: 39 / 51; 131072 x 16, nnz 1: 66 / 42.
+//  * Two lanes per entry, Float64: tiles of 4 vectors write 32-byte pieces of rows (2^20 x 64, nnz 1:
+//    302 / 401), and with nnz 3 the words of 2^20 long indices are read again for every four
+//    columns (2^20 x 64: 415 / 485; 131072 x 200: 226 / 178).
+template <class T>
+static bool lift_pays(const rla_sketch *sk, int lpe, int64_t x_es, int64_t nv, int64_t y_es) {
+    if (nv < 2) return false;
+    const int64_t L = sk->L, nnz = sk->nnz, staged = sk->s * lpe;
+    const bool unrolled = nnz == 1 || nnz == 2 || nnz == 4 || nnz == 8, narrow64 = sizeof(T) == 8 && lpe == 2;
+    if (y_es != 1) {
+        if (narrow64 && nv > 32 && nnz != 8) return false;
+        return L * ceil_div(nv, 128) * (8 + nnz) >= std::max<int64_t>(115 * staged, 300000);
+    }
+    if (narrow64 && !unrolled && nnz < 8 && L >= (1 << 19)) return false;
+    if (nv < (nnz >= 8 ? 4 : unrolled ? 8 : 16)) return false;
+    return L * nv * (2 + nnz) >= std::max<int64_t>(1000 * staged * (x_es == 1 ? 1 : 2), 6000000);
+}
+
 template <class T>
 int sparse_lift(rla_ctx *ctx, const rla_sketch *sk, const T *X, int64_t x_es, int64_t x_vs, int64_t nv, T *Y,
                 int64_t y_es, int64_t y_vs, T alpha, T beta, bool beta_zero, bool *taken) {
     size_t smem = 0;
     const int lpe = lift_lanes<T>(ctx, sk, &smem);
-    *taken = lpe != 0;
-    if (!lpe) return RLA_OK;
+    *taken = lpe != 0 && lift_pays<T>(sk, lpe, x_es, nv, y_es);
+    if (!*taken) return RLA_OK;
     const int64_t C = lpe * (16 / (int64_t)sizeof(T)), nblk = ceil_div(sk->L, 32);
     // fewer warps per CTA while that spreads a small call over more SMs (every CTA stages X)
     int warps = LIFT_WARPS;

@@ -29,3 +29,38 @@ def test_partial_sums_of_one_tile_are_spread(fake, dtype, s):
     (x, y, threads), = grids(fake.log(), "tile_reduce")
     windows = -(-s // 1040)
     assert x * y * threads >= s * (32 if dtype == F32 else 16) and x == windows
+
+
+#        L, s, nnz, nv, dtype, row_major, kernel
+EXPANDS = [
+    # column-major results: few vectors, unrolled and general entry counts
+    (1 << 20, 512, 8, 1, F32, False, "expand_kernel"), (1 << 20, 512, 8, 3, F32, False, "expand_kernel"),
+    (1 << 20, 512, 8, 4, F32, False, "lift_kernelIfLi8ELi8E"), (1 << 20, 100, 1, 7, F32, False, "expand_kernel"),
+    (1 << 20, 100, 1, 8, F32, False, "lift_kernelIfLi8ELi1E"), (1 << 20, 500, 3, 15, F64, False, "expand_kernel"),
+    (1 << 20, 500, 3, 16, F64, False, "lift_kernelIdLi8ELi0E"),
+    # not enough outputs for the staging
+    (4096, 1000, 8, 64, F32, False, "expand_kernel"), (30000, 1000, 8, 16, F32, False, "expand_kernel"),
+    (30000, 1000, 8, 64, F32, False, "lift_kernelIfLi8ELi8E"), (4096, 64, 1, 200, F32, False, "expand_kernel"),
+    (4096, 64, 1, 1000, F32, False, "lift_kernelIfLi8ELi1E"),
+    # narrower staged rows and the last one that fits
+    (131072, 1095, 8, 200, F32, False, "lift_kernelIfLi8ELi8E"), (131072, 1096, 8, 200, F32, False, "lift_kernelIfLi4ELi8E"),
+    (131072, 2380, 8, 200, F64, False, "lift_kernelIdLi4ELi8E"), (131072, 2381, 8, 200, F64, False, "lift_kernelIdLi2ELi8E"),
+    (131072, 4309, 8, 200, F64, False, "lift_kernelIdLi2ELi8E"), (131072, 4310, 8, 200, F64, False, "expand_kernel"),
+    (1 << 20, 4000, 3, 64, F64, False, "expand_kernel"), (131072, 4000, 3, 200, F64, False, "lift_kernelIdLi2ELi0E"),
+    # row-major results
+    (1 << 20, 64, 2, 1, F32, True, "expand_kernel"), (1 << 20, 64, 2, 2, F32, True, "lift_kernelIfLi8ELi2E"),
+    (30000, 1000, 8, 32, F32, True, "expand_kernel"), (30000, 1000, 8, 1000, F32, True, "lift_kernelIfLi8ELi8E"),
+    (4096, 64, 4, 64, F32, True, "expand_kernel"), (1 << 20, 4000, 1, 64, F64, True, "expand_kernel"),
+    (1 << 20, 4000, 1, 32, F64, True, "lift_kernelIdLi2ELi1E"), (1 << 20, 4000, 8, 64, F64, True, "lift_kernelIdLi2ELi8E"),
+]
+
+
+@pytest.mark.parametrize("case", EXPANDS)
+def test_expand_routes(fake, case):
+    L, s, nnz, nv, dtype, row_major, kernel = case
+    ctx = fake.context()
+    sk = fake.sketch(ctx, "sparse_sign", s, L, dtype=dtype, nnz=nnz)
+    fake.reset()
+    assert fake.mul(ctx, sk, (s, L, nv), LEFT, adjoint=True, row_a=row_major, row_c=row_major) == 0
+    launched = fake.launches()
+    assert len(launched) == 1 and kernel in launched[0], launched
