@@ -4,6 +4,7 @@ import re
 
 import pytest
 
+import test_gpu_sparse_lift_sizes as lift
 from fake_cuda import F32, F64, LEFT, RIGHT, fake  # noqa: F401 (fixture)
 
 
@@ -64,3 +65,20 @@ def test_expand_routes(fake, case):
     assert fake.mul(ctx, sk, (s, L, nv), LEFT, adjoint=True, row_a=row_major, row_c=row_major) == 0
     launched = fake.launches()
     assert len(launched) == 1 and kernel in launched[0], launched
+
+
+@pytest.mark.parametrize("card", [LEFT, RIGHT])
+@pytest.mark.parametrize("dtype", [F32, F64])
+def test_lift_sizes_reach_the_staged_kernel(fake, dtype, card):
+    """Every size of test_gpu_sparse_lift_sizes.py, in each of its layouts."""
+    ctx = fake.context()
+    for layout, (row_y, row_c, pad, _, beta) in lift.LAYOUTS.items():
+        for L, s, nnz, nv, lanes in lift.sizes(layout):
+            sk = fake.sketch(ctx, "sparse_sign", s, L, card=card, dtype=dtype, nnz=nnz)
+            fake.reset()
+            rows = (row_y, row_c) if card == LEFT else (not row_y, not row_c)
+            assert fake.mul(ctx, sk, (s, L, nv), card, True, *rows, beta=beta, pad=pad) == 0
+            fixed = nnz if nnz in (1, 2, 4, 8) else 0
+            name = "lift_kernelI%sLi%dELi%dE" % ("f" if dtype == F32 else "d", lanes, fixed)
+            assert len(fake.launches()) == 1 and name in fake.launches()[0], (layout, L, s, nnz, nv, fake.launches())
+            fake.lib.rla_sketch_destroy(sk)
