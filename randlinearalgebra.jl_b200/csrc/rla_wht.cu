@@ -550,9 +550,9 @@ __global__ void srht_expand_kernel(const T *X, int64_t x_es, int64_t x_vs, int64
 // The columns of a batch are one run of nv * N elements (N >= 2^(VB+8)); a CTA takes 2^CH of them:
 // a chunk of a column, or several short columns.  The butterflies are those of the fused kernel's
 // three register passes, with the top stages left out for short columns.  The source is the
-// operand itself (sign flip and padding while loading), the batch workspace, the transposed
-// sampling matrix of the FJLT or the samples of the SRHT; the result goes to the workspace, to
-// the output with its signs, or is sampled from shared memory.  Columns above 2^CH take
+// operand itself (sign flip and padding while loading), the batch workspace or the samples of the
+// SRHT; the result goes to the workspace, to the output with its signs, or is sampled from shared
+// memory.  Columns above 2^CH take
 // wht_far_kernel for the remaining bits.  Workspace batches hold at most 64 MB, so that the passes
 // between the first read and the last write stay in L2 (126 MB).
 //
@@ -562,7 +562,7 @@ __global__ void srht_expand_kernel(const T *X, int64_t x_es, int64_t x_vs, int64
 // pass over the workspace per bit above 2^12; SRHT expand to 360737 x 61: 156 against 416 us, SRHT
 // 5003 -> 300 of 200 columns 28 against 85 us.
 // ------------------------------------------------------------------------------------
-enum WhtIn { WHT_IN_X, WHT_IN_W, WHT_IN_KT, WHT_IN_SAMPLES };
+enum WhtIn { WHT_IN_X, WHT_IN_W, WHT_IN_SAMPLES };
 enum WhtOut { WHT_OUT_W, WHT_OUT_Y, WHT_OUT_ROWS };
 
 template <class T>
@@ -573,8 +573,7 @@ struct WhtParams {
     int64_t L, N, nv;
     int log_n, top;      // top: stages over bits [VB+8, VB+8+top) of the chunk
     const uint32_t *signbits;
-    const int32_t *ptr, *idx;  // IN_KT: CSR of the transposed sampling matrix; IN_SAMPLES: idx = [samples | their rows] by low position
-    const T *val;
+    const int32_t *idx;        // IN_SAMPLES: [samples | their rows] by low position
     const int32_t *rows;       // IN_SAMPLES, OUT_ROWS
     int64_t s;
     T *W;
@@ -666,19 +665,8 @@ __global__ void __launch_bounds__(256, 2) wht_near_kernel(WhtParams<T> p) {
                         for (int i = 0; i < VW; ++i)
                             if (i < left) qe[i] = __ldg(x + i);
                     }
-                } else if constexpr (IN == WHT_IN_W) {
-                    if (v < p.nv) q = *reinterpret_cast<const V *>(p.W + base + o);
-                } else if (v < p.nv) {  // IN_KT: rows e .. of the transposed matrix
-                    int a = __ldg(p.ptr + e);
-#pragma unroll
-                    for (int i = 0; i < VW; ++i) {
-                        const int b = __ldg(p.ptr + e + i + 1);
-                        T sum = T(0);
-                        for (int k2 = a; k2 < b; ++k2)
-                            sum += __ldg(p.val + k2) * __ldg(p.X + (int64_t)__ldg(p.idx + k2) * p.x_es + v * p.x_vs);
-                        qe[i] = sum;
-                        a = b;
-                    }
+                } else if (v < p.nv) {
+                    q = *reinterpret_cast<const V *>(p.W + base + o);
                 }
                 set_vec(r, k, q);
             }
@@ -1155,9 +1143,6 @@ int fjlt_expand(rla_ctx *ctx, const rla_sketch *sk, const T *X, int64_t x_es, in
     WhtParams<T> p = wht_params<T>(sk, nv);
     p.x_es = x_es;
     p.x_vs = x_vs;
-    p.ptr = sk->kt_ptr;
-    p.idx = sk->kt_row;
-    p.val = (const T *)sk->kt_val;
     p.W = (T *)w;
     p.y_es = y_es;
     p.y_vs = y_vs;
@@ -1168,10 +1153,14 @@ int fjlt_expand(rla_ctx *ctx, const rla_sketch *sk, const T *X, int64_t x_es, in
         p.nv = std::min(nb, nv - v);
         p.X = X + v * x_vs;
         p.Y = Y + v * y_vs;
+        // A kernel of its own for the gather: inside the transform's loads each thread would walk 64
+        // rows after another, with as few CTAs as there are chunks (600 x 64 Float32, s = 300:
+        // 36 us a call, 102 inside; 40 before these kernels; 100003 x 512: 480 us, 610 inside).
+        const int grid = (int)std::min<int64_t>(ceil_div(N * p.nv, 256), (int64_t)ctx->sm_count * 32);
+        csr_t_gather_kernel<T><<<grid, 256, 0, ctx->stream>>>(sk->kt_ptr, sk->kt_row, (const T *)sk->kt_val, N, p.X, x_es,
+                                                              x_vs, p.nv, p.W);
+        RLA_TRY(check_launch(ctx, "fjlt_csr_t_gather"));
         if (N < wht_near_min<T>()) {
-            const int grid = (int)std::min<int64_t>(ceil_div(N * p.nv, 256), (int64_t)ctx->sm_count * 32);
-            csr_t_gather_kernel<T><<<grid, 256, 0, ctx->stream>>>(p.ptr, p.idx, p.val, N, p.X, x_es, x_vs, p.nv, p.W);
-            RLA_TRY(check_launch(ctx, "fjlt_csr_t_gather"));
             wht_short_kernel<T><<<(unsigned)std::min<int64_t>(p.nv, (int64_t)ctx->sm_count * 16), 256, N * sizeof(T),
                                   ctx->stream>>>(p.W, N, p.nv);
             RLA_TRY(check_launch(ctx, "wht_short"));
@@ -1180,10 +1169,10 @@ int fjlt_expand(rla_ctx *ctx, const rla_sketch *sk, const T *X, int64_t x_es, in
         }
         const bool far = p.log_n > WhtCfg<T>::CH, direct = y_es == 1;
         if (!far && direct) {
-            RLA_TRY((launch_near<T, WHT_IN_KT, WHT_OUT_Y>(ctx, p)));
+            RLA_TRY((launch_near<T, WHT_IN_W, WHT_OUT_Y>(ctx, p)));
             continue;
         }
-        RLA_TRY((launch_near<T, WHT_IN_KT, WHT_OUT_W>(ctx, p)));
+        RLA_TRY((launch_near<T, WHT_IN_W, WHT_OUT_W>(ctx, p)));
         RLA_TRY(launch_far(ctx, p, direct));
         if (!direct) RLA_TRY(launch_out(ctx, p));
     }

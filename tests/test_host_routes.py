@@ -82,3 +82,19 @@ def test_lift_sizes_reach_the_staged_kernel(fake, dtype, card):
             name = "lift_kernelI%sLi%dELi%dE" % ("f" if dtype == F32 else "d", lanes, fixed)
             assert len(fake.launches()) == 1 and name in fake.launches()[0], (layout, L, s, nnz, nv, fake.launches())
             fake.lib.rla_sketch_destroy(sk)
+
+
+@pytest.mark.parametrize("dtype", [F32, F64])
+@pytest.mark.parametrize("L", [600, 1000, 5003, 16384, 100003])
+def test_fjlt_expand_gathers_with_one_thread_per_element(fake, dtype, L):
+    """The rows of the transposed sampling matrix differ in length and a short transform has few CTAs:
+    S' * Y gathers into the workspace first, then transforms it."""
+    ctx = fake.context()
+    nv = 64
+    sk = fake.sketch(ctx, "fjlt", 300, L, dtype=dtype)
+    fake.reset()
+    assert fake.mul(ctx, sk, (300, L, nv), LEFT, adjoint=True) == 0
+    padded = 1 << (L - 1).bit_length()
+    (x, _, threads), = grids(fake.log(), "csr_t_gather")
+    assert x * threads >= min(padded * nv, 148 * 32 * 256)
+    assert fake.launches()[0].find("csr_t_gather") > 0
