@@ -1075,10 +1075,13 @@ int srht_expand(rla_ctx *ctx, const rla_sketch *sk, const T *X, int64_t x_es, in
     p.beta = (T)beta;
     p.beta_zero = beta == 0.0;
     const int64_t nb = std::min<int64_t>(wht_batch<T>(sk->N, nv), 65535 * 32);
-    // not in a graph capture: the graph would keep the scratch after a later call had grown it
+    // not for a few vectors, whose 32-wide tiles are mostly empty (2^20 long, direct / staged in us:
+    // Float32 x 2 38 / 122, x 12 108 / 139, x 16 144 / 145, x 32 600 / 271; Float64 x 12 118 / 273, x 16
+    // 359 / 285), nor in a graph capture: the graph would keep the scratch after a later call had
+    // grown it
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     RLA_CUDA_TRY(ctx, cudaStreamIsCapturing(ctx->stream, &cap));
-    if (y_es == 1 || cap != cudaStreamCaptureStatusNone)
+    if (y_es == 1 || nv <= (sizeof(T) == 4 ? 16 : 12) || cap != cudaStreamCaptureStatusNone)
         return launch_near<T, WHT_IN_SAMPLES, WHT_OUT_Y>(ctx, p);
     void *w;
     RLA_TRY(scratch_get(ctx, (size_t)(sk->N * nb) * sizeof(T), &w));

@@ -98,3 +98,15 @@ def test_fjlt_expand_gathers_with_one_thread_per_element(fake, dtype, L):
     (x, _, threads), = grids(fake.log(), "csr_t_gather")
     assert x * threads >= min(padded * nv, 148 * 32 * 256)
     assert fake.launches()[0].find("csr_t_gather") > 0
+
+
+@pytest.mark.parametrize("dtype,direct,staged", [(F32, 16, 17), (F64, 12, 13)])
+def test_srht_expand_writes_few_row_major_vectors_directly(fake, dtype, direct, staged):
+    """Tiles of 32 vectors that are mostly empty cost more than uncoalesced writes of a few vectors."""
+    ctx = fake.context()
+    L, s = 1 << 20, 100
+    sk = fake.sketch(ctx, "srht", s, L, dtype=dtype)
+    for nv in (2, direct, staged, 64):
+        fake.reset()
+        assert fake.mul(ctx, sk, (s, L, nv), LEFT, adjoint=True, row_c=True) == 0
+        assert any("fjlt_expand_out" in k for k in fake.launches()) == (nv >= staged), nv
