@@ -110,3 +110,13 @@ def test_srht_expand_writes_few_row_major_vectors_directly(fake, dtype, direct, 
         fake.reset()
         assert fake.mul(ctx, sk, (s, L, nv), LEFT, adjoint=True, row_c=True) == 0
         assert any("fjlt_expand_out" in k for k in fake.launches()) == (nv >= staged), nv
+
+
+@pytest.mark.parametrize("s,nv", [(100, 100), (64, 100), (33, 7)])
+def test_gaussian_split_sums_have_a_thread_per_element(fake, s, nv):
+    ctx = fake.context()
+    sk = fake.sketch(ctx, "gaussian", s, 16384)
+    fake.reset()
+    assert fake.mul(ctx, sk, (s, 16384, nv), LEFT) == 0
+    (x, y, threads), = grids(fake.log(), "conv_reduce")
+    assert x * y * threads >= s * nv
