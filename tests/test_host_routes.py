@@ -112,6 +112,23 @@ def test_srht_expand_writes_few_row_major_vectors_directly(fake, dtype, direct, 
         assert any("fjlt_expand_out" in k for k in fake.launches()) == (nv >= staged), nv
 
 
+#       s, L, nv, tiles of 128 x 64, splits of K
+GAUSS_SPLITS = [(64, 16384, 100, 1, 64), (200, 16384, 260, 12, 12), (250, 60000, 260, 12, 12), (100, 16384, 100, 2, 64),
+                (64, 4096, 9600, 75, 1), (64, 4096, 9472, 74, 2)]
+
+
+@pytest.mark.parametrize("case", GAUSS_SPLITS)
+def test_gaussian_k_splits_stay_in_one_round(fake, case):
+    """The K splits of a Gaussian product are not more CTAs than SMs."""
+    s, L, nv, tiles, splits = case
+    ctx = fake.context()
+    sk = fake.sketch(ctx, "gaussian", s, L)
+    fake.reset()
+    assert fake.mul(ctx, sk, (s, L, nv), LEFT) == 0
+    (x, y, _), = grids(fake.log(), "conv_gemm")
+    assert (x, y) == (tiles, splits) and x * y <= 148
+
+
 @pytest.mark.parametrize("s,nv", [(100, 100), (64, 100), (33, 7)])
 def test_gaussian_split_sums_have_a_thread_per_element(fake, s, nv):
     ctx = fake.context()
