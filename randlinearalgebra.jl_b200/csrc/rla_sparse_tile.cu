@@ -311,10 +311,9 @@ enum { TILE_CONTIG = 0, TILE_SHIFT = 1, TILE_ROWS = 2, TILE_ROWS_ANY = 3 };
 template <class T, int MODE, int GS>
 __global__ void __launch_bounds__(BL_WARPS * 32, 1) tile_compress_kernel(TileParams<T> p) {
     using V = typename TileVec<T>::type;
-    constexpr int VR = TileCfg<T>::VR, C = TileCfg<T>::C, PE = BL_PITCH / (int)sizeof(T);
+    constexpr int VR = TileCfg<T>::VR, C = TileCfg<T>::C;
     extern __shared__ __align__(128) unsigned char smem_raw[];
     unsigned char *bin_raw = smem_raw + BL_TILE_BYTES;
-    const T *bins = reinterpret_cast<const T *>(bin_raw);
     const int t = threadIdx.x, lane = t & 31, wp = t >> 5, l8 = lane & 7;
     const uint32_t lane16 = (uint32_t)l8 << 4;
     const int64_t nchunk = p.g.nchunk;
@@ -521,71 +520,97 @@ __global__ void __launch_bounds__(BL_WARPS * 32, 1) tile_compress_kernel(TilePar
         const int64_t lo = (int64_t)win_u * p.g.sw;
         const int cnt = (int)min((int64_t)p.g.sw, p.s - lo);
         const int nc = (int)min((int64_t)C, p.nv - v0);
-        auto bin = [&](int b, int c) {
-            T a = bins[b * PE + c];
-            for (int r = 1; r < p.g.G; ++r) a += bins[(r * p.g.sw + b) * PE + c];
+        // bins of bucket b, 16 bytes from column q * VR on (lanes along b: conflict-free)
+        auto bin = [&](int b, int q) {
+            V a = *reinterpret_cast<const V *>(bin_raw + b * BL_PITCH + q * 16);
+            for (int r = 1; r < p.g.G; ++r) {
+                const V x = *reinterpret_cast<const V *>(bin_raw + (r * p.g.sw + b) * BL_PITCH + q * 16);
+                T *ae = reinterpret_cast<T *>(&a);
+                const T *xe = reinterpret_cast<const T *>(&x);
+#pragma unroll
+                for (int e = 0; e < VR; ++e) ae[e] += xe[e];
+            }
             return a;
         };
-        auto put = [&](int b, int c) {
-            T *yp = p.Y + (lo + b) * p.y_es + (v0 + c) * p.y_vs;
-            T r = p.alpha * bin(b, c);
-            if (!p.beta_zero) r += p.beta * *yp;
-            *yp = r;
-        };
         if (u0 <= gbeg && gbeg + nchunk <= u1) {
-            if (p.y_es == 1) {
-                for (int c = wp; c < nc; c += BL_WARPS)
-                    for (int b = lane; b < cnt; b += 32) put(b, c);
-            } else {
-                for (int i = t; i < cnt * C; i += BL_WARPS * 32)
-                    if (i % C < nc) put(i / C, i % C);
+            // lanes along the dimension that is contiguous in memory
+            const bool down = p.y_es == 1;
+            for (int i = t; i < (down ? (cnt + 31) / 32 * 32 : cnt) * 8; i += BL_WARPS * 32) {
+                const int b = down ? (i >> 8) * 32 + lane : i >> 3, q = down ? (i >> 5) & 7 : i & 7;
+                if (b >= cnt || q * VR >= nc) continue;
+                const V a = bin(b, q);
+                const T *ae = reinterpret_cast<const T *>(&a);
+                T *yp = p.Y + (lo + b) * p.y_es + (v0 + q * VR) * p.y_vs;
+#pragma unroll
+                for (int e = 0; e < VR; ++e)
+                    if (q * VR + e < nc) {
+                        T r = p.alpha * ae[e];
+                        if (!p.beta_zero) r += p.beta * yp[e * p.y_vs];
+                        yp[e * p.y_vs] = r;
+                    }
             }
         } else {
-            T *part = p.partials + (int64_t)p.split.slot(blockIdx.x, gbeg) * p.g.sw * C;
-            for (int i = t; i < cnt * C; i += BL_WARPS * 32) part[i] = bin(i / C, i % C);
+            V *part = reinterpret_cast<V *>(p.partials + (int64_t)p.split.slot(blockIdx.x, gbeg) * p.g.sw * C);
+            for (int i = t; i < cnt * 8; i += BL_WARPS * 32) part[i] = bin(i >> 3, i & 7);
         }
         __syncthreads();
         if (u + 1 < u1) zero_bins();
     }
 }
 
-// Adds the partial bins of every (tile, window) shared by several CTAs, in CTA order; one thread per
-// element, 256 elements per CTA, TR_AHEAD partials in flight: a single tile has up to 148 of them,
-// and their latency is all this kernel does (131072 x 1 Float32 to 100 buckets, nnz 2: 45 us a call;
-// 108 us with four elements per thread and four partials in flight).
+// Adds the partial bins of the (tile, window)s shared by several CTAs, in CTA order; 256 accesses of
+// E elements per CTA, TR_AHEAD partials in flight.  One element per thread spreads a few (tile,
+// window)s over the GPU: a single one has up to 148 partials, whose latency is all this kernel does
+// (131072 x 1 Float32 to 100 buckets, nnz 2: 45 us a call; 108 us with four elements per thread and
+// four partials in flight).  16 bytes per thread otherwise: the number of CTAs, most of them with two
+// partials, counts then.  by_cut: CTA column x takes the (tile, window) that is cut where worker x + 1
+// starts, if that is its first cut (at most W - 1 of them are shared, whatever their number); else
+// (tile, window) x.
 constexpr int TR_AHEAD = 16;
-template <class T>
-__global__ void __launch_bounds__(256) tile_reduce_kernel(TileParams<T> p) {
-    constexpr int C = TileCfg<T>::C, NB = 256 / C;  // buckets per CTA
+template <class T, int E>
+__global__ void __launch_bounds__(256) tile_reduce_kernel(TileParams<T> p, int by_cut) {
+    constexpr int C = TileCfg<T>::C, NB = 256 * E / C, AHEAD = TR_AHEAD / E;  // NB: buckets per CTA
+    using V = std::conditional_t<E == 1, T, typename TileVec<T>::type>;
     __shared__ T tile[NB][C + 1];
-    const int64_t grp = blockIdx.x, gbeg = grp * p.g.nchunk;
+    const int64_t cut = by_cut ? p.split.start(blockIdx.x + 1) : 0;
+    const int64_t grp = by_cut ? cut / p.g.nchunk : blockIdx.x, gbeg = grp * p.g.nchunk;
+    if (by_cut && cut == gbeg) return;
     const int gf = p.split.owner(gbeg), gl = p.split.owner(gbeg + p.g.nchunk - 1);
-    if (gf == gl) return;  // written by its only CTA
+    if (by_cut ? gf != (int)blockIdx.x : gf == gl) return;  // another CTA's, or written by its only worker
     const int64_t lo = (grp % p.g.nwin) * p.g.sw, v0 = (grp / p.g.nwin) * C;
     const int cnt = (int)min((int64_t)p.g.sw, p.s - lo);
-    const int b0 = blockIdx.y * NB, i = threadIdx.x;
+    const int b0 = blockIdx.y * NB, i = threadIdx.x * E;
     if (b0 >= cnt) return;
     const int64_t ps = (int64_t)p.g.sw * C;
     if (b0 + i / C < cnt) {
         const T *part = p.partials + b0 * C + i;
-        T a = part[p.split.slot(gf, gbeg) * ps];
-        for (int g0 = gf + 1; g0 <= gl; g0 += TR_AHEAD) {
-            T v[TR_AHEAD];
+        T a[E];
+        *reinterpret_cast<V *>(a) = ld_ahead(reinterpret_cast<const V *>(part + p.split.slot(gf, gbeg) * ps));
+        for (int g0 = gf + 1; g0 <= gl; g0 += AHEAD) {
+            V v[AHEAD];
 #pragma unroll
-            for (int k = 0; k < TR_AHEAD; ++k) v[k] = ld_ahead(part + 2 * (int64_t)min(g0 + k, gl) * ps);
+            for (int k = 0; k < AHEAD; ++k) v[k] = ld_ahead(reinterpret_cast<const V *>(part + 2 * (int64_t)min(g0 + k, gl) * ps));
 #pragma unroll
-            for (int k = 0; k < TR_AHEAD; ++k)
-                if (g0 + k <= gl) a += v[k];
+            for (int k = 0; k < AHEAD; ++k)
+                if (g0 + k <= gl) {
+#pragma unroll
+                    for (int e = 0; e < E; ++e) a[e] += reinterpret_cast<const T *>(&v[k])[e];
+                }
         }
-        tile[i / C][i % C] = a;
+#pragma unroll
+        for (int e = 0; e < E; ++e) tile[i / C][i % C + e] = a[e];
     }
     __syncthreads();
-    const int b = p.y_es == 1 ? i % NB : i / C, c = p.y_es == 1 ? i / NB : i % C;
-    if (b0 + b >= cnt || v0 + c >= p.nv) return;
-    T *yp = p.Y + (lo + b0 + b) * p.y_es + (v0 + c) * p.y_vs;
-    T r = p.alpha * tile[b][c];
-    if (!p.beta_zero) r += p.beta * *yp;
-    *yp = r;
+#pragma unroll
+    for (int q = 0; q < E; ++q) {
+        const int k = threadIdx.x + 256 * q;
+        const int b = p.y_es == 1 ? k % NB : k / C, c = p.y_es == 1 ? k / NB : k % C;
+        if (b0 + b >= cnt || v0 + c >= p.nv) continue;
+        T *yp = p.Y + (lo + b0 + b) * p.y_es + (v0 + c) * p.y_vs;
+        T r = p.alpha * tile[b][c];
+        if (!p.beta_zero) r += p.beta * *yp;
+        *yp = r;
+    }
 }
 
 template <class T>
@@ -598,8 +623,8 @@ int tile_compress(rla_ctx *ctx, const rla_sketch *sk, const T *X, int64_t x_es, 
     int W = (int)std::min<int64_t>(ctx->sm_count, units);
     void *part = nullptr;
     const size_t part_bytes = (size_t)(2 * W) * g.sw * C * sizeof(T);
-    // no partial sums when each CTA has whole (tile, window)s, also in a graph capture that finds
-    // the scratch too small, or has four rounds of them (a captured scratch must not be grown later)
+    // No partial sums when each CTA has whole (tile, window)s: in a graph capture that finds the
+    // scratch too small, or has four rounds of them (a captured scratch must not be grown later).
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     RLA_CUDA_TRY(ctx, cudaStreamIsCapturing(ctx->stream, &cap));
     const bool whole = cap != cudaStreamCaptureStatusNone &&
@@ -625,7 +650,14 @@ int tile_compress(rla_ctx *ctx, const rla_sketch *sk, const T *X, int64_t x_es, 
     };
     RLA_TRY(g.gs == 4 ? by_mode(std::integral_constant<int, 4>()) : by_mode(std::integral_constant<int, 1>()));
     if (!shared) return RLA_OK;
-    tile_reduce_kernel<T><<<dim3((unsigned)groups, ceil_div_i(g.sw, 256 / C)), 256, 0, ctx->stream>>>(p);
+    const int by_cut = groups > W - 1;
+    const unsigned gx = (unsigned)(by_cut ? W - 1 : groups);
+    // one element per thread while its grid is one round of CTAs (8 per SM)
+    const int scalar = ceil_div_i(g.sw, 256 / C);
+    if ((int64_t)gx * scalar <= (int64_t)ctx->sm_count * 8)
+        tile_reduce_kernel<T, 1><<<dim3(gx, scalar), 256, 0, ctx->stream>>>(p, by_cut);
+    else
+        tile_reduce_kernel<T, VR><<<dim3(gx, ceil_div_i(g.sw, 256 * VR / C)), 256, 0, ctx->stream>>>(p, by_cut);
     return check_launch(ctx, "tile_reduce");
 }
 

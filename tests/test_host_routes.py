@@ -137,3 +137,22 @@ def test_gaussian_split_sums_have_a_thread_per_element(fake, s, nv):
     assert fake.mul(ctx, sk, (s, 16384, nv), LEFT) == 0
     (x, y, threads), = grids(fake.log(), "conv_reduce")
     assert x * y * threads >= s * nv
+
+
+#       L, s, nnz, nv, dtype: calls whose (tile, window)s are cut between CTAs
+CUTS = [(100000, 500, 8, 500, F32), (10000, 8320, 2, 3000, F32), (150001, 1332, 8, 333, F32),
+        (100000, 6240, 3, 16, F64)]
+
+
+@pytest.mark.parametrize("case", CUTS)
+def test_tile_reduction_covers_the_cut_tiles_only(fake, case):
+    """At most W - 1 (tile, window)s are cut by the borders of W workers, whatever their number is."""
+    L, s, nnz, nv, dtype = case
+    ctx = fake.context()
+    sk = fake.sketch(ctx, "sparse_sign", s, L, dtype=dtype, nnz=nnz)
+    fake.reset()
+    assert fake.mul(ctx, sk, (s, L, nv), LEFT) == 0
+    (w, _, _), = grids(fake.log(), "tile_compress")
+    (x, y, threads), = grids(fake.log(), "tile_reduce")
+    tiles = -(-nv // (32 if dtype == F32 else 16)) * -(-s // 1040)
+    assert x == min(tiles, w - 1)
