@@ -613,6 +613,18 @@ __global__ void __launch_bounds__(256) tile_reduce_kernel(TileParams<T> p, int b
     }
 }
 
+// Whether cutting (tile, window)s between W CTAs pays for the partial sums, against CTAs with whole
+// ones.  It saves chunks on the longest CTA, each 2.7 us and 0.9 us per entry and window, and costs the
+// reduction, 6.5 us and 5 us per 100000 partial bins (least squares over 1113 calls of nnz 2 to 8, s up
+// to 8320, 700 to 100000 long, both types; us a call, whole / cut):
+//   Float32, nnz 2: 2000 x 1000 to 1000 43 / 38; 1000 x 3000 to 1000 39 / 54; 4000 x 10000 to 2080 188 / 191;
+//   100000 x 200 to 500 677 / 70.
+static bool sharing_pays(const rla_sketch *sk, const BlGeom &g, int64_t groups, int64_t W) {
+    const int64_t saved = ceil_div(groups, W) * g.nchunk - ceil_div(groups * g.nchunk, W);
+    const double bins = (double)std::min<int64_t>(2 * W, W + groups) * g.sw;
+    return saved * (2.7 + 0.9 * sk->nnz / g.nwin) > 6.5 + 5e-5 * bins;
+}
+
 template <class T>
 int tile_compress(rla_ctx *ctx, const rla_sketch *sk, const T *X, int64_t x_es, int64_t x_vs, int64_t nv, T *Y,
                   int64_t y_es, int64_t y_vs, T alpha, T beta, bool beta_zero) {
@@ -629,7 +641,7 @@ int tile_compress(rla_ctx *ctx, const rla_sketch *sk, const T *X, int64_t x_es, 
     RLA_CUDA_TRY(ctx, cudaStreamIsCapturing(ctx->stream, &cap));
     const bool whole = cap != cudaStreamCaptureStatusNone &&
                        (ctx->scratch.bytes < part_bytes || groups >= 4 * (int64_t)ctx->sm_count);
-    const bool shared = W > 1 && g.nchunk > 1 && !whole;
+    const bool shared = W > 1 && g.nchunk > 1 && !whole && sharing_pays(sk, g, groups, W);
     if (shared) RLA_TRY(scratch_get(ctx, part_bytes, &part));
     else W = (int)std::min<int64_t>(ctx->sm_count, groups);
     const bool contig = x_es == 1;

@@ -156,3 +156,14 @@ def test_tile_reduction_covers_the_cut_tiles_only(fake, case):
     (x, y, threads), = grids(fake.log(), "tile_reduce")
     tiles = -(-nv // (32 if dtype == F32 else 16)) * -(-s // 1040)
     assert x == min(tiles, w - 1)
+
+
+@pytest.mark.parametrize("case", [(1000, 1000, 2, 3000, F32), (640, 40, 8, 100000, F32), (1000, 1000, 3, 10000, F64)])
+def test_short_tiles_are_not_cut(fake, case):
+    """With a chunk or two per tile a CTA takes whole tiles: the partial sums would take longer."""
+    L, s, nnz, nv, dtype = case
+    ctx = fake.context()
+    sk = fake.sketch(ctx, "sparse_sign", s, L, dtype=dtype, nnz=nnz)
+    fake.reset()
+    assert fake.mul(ctx, sk, (s, L, nv), LEFT) == 0
+    assert len(fake.launches()) == 1 and "tile_compress" in fake.launches()[0]

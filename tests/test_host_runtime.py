@@ -197,7 +197,7 @@ def test_wide_strided_compress_keeps_no_scratch_in_a_capture(fake):
     """A * S with so many rows that their tiles fill the device many times over needs no partial sums:
     a graph capture takes none from the scratch, whose growth would release them."""
     ctx = fake.context()
-    s, L, nv = 40, 3000, 80000
+    s, L, nv = 40, 3000, 19200  # 600 tiles of 5 chunks: 21 chunks per CTA, 25 with whole tiles
     sk = fake.sketch(ctx, "sparse_sign", s, L, card=RIGHT, nnz=4)
     wide = fake.sketch(ctx, "srht", 4000, 5000)
     assert fake.mul(ctx, wide, (4000, 5000, 5000), LEFT, row_a=True) == 0  # a large scratch
