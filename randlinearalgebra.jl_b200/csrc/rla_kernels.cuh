@@ -50,6 +50,7 @@ int sparse_lift(rla_ctx *ctx, const rla_sketch *sk, const T *X, int64_t x_es, in
                 int64_t y_es, int64_t y_vs, T alpha, T beta, bool beta_zero, bool *taken);
 
 // SRHT / FJLT (rla_wht.cu)
+constexpr int64_t SRHT_COLUMN_N = 4096;  // longest column that may have a CTA of its own
 // Builds sk->sign_tl (per-thread sign masks of the fused compress kernel) from sk->signbits.
 int build_srht_sign_table(rla_ctx *ctx, rla_sketch *sk);
 template <class T>

@@ -18,6 +18,7 @@
 #include <mutex>
 
 #include "rla_internal.cuh"
+#include "rla_kernels.cuh"
 
 namespace rla {
 
@@ -463,8 +464,8 @@ int build_srht_sign_table(rla_ctx *ctx, rla_sketch *sk) {
     return check_launch(ctx, "sign_table");
 }
 
-// Small padded sizes (N < 2^(VB+8)): one CTA per column, the whole padded column in
-// shared memory, log2(N) butterfly stages.
+// Short columns (N <= SRHT_COLUMN_N, see column_per_cta): one CTA per column, the whole padded column
+// in shared memory, log2(N) butterfly stages.
 template <class T>
 __global__ void srht_small_kernel(const T *X, int64_t x_ld, int64_t L, int64_t N, int64_t nv,
                                   const uint32_t *signbits, const int32_t *rows, int64_t s, T *Y, int64_t y_es,
@@ -497,48 +498,37 @@ __global__ void srht_small_kernel(const T *X, int64_t x_ld, int64_t L, int64_t N
     }
 }
 
-// Expand: out(r, v) = alpha*scale*d_r * sum_k H[r, rows_k] x(k, v) + beta*out(r, v), r < L.
-// One CTA per (column, output chunk of `ch` rows).
+// Expand of short columns: out(r, v) = alpha*scale*d_r * sum_k H[r, rows_k] x(k, v) + beta*out(r, v),
+// r < L, one CTA per column.
 template <class T>
 __global__ void srht_expand_kernel(const T *X, int64_t x_es, int64_t x_vs, int64_t L, int64_t N, int64_t nv,
-                                   const uint32_t *signbits, const int32_t *rows, const int32_t *p2_ptr,
-                                   const int32_t *p2_list, int ch, int log_ch, T *Y, int64_t y_es, int64_t y_vs,
-                                   T alpha, T beta, int beta_zero) {
+                                   const uint32_t *signbits, const int32_t *p2_ptr, const int32_t *p2_list, T *Y,
+                                   int64_t y_es, int64_t y_vs, T alpha, T beta, int beta_zero) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     T *z = reinterpret_cast<T *>(smem_raw);
-    const int64_t nchunks = N >> log_ch;
-    for (int64_t blk = blockIdx.x; blk < nv * nchunks; blk += gridDim.x) {
-        const int64_t v = blk / nchunks, oc = blk % nchunks;
-        if ((oc << log_ch) >= L) continue;  // block-uniform: chunk entirely in the padding
-        for (int p2 = threadIdx.x; p2 < ch; p2 += blockDim.x) {
+    const int n = (int)N;
+    for (int64_t v = blockIdx.x; v < nv; v += gridDim.x) {
+        for (int p2 = threadIdx.x; p2 < n; p2 += blockDim.x) {
             T sum = T(0);
-            for (int q = p2_ptr[p2]; q < p2_ptr[p2 + 1]; ++q) {
-                const int k = p2_list[q];
-                const int64_t r1 = (int64_t)rows[k] >> log_ch;
-                const T x = X[(int64_t)k * x_es + v * x_vs];
-                sum += (__popcll((unsigned long long)(r1 & oc)) & 1) ? -x : x;
-            }
+            for (int q = p2_ptr[p2]; q < p2_ptr[p2 + 1]; ++q) sum += X[(int64_t)p2_list[q] * x_es + v * x_vs];
             z[p2] = sum;
         }
         __syncthreads();
-        for (int h = 1; h < ch; h <<= 1) {
-            for (int q = threadIdx.x; q < ch / 2; q += blockDim.x) {
-                const int i = (q / h) * 2 * h + (q % h);
-                T a = z[i], b = z[i + h];
+        for (int h = 1; h < n; h <<= 1) {
+            for (int q = threadIdx.x; q < n / 2; q += blockDim.x) {
+                const int i = (q & ~(h - 1)) * 2 + (q & (h - 1));
+                const T a = z[i], b = z[i + h];
                 z[i] = a + b;
                 z[i + h] = a - b;
             }
             __syncthreads();
         }
-        for (int r2 = threadIdx.x; r2 < ch; r2 += blockDim.x) {
-            const int64_t r = (oc << log_ch) + r2;
-            if (r < L) {
-                const T d = ((signbits[r >> 5] >> (r & 31)) & 1u) ? alpha : -alpha;
-                T *yp = Y + r * y_es + v * y_vs;
-                T res = d * z[r2];
-                if (!beta_zero) res += beta * *yp;
-                *yp = res;
-            }
+        for (int r = threadIdx.x; r < (int)L; r += blockDim.x) {
+            const T d = ((signbits[r >> 5] >> (r & 31)) & 1u) ? alpha : -alpha;
+            T *yp = Y + r * y_es + v * y_vs;
+            T res = d * z[r];
+            if (!beta_zero) res += beta * *yp;
+            *yp = res;
         }
         __syncthreads();
     }
@@ -972,11 +962,31 @@ static int launch_out(rla_ctx *ctx, const WhtParams<T> &p) {
     return check_launch(ctx, "wht_out");
 }
 
-// Columns shorter than a chunk: several per CTA, sampled from shared memory.
+// Columns of up to SRHT_COLUMN_N: whether the kernels with a CTA per column take a call.  wht_near_kernel puts
+// 2^CH elements into a CTA, so that a few short columns with many samples run their gathers on a few
+// SMs: per_sample us for each sample of a chunk and round of CTAs; a CTA per column costs start us per
+// 1024 elements of a column above the first 1024, and per_col us per 1024 elements of all columns
+// (per 16 CTAs of an SM).  Fitted to calls of 1 to 4000 columns, us, a CTA per column / several:
+//   compress, Float32: 1000 x 32 to 800 27 / 32, rows of a row-major matrix 31 / 40; 2000 x 32 to 2000 35 / 34;
+//     2000 x 500 to 300 43 / 29;
+//   expand, Float32: to 1000 x 128 from 300 28 / 37, to 2000 x 128 from 2000 34 / 60, from 300 33 / 32, to
+//     4000 x 64 from 4000 44 / 62, to 4000 x 2000 from 4000 131 / 116.
+template <class T>
+static bool column_per_cta(const rla_ctx *ctx, const rla_sketch *sk, int64_t nv, double per_sample, double first, double start,
+                           double per_col) {
+    if (sk->N < wht_near_min<T>()) return true;
+    if (sk->N > SRHT_COLUMN_N) return false;
+    const int64_t cols = ((int64_t)1 << WhtCfg<T>::CH) / sk->N;  // per chunk
+    const int64_t rounds = ceil_div(ceil_div(nv, cols), 2 * (int64_t)ctx->sm_count);
+    const double n = sk->N / 1024.0;
+    return per_sample * (sk->s * std::min(cols, nv)) * rounds > first + start * (n - 1) + per_col * nv * n;
+}
+
+// Columns shorter than a chunk, sampled from shared memory.
 template <class T>
 static int srht_short(rla_ctx *ctx, const rla_sketch *sk, const T *X, int64_t ldx, int64_t nv, T *Y, int64_t y_es,
                       int64_t y_vs, T alpha, T beta, bool beta_zero) {
-    if (sk->N < wht_near_min<T>()) {
+    if (column_per_cta<T>(ctx, sk, nv, y_es == 1 ? 0.4e-3 : 0.8e-3, sizeof(T) == 4 ? 0.0 : 4.0, 7.0, 16e-3)) {
         const int grid = (int)std::min<int64_t>(nv, (int64_t)ctx->sm_count * 8);
         srht_small_kernel<T><<<grid, 256, (size_t)sk->N * sizeof(T), ctx->stream>>>(
             X, ldx, sk->L, sk->N, nv, sk->signbits, sk->rows, sk->s, Y, y_es, y_vs, alpha, beta, beta_zero);
@@ -1052,15 +1062,10 @@ int srht_expand(rla_ctx *ctx, const rla_sketch *sk, const T *X, int64_t x_es, in
                 int64_t y_es, int64_t y_vs, double alpha, double beta) {
     if (nv == 0) return RLA_OK;
     const T a = (T)(alpha * sk->scale);
-    if (sk->N < wht_near_min<T>()) {
-        const int ch = (int)sk->chunk;
-        const int log_ch = ilog2(ch);
-        const int64_t nblk = nv * (sk->N >> log_ch);
-        const int grid = (int)std::min<int64_t>(nblk, (int64_t)ctx->sm_count * 16);
-        const size_t smem = (size_t)ch * sizeof(T);
-        srht_expand_kernel<T><<<grid, 256, smem, ctx->stream>>>(X, x_es, x_vs, sk->L, sk->N, nv, sk->signbits, sk->rows,
-                                                                sk->p2_ptr, sk->p2_list, ch, log_ch, Y, y_es, y_vs, a,
-                                                                (T)beta, beta == 0.0);
+    if (column_per_cta<T>(ctx, sk, nv, x_es == 1 ? 2e-3 : 2.6e-3, sizeof(T) == 4 ? 0.0 : 2.0, 5.0, 11.5e-3)) {
+        const int grid = (int)std::min<int64_t>(nv, (int64_t)ctx->sm_count * 16);
+        srht_expand_kernel<T><<<grid, 256, (size_t)sk->N * sizeof(T), ctx->stream>>>(
+            X, x_es, x_vs, sk->L, sk->N, nv, sk->signbits, sk->p2_ptr, sk->p2_list, Y, y_es, y_vs, a, (T)beta, beta == 0.0);
         return check_launch(ctx, "srht_expand");
     }
     WhtParams<T> p = wht_params<T>(sk, nv);

@@ -5,6 +5,7 @@ import re
 import pytest
 
 import test_gpu_sparse_lift_sizes as lift
+import test_gpu_srht_short as srht_short
 from fake_cuda import F32, F64, LEFT, RIGHT, fake  # noqa: F401 (fixture)
 
 
@@ -167,3 +168,38 @@ def test_short_tiles_are_not_cut(fake, case):
     fake.reset()
     assert fake.mul(ctx, sk, (s, L, nv), LEFT) == 0
     assert len(fake.launches()) == 1 and "tile_compress" in fake.launches()[0]
+
+
+#       L, s, nv, dtype, expand: a CTA per column, compress: a CTA per column
+SRHT_SHORT = [(1000, 800, 40, F32, True, True), (1000, 300, 128, F32, True, False), (1000, 800, 4000, F32, False, False),
+              (1000, 10, 128, F32, False, False), (2000, 2000, 64, F32, True, False), (2000, 300, 128, F32, False, False),
+              (2000, 2000, 2000, F32, False, False), (4000, 4000, 64, F32, True, False), (4000, 4000, 2000, F32, False, False),
+              (4000, 300, 8, F32, False, False), (8000, 4000, 8, F32, False, False), (500, 400, 5000, F32, True, True),
+              (1000, 800, 128, F64, True, False), (2000, 2000, 128, F64, True, False), (4000, 2000, 128, F64, False, False)]
+
+
+@pytest.mark.parametrize("case", SRHT_SHORT)
+def test_srht_short_columns(fake, case):
+    """A few short columns with many samples have a CTA each; otherwise several share one."""
+    L, s, nv, dtype, expand, compress = case
+    ctx = fake.context()
+    sk = fake.sketch(ctx, "srht", s, L, dtype=dtype)
+    for adjoint, column in ((True, expand), (False, compress)):
+        fake.reset()
+        assert fake.mul(ctx, sk, (s, L, nv), LEFT, adjoint=adjoint) == 0
+        kernel = ("srht_expand_kernel" if adjoint else "srht_small_kernel") if column else "wht_near_kernel"
+        assert len(fake.launches()) == 1 and kernel in fake.launches()[0], (adjoint, fake.launches())
+
+
+@pytest.mark.parametrize("dtype", [F32, F64])
+@pytest.mark.parametrize("adjoint", [False, True])
+def test_srht_short_gpu_sizes_run_both_kernels(fake, dtype, adjoint):
+    ctx = fake.context()
+    seen = set()
+    for L, s, nv in srht_short.SHORT:
+        for card in (LEFT, RIGHT):
+            sk = fake.sketch(ctx, "srht", s, L, dtype=dtype, card=card)
+            fake.reset()
+            assert fake.mul(ctx, sk, (s, L, nv), card, adjoint=adjoint) == 0
+            seen.update(name for name in ("near", "srht_expand", "srht_small") for k in fake.launches() if name in k)
+    assert seen == {"near", "srht_expand" if adjoint else "srht_small"}
