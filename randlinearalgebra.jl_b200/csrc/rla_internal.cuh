@@ -335,9 +335,8 @@ struct rla_sketch {
     int32_t *rows = nullptr;       // [s] sampled padded rows (op)
     uint32_t *signbits = nullptr;  // [ceil(N/32)] bit r = 1 means +1
     uint4 *sign_tl = nullptr;      // fused compress kernel: per (chunk, thread) sign bits in register order (FP32: 64 as uint2, FP64: 128)
-    int32_t *p2_ptr = nullptr;     // expand tables: per low-bit position, samples sorted
+    int32_t *p2_ptr = nullptr;     // expand tables: per position of a short column, its first sample in p2_list
     int32_t *p2_list = nullptr;    // [2s] samples by low position, then their rows in that order
-    int64_t chunk = 0;             // WHT chunk length used by the expand tables
     // FJLT: compress matrix Kc (s x N) in CSR, and its transpose (N x s) in CSR
     int32_t *k_ptr = nullptr, *k_col = nullptr;
     void *k_val = nullptr;

@@ -139,7 +139,7 @@ cudaError_t cudaMemcpy(void *d, const void *s, size_t n, cudaMemcpyKind) {
     return cudaSuccess;
 }
 cudaError_t cudaMemcpyAsync(void *d, const void *s, size_t n, cudaMemcpyKind, cudaStream_t st) {
-    note("cudaMemcpyAsync %p stream=%p", d, (void *)st);
+    note("cudaMemcpyAsync %p stream=%p bytes=%zu", d, (void *)st, n);
     memcpy(d, s, n);
     return cudaSuccess;
 }

@@ -207,3 +207,17 @@ def test_wide_strided_compress_keeps_no_scratch_in_a_capture(fake):
         assert fake.mul(ctx, sk, (s, L, nv), RIGHT, wait=False) == 0
         k = fake.launches()
         assert any("tile_compress" in x for x in k) and any("tile_reduce" in x for x in k) == (not capturing)
+
+
+@pytest.mark.parametrize("dtype", [F32, F64])
+@pytest.mark.parametrize("L,s", [(1 << 20, 40), (100003, 300), (5000, 40), (4096, 40), (700, 9)])
+def test_srht_tables_are_as_short_as_the_samples(fake, dtype, L, s):
+    """A draw copies tables of its samples to the device, and of a short column's positions."""
+    ctx = fake.context()
+    fake.reset()
+    sk = fake.sketch(ctx, "srht", s, L, dtype=dtype)
+    copied = sum(int(ln.split("bytes=")[1]) for ln in fake.log() if ln.startswith("cudaMemcpyAsync"))
+    padded = 1 << (L - 1).bit_length()
+    assert copied <= 4 * (3 * s + (padded + 1 if padded <= 4096 else 0))
+    fake.lib.rla_sketch_destroy(sk)
+    fake.lib.rla_ctx_destroy(ctx)
