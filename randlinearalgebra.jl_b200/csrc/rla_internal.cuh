@@ -102,9 +102,10 @@ inline cudaError_t set_smem_max(K kern) {
 // shared by its contexts and keeps at most 256 MB of freed memory mapped (given back with the
 // last context): a cudaMalloc / cudaFree pair of a few MB takes 100-300 us, a solve on a new
 // problem makes twenty.  Allocated in the order of ctx->stream: other streams may use it once that
-// stream has been waited for.  dev_free: after the work that uses the memory has completed.
+// stream has been waited for.  Buffers that the pool could not keep come from cudaMalloc.  dev_free: in
+// the order of the stream; on the legacy stream after the work that uses the memory has completed.
 cudaError_t dev_alloc(rla_ctx *ctx, void **p, size_t bytes);
-void dev_free(void *p);
+void dev_free(void *p, cudaStream_t stream = nullptr);
 // Counts the device's contexts; the last one gives the pool's free memory back.
 void pool_contexts(int device, int change);
 template <class P>

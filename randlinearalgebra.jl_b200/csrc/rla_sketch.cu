@@ -355,9 +355,9 @@ static int fjlt_build(rla_ctx *ctx, rla_sketch *sk, const Rng &rng) {
     std::vector<int32_t> hp(s + 1, 0);
     for (int64_t i = 0; i < s; ++i) hp[i + 1] = hp[i] + hc[i];
     int64_t nnz = hp[s];
-    if (sk->k_ptr) cudaFreeAsync(sk->k_ptr, ctx->stream);
-    if (sk->k_col) cudaFreeAsync(sk->k_col, ctx->stream);
-    if (sk->k_val) cudaFreeAsync(sk->k_val, ctx->stream);
+    dev_free(sk->k_ptr, ctx->stream);
+    dev_free(sk->k_col, ctx->stream);
+    dev_free(sk->k_val, ctx->stream);
     RLA_CUDA_TRY(ctx, cudaMallocAsync(&sk->k_ptr, sizeof(int32_t) * (s + 1), ctx->stream));
     RLA_CUDA_TRY(ctx, cudaMallocAsync(&sk->k_col, sizeof(int32_t) * std::max<int64_t>(nnz, 1), ctx->stream));
     RLA_CUDA_TRY(ctx, cudaMallocAsync(&sk->k_val, sizeof(T) * std::max<int64_t>(nnz, 1), ctx->stream));
@@ -394,9 +394,9 @@ static int fjlt_transpose(rla_ctx *ctx, rla_sketch *sk) {
             tr[d] = (int32_t)i;
             tv[d] = v[k];
         }
-    if (sk->kt_ptr) cudaFreeAsync(sk->kt_ptr, ctx->stream);
-    if (sk->kt_row) cudaFreeAsync(sk->kt_row, ctx->stream);
-    if (sk->kt_val) cudaFreeAsync(sk->kt_val, ctx->stream);
+    dev_free(sk->kt_ptr, ctx->stream);
+    dev_free(sk->kt_row, ctx->stream);
+    dev_free(sk->kt_val, ctx->stream);
     RLA_CUDA_TRY(ctx, cudaMallocAsync(&sk->kt_ptr, sizeof(int32_t) * (N + 1), ctx->stream));
     RLA_CUDA_TRY(ctx, cudaMallocAsync(&sk->kt_row, sizeof(int32_t) * std::max<int64_t>(nnz, 1), ctx->stream));
     RLA_CUDA_TRY(ctx, cudaMallocAsync(&sk->kt_val, sizeof(T) * std::max<int64_t>(nnz, 1), ctx->stream));
@@ -511,7 +511,7 @@ static int build_meta(rla_ctx *ctx, rla_sketch *sk) {
     if (tot >= (int64_t(1) << 23)) return set_error(ctx, RLA_E_UNSUPPORTED, "too many deferred rounds");
     if (tot > sk->extra_rounds_cap) {
         // in stream order (cudaFree would return pool memory without waiting for its readers)
-        if (sk->extra) RLA_CUDA_TRY(ctx, cudaFreeAsync(sk->extra, ctx->stream));
+        dev_free(sk->extra, ctx->stream);
         sk->extra = nullptr;
         sk->extra_rounds_cap = 0;
         const int64_t cap = std::max<int64_t>(tot, 1) + tot / 4;
@@ -887,7 +887,7 @@ int rla_sketch_set_draws(rla_ctx *ctx, rla_sketch *sk, const int64_t *idx, const
             // reads the old matrix (cudaFree would return pool memory without waiting)
             RLA_CUDA_TRY(ctx, cudaDeviceSynchronize());
             for (void *p : {(void *)sk->k_ptr, (void *)sk->k_col, (void *)sk->k_val})
-                if (p) cudaFreeAsync(p, ctx->stream);
+                dev_free(p, ctx->stream);
             sk->k_ptr = sk->k_col = nullptr;
             sk->k_val = nullptr;
             RLA_CUDA_TRY(ctx, dev_alloc_t(ctx, &sk->k_ptr, (sk->s + 1) * 4));

@@ -209,6 +209,20 @@ def test_wide_strided_compress_keeps_no_scratch_in_a_capture(fake):
         assert any("tile_compress" in x for x in k) and any("tile_reduce" in x for x in k) == (not capturing)
 
 
+@pytest.mark.parametrize("s,L,large", [(1000, 10000, False), (1000, 90000, False), (1000, 101000, True), (2100, 100000, True)])
+def test_buffers_that_the_pool_cannot_keep_are_not_pool_memory(fake, s, L, large):
+    """The pool unmaps what it holds above its threshold, and maps it again for the next allocation."""
+    ctx = fake.context()
+    fake.reset()
+    sk = fake.sketch(ctx, "gaussian", s, L)
+    log = fake.log()
+    assert any(ln.startswith("cudaMalloc ") for ln in log) == large
+    fake.lib.rla_sketch_destroy(sk)
+    assert mismatched_releases(fake.log()) == [] and freed_while_queued(fake.log()) == []
+    assert any(ln.startswith("cudaFree ") for ln in fake.log()) == large
+    fake.lib.rla_ctx_destroy(ctx)
+
+
 @pytest.mark.parametrize("dtype", [F32, F64])
 @pytest.mark.parametrize("L,s", [(1 << 20, 40), (100003, 300), (5000, 40), (4096, 40), (700, 9)])
 def test_srht_tables_are_as_short_as_the_samples(fake, dtype, L, s):
