@@ -108,95 +108,141 @@ static bool bl_geometry(const rla_sketch *sk, BlGeom *g) {
     return true;
 }
 
-// One CTA per chunk: a stable counting sort by (window, warp, bucket).  Warp w counts and later
-// places rows [w*R/8, (w+1)*R/8) in increasing order; ranks inside a warp access come from
-// match_any, so the order of a bucket's entries is the order of the long indices.
+// One CTA per chunk: a stable counting sort by (window, warp, bucket).  All threads fetch the
+// entries' keys; each of H warps ranks the entries of R/H rows in increasing order against its own
+// counters (ranks inside a warp access come from match_any, so the order of a bucket's entries is
+// the order of the long indices); then all threads place them.  Entry while sorting: bits 0..13
+// key, 14..28 rank, 31 sign.
+constexpr int BL_KEY_BITS = 14;
+static_assert(BL_MAX_WIN * (BL_MAX_SW + BL_WARPS) <= 1 << BL_KEY_BITS && BL_R * BL_MAX_NNZ < 1 << (31 - BL_KEY_BITS), "entry fields");
 template <class T>
 __global__ void __launch_bounds__(BL_BUILD_WARPS * 32) bl_build_kernel(const int32_t *bucket, const uint8_t *negative,
-                                                                       int64_t L, int nnz, BlGeom g, uint32_t *words,
+                                                                       int64_t L, int nnz, BlGeom g, int H, uint32_t *words,
                                                                        int2 *lists) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int K = g.nwin * BL_WARPS * g.spw, nlist = g.nwin * BL_WARPS;
-    uint16_t *hist = reinterpret_cast<uint16_t *>(smem_raw);  // [8][K] counts, then offsets inside the bucket
-    uint16_t *tot = hist + BL_BUILD_WARPS * K;                // [K]
-    uint16_t *koff = tot + K;                                 // [K] first group of the bucket in its list
+    uint32_t *ent = reinterpret_cast<uint32_t *>(smem_raw);            // [R * nnz]
+    uint16_t *hist = reinterpret_cast<uint16_t *>(ent + BL_R * nnz);   // [H][K] counts, then offsets inside the bucket
+    uint16_t *koff = hist + H * K;                                     // [K] entries, then first group of the bucket in its list
     __shared__ int lstart[BL_MAX_WIN * BL_WARPS], lpart[BL_MAX_WIN * BL_WARPS], lslow[BL_MAX_WIN * BL_WARPS];
-    const int t = threadIdx.x, nt = blockDim.x, lane = t & 31, w = t >> 5;
+    __shared__ int all_words;
+    constexpr int nt = BL_BUILD_WARPS * 32;
+    const int t = threadIdx.x, lane = t & 31, w = t >> 5, gsh = g.gs == 4 ? 2 : 0;
     const int64_t chunk = blockIdx.x, row0 = chunk * BL_R;
-    for (int i = t; i < BL_BUILD_WARPS * K; i += nt) hist[i] = 0;
-    __syncthreads();
-    constexpr int rows_w = BL_R / BL_BUILD_WARPS;
-    const int rlo = w * rows_w;
-    const int rcnt = (int)max((int64_t)0, min((int64_t)rows_w, L - row0 - rlo));
-    const int ne = rcnt * nnz;
-    const int64_t base = (row0 + rlo) * nnz;
-    uint16_t *myh = hist + w * K;
+    const int rows = (int)min((int64_t)BL_R, L - row0), ne = rows * nnz, rows_w = BL_R / H;
+    const int64_t base = row0 * nnz;
     uint32_t *out = words + chunk * g.cap;
-    for (int pass = 0; pass < 2; ++pass) {
-        for (int i0 = 0; i0 < ne; i0 += 32) {
+    for (int i = t; i < H * K / 8; i += nt) reinterpret_cast<uint4 *>(hist)[i] = make_uint4(0, 0, 0, 0);
+    for (int i = t; i < ne; i += nt) {
+        const int jl = i / nnz;
+        const uint32_t b = (uint32_t)__ldg(bucket + base + i);
+        const int win = (int)(b / (uint32_t)g.sw);
+        const int vlb = (jl & (g.G - 1)) * g.sw + (int)b - win * g.sw;
+        const int list = win * BL_WARPS + (vlb & (BL_WARPS - 1));
+        ent[i] = (uint32_t)(list * g.spw + vlb / BL_WARPS) | ((uint32_t)__ldg(negative + base + i) << 31);
+    }
+    __syncthreads();
+    if (w < H) {
+        uint16_t *myh = hist + w * K;
+        const int hi = min((w + 1) * rows_w, rows) * nnz;
+        for (int i0 = w * rows_w * nnz; i0 < hi; i0 += 32) {
             const int i = i0 + lane;
-            const bool valid = i < ne;
-            const int jl = rlo + (valid ? i / nnz : 0);
-            const uint32_t b = valid ? (uint32_t)bucket[base + i] : 0u;
-            const int win = (int)(b / (uint32_t)g.sw);
-            const int vlb = (jl & (g.G - 1)) * g.sw + (int)b - win * g.sw;
-            const int list = win * BL_WARPS + (vlb & (BL_WARPS - 1));
-            const int key = list * g.spw + vlb / BL_WARPS;
+            const bool valid = i < hi;
+            const uint32_t e = valid ? ent[i] : 0u;
+            const int key = (int)(e & ((1u << BL_KEY_BITS) - 1u));
             const unsigned grp = __match_any_sync(FULL, valid ? key : -1 - lane);
             const int rank = __popc(grp & ((1u << lane) - 1u));
             const int before = valid ? myh[key] : 0;
             __syncwarp();
             if (valid && rank == 0) myh[key] = (uint16_t)(before + __popc(grp));
+            if (valid) ent[i] = e | ((uint32_t)(before + rank) << BL_KEY_BITS);
             __syncwarp();
-            if (pass == 1 && valid) {
-                const uint32_t neg = (uint32_t)negative[base + i];
-                const int r = before + rank, k = koff[key] + r / g.gs, part = lpart[list];
-                const int o = k / part, q = k - o * part;
-                const int gpw = 4 / g.gs;  // groups per 16-byte word of an octet
-                out[lstart[list] + (((q / gpw) * 4 + o) << 2) + (q % gpw) * g.gs + r % g.gs] =
-                    tile_off<T>(jl, 0) | ((uint32_t)(vlb * (BL_PITCH / 16)) << BL_BIN_SHIFT) | (neg << 31);
-            }
         }
-        if (pass == 1) break;
-        __syncthreads();
-        for (int k = t; k < K; k += nt) {  // counts -> exclusive offsets over the warps
-            int run = 0;
-#pragma unroll
-            for (int q = 0; q < BL_BUILD_WARPS; ++q) {
-                const int c = hist[q * K + k];
-                hist[q * K + k] = (uint16_t)run;
-                run += c;
-            }
-            tot[k] = (uint16_t)run;
+    }
+    __syncthreads();
+    for (int k = t; k < K; k += nt) {  // counts -> exclusive offsets over the warps
+        int run = 0;
+        for (int q = 0; q < H; ++q) {
+            const int c = hist[q * K + k];
+            hist[q * K + k] = (uint16_t)run;
+            run += c;
         }
-        __syncthreads();
-        for (int l = t; l < nlist; l += nt) {
-            int run = 0, most = 0;
-            for (int k = l * g.spw; k < (l + 1) * g.spw; ++k) {
-                const int ng = (tot[k] + g.gs - 1) / g.gs;
-                koff[k] = (uint16_t)run;
+        koff[k] = (uint16_t)run;
+    }
+    __syncthreads();
+    {  // first group of each bucket: P lanes per list, a segment of its keys each
+        const int P = g.nwin == 1 ? 16 : g.nwin == 2 ? 8 : g.nwin <= 4 ? 4 : 2;
+        const int l = t / P, seg = (g.spw + P - 1) / P;
+        const int k0 = l * g.spw + min(t % P * seg, g.spw), k1 = l * g.spw + min((t % P + 1) * seg, g.spw);
+        int run = 0, most = 0;
+        if (l < nlist)
+            for (int k = k0; k < k1; ++k) {
+                const int ng = (koff[k] + g.gs - 1) >> gsh;
                 run += ng;
                 most = max(most, ng);
             }
-            const int gpw = 4 / g.gs, part = ((run + 3) / 4 + gpw - 1) / gpw * gpw, slow = most > part;
-            lpart[l] = part;
-            lslow[l] = slow;
+        int before = run;  // inclusive over the list's lanes
+        for (int d = 1; d < P; d <<= 1) {
+            const int v = __shfl_up_sync(FULL, before, d, P), m = __shfl_xor_sync(FULL, most, d, P);
+            if (t % P >= d) before += v;
+            most = max(most, m);
         }
-        __syncthreads();
-        if (t == 0) {
-            int run = 0;
-            for (int l = 0; l < nlist; ++l) {
-                lstart[l] = run;
-                run += 4 * g.gs * lpart[l];
+        const int total = __shfl_sync(FULL, before, P - 1, P);
+        before -= run;
+        if (l < nlist) {
+            for (int k = k0; k < k1; ++k) {
+                const int ng = (koff[k] + g.gs - 1) >> gsh;
+                koff[k] = (uint16_t)before;
+                before += ng;
+            }
+            if (t % P == 0) {
+                const int gpw = 4 >> gsh, part = ((total + 3) / 4 + gpw - 1) / gpw * gpw;
+                lpart[l] = part;
+                lslow[l] = most > part;
             }
         }
-        __syncthreads();
-        for (int l = t; l < nlist; l += nt)
-            lists[chunk * nlist + l] = make_int2(lstart[l] / 16, lpart[l] * g.gs / 4 | (lslow[l] ? BL_SLOW : 0));
-        const int all = lstart[nlist - 1] + 4 * g.gs * lpart[nlist - 1];
-        const uint32_t fill = BL_ZERO_ROW | ((uint32_t)(g.sw * g.G * (BL_PITCH / 16)) << BL_BIN_SHIFT);
-        for (int i = t; i < all + BL_SLACK; i += nt) out[i] = fill;
-        __syncthreads();
+    }
+    __syncthreads();
+    if (w == 0) {  // first word of each list
+        constexpr int PER = BL_MAX_WIN * BL_WARPS / 32;
+        int len[PER], run = 0;
+#pragma unroll
+        for (int i = 0; i < PER; ++i) {
+            const int l = lane * PER + i;
+            len[i] = l < nlist ? 4 * g.gs * lpart[l] : 0;
+            run += len[i];
+        }
+        int before = run;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const int v = __shfl_up_sync(FULL, before, d);
+            if (lane >= d) before += v;
+        }
+        if (lane == 31) all_words = before;
+        before -= run;
+#pragma unroll
+        for (int i = 0; i < PER; ++i) {
+            if (lane * PER + i < nlist) lstart[lane * PER + i] = before;
+            before += len[i];
+        }
+    }
+    __syncthreads();
+    for (int l = t; l < nlist; l += nt)
+        lists[chunk * nlist + l] = make_int2(lstart[l] / 16, (lpart[l] * g.gs / 4) | (lslow[l] ? BL_SLOW : 0));
+    const uint32_t fill = BL_ZERO_ROW | ((uint32_t)(g.sw * g.G * (BL_PITCH / 16)) << BL_BIN_SHIFT);
+    for (int i = t; i < (all_words + BL_SLACK) / 4; i += nt)
+        reinterpret_cast<uint4 *>(out)[i] = make_uint4(fill, fill, fill, fill);
+    __syncthreads();
+    for (int i = t; i < ne; i += nt) {
+        const uint32_t e = ent[i];
+        const int jl = i / nnz, key = (int)(e & ((1u << BL_KEY_BITS) - 1u)), list = key / g.spw;
+        const int r = hist[jl / rows_w * K + key] + (int)((e & 0x7fffffffu) >> BL_KEY_BITS);
+        const int k = koff[key] + (r >> gsh), part = lpart[list];
+        const int o = k / part, q = k - o * part;
+        const int gpw = 4 >> gsh;  // groups per 16-byte word of an octet
+        const int vlb = (key - list * g.spw) * BL_WARPS + (list & (BL_WARPS - 1));
+        out[lstart[list] + (((q / gpw) * 4 + o) << 2) + (q % gpw) * g.gs + (r & (g.gs - 1))] =
+            tile_off<T>(jl, 0) | ((uint32_t)(vlb * (BL_PITCH / 16)) << BL_BIN_SHIFT) | (e & 0x80000000u);
     }
 }
 
@@ -207,10 +253,15 @@ int tile_plan_build(rla_ctx *ctx, rla_sketch *sk) {
     const int nlist = g.nwin * BL_WARPS, K = nlist * g.spw;
     if (!sk->bl_words) RLA_CUDA_TRY(ctx, dev_alloc_t(ctx, &sk->bl_words, sizeof(uint32_t) * (size_t)(g.nchunk * g.cap)));
     if (!sk->bl_lists) RLA_CUDA_TRY(ctx, dev_alloc_t(ctx, &sk->bl_lists, sizeof(int2) * (size_t)(g.nchunk * nlist)));
-    const size_t smem = sizeof(uint16_t) * (size_t)K * (BL_BUILD_WARPS + 2);
+    // Ranking warps: each has counters of its own for every key, which cost shared memory (CTAs per SM)
+    // and time to add up, while fewer warps rank one after another.  Update of 2^20 -> s, us, with
+    // 8 / 4 / 2 / 1: nnz 1, s = 1000 54 / 51 / 53 / 54, s = 4096 131 / 108 / 107 / 108, s = 8320 185 / 121 / 104 / 99;
+    // nnz 8, s = 1000 279 / 279 / 283 / 301, s = 8320 418 / 332 / 331 / 359; of 10^4 -> 1000, nnz 8: 43 / 45 / 56 / 75.
+    const int H = K <= 1100 ? 8 : K > 6000 && sk->nnz <= 2 ? 2 : 4;
+    const size_t smem = sizeof(uint32_t) * BL_R * sk->nnz + sizeof(uint16_t) * (size_t)K * (H + 1);
     auto go = [&](auto kern) -> int {
         RLA_CUDA_TRY(ctx, set_smem_max(kern));
-        kern<<<(unsigned)g.nchunk, BL_BUILD_WARPS * 32, smem, ctx->stream>>>(sk->bucket, sk->negative, sk->L, (int)sk->nnz, g,
+        kern<<<(unsigned)g.nchunk, BL_BUILD_WARPS * 32, smem, ctx->stream>>>(sk->bucket, sk->negative, sk->L, (int)sk->nnz, g, H,
                                                                              sk->bl_words, sk->bl_lists);
         return check_launch(ctx, "bl_build");
     };

@@ -5,6 +5,7 @@ import re
 import pytest
 
 import test_gpu_sparse_lift_sizes as lift
+import test_gpu_sparse_tile_windows as windows
 import test_gpu_srht_short as srht_short
 from fake_cuda import F32, F64, LEFT, RIGHT, fake  # noqa: F401 (fixture)
 
@@ -203,3 +204,28 @@ def test_srht_short_gpu_sizes_run_both_kernels(fake, dtype, adjoint):
             assert fake.mul(ctx, sk, (s, L, nv), card, adjoint=adjoint) == 0
             seen.update(name for name in ("near", "srht_expand", "srht_small") for k in fake.launches() if name in k)
     assert seen == {"near", "srht_expand" if adjoint else "srht_small"}
+
+
+@pytest.mark.parametrize("nnz,s,ctas", [(1, 1000, 8), (2, 1000, 7), (1, 4096, 4), (1, 8320, 4), (2, 8320, 4), (8, 8320, 2)])
+def test_tile_plans_of_many_buckets_leave_room_for_several_ctas(fake, nnz, s, ctas):
+    """The counters of the plan's ranking warps bound the CTAs per SM (228 KB of shared memory)."""
+    ctx = fake.context()
+    fake.reset()
+    fake.sketch(ctx, "count_sketch" if nnz == 1 else "sparse_sign", s, 1 << 17, card=RIGHT, nnz=nnz)
+    smem, = [int(re.search(r"smem=(\d+)", ln).group(1)) for ln in fake.log() if "bl_build" in ln]
+    assert 228 * 1024 // (smem + 3072) >= ctas
+
+
+@pytest.mark.parametrize("dtype", [F32, F64])
+@pytest.mark.parametrize("card", [LEFT, RIGHT])
+@pytest.mark.parametrize("row_major", [False, True])
+def test_window_sizes_run_the_tile_kernel_up_to_its_limits(fake, dtype, card, row_major):
+    ctx = fake.context()
+    for L, s, nnz, nv in windows.WINDOWS:
+        sk = fake.sketch(ctx, "count_sketch" if nnz == 1 else "sparse_sign", s, L, card=card, dtype=dtype, nnz=nnz)
+        fake.reset()
+        assert fake.mul(ctx, sk, (s, L, nv), card, row_a=row_major, row_c=row_major) == 0
+        strided = (card == LEFT) == row_major
+        tile = s <= 8320 and nnz <= 32 and (nnz > 1 or s <= 2080 or (card == RIGHT and strided))
+        assert ("tile_compress" in fake.launches()[0]) == tile, (L, s, nnz, nv, fake.launches())
+        fake.lib.rla_sketch_destroy(sk)
