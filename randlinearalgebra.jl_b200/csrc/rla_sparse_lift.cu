@@ -247,32 +247,81 @@ static int lift_lanes(const rla_ctx *ctx, const rla_sketch *sk, size_t *smem) {
     return 0;
 }
 
+// How a call is spread: fewer warps per CTA while that spreads a small call over more SMs (every CTA
+// stages X).
+struct LiftGrid {
+    int64_t tiles, blocks_per_tile, units;  // vector tiles, groups of a block per warp, their product
+    int warps, W;
+    int64_t stagings;  // most tiles that a CTA stages
+    static LiftGrid make(const rla_ctx *ctx, int64_t L, int64_t nv, int64_t C) {
+        LiftGrid g;
+        const int64_t nblk = ceil_div(L, 32);
+        g.tiles = ceil_div(nv, C);
+        g.warps = LIFT_WARPS;
+        while (g.warps > 4 && g.tiles * ceil_div(nblk, g.warps) < ctx->sm_count) g.warps /= 2;
+        g.blocks_per_tile = ceil_div(nblk, g.warps);
+        g.units = g.tiles * g.blocks_per_tile;
+        g.W = (int)std::min<int64_t>(ctx->sm_count, g.units);
+        g.stagings = ceil_div(ceil_div(g.units, g.W), g.blocks_per_tile);
+        return g;
+    }
+};
+
 // Whether staging pays, against a thread per output element (rla_sparse.cu).  Times of a call in
 // us, that kernel / this one, Float32 unless named:
-//  * Column-major results.  That kernel takes about (2 + nnz) ps more per output; staging costs
-//    about 8 us at s = 1000 (8 lanes), twice that from a row-major short operand: 30000 x 16,
-//    nnz 8, s = 1000: 33 / 38; 131072 x 32, nnz 1: 42 / 36.  A tile of 32 (Float64: 16) vectors
+//  * Column-major results of 1024 rows and more.  That kernel takes about (2 + nnz) ps more per output;
+//    staging costs about 8 us at s = 1000 (8 lanes), twice that from a row-major short operand: 30000 x
+//    16, nnz 8, s = 1000: 33 / 38; 131072 x 32, nnz 1: 42 / 36.  A tile of 32 (Float64: 16) vectors
 //    that is mostly empty costs as much as a full one: 2^20 long indices of nnz 8, 1 vector
 //    38 / 73, 4 vectors 81 / 72; nnz 1, 4 vectors 41 / 48, 8 vectors 57 / 49; nnz 3 (no unrolled
 //    loop) 8 vectors 67 / 73, 16 vectors 110 / 81.
-//  * Row-major results.  That kernel's blocks hold 128 vectors whatever their number is, so this
-//    one pays from two vectors on when there are enough long indices per staged row: 2^20 x 2,
-//    nnz 8: 300 / 95; 30000 x 32, nnz 8, s = 1000: 39 / 51; 131072 x 16, nnz 1: 66 / 42.
+//  * Other results by the sum of what each kernel spends (below).  Row-major: that kernel's blocks
+//    hold 128 vectors whatever their number is, and read a column-major operand across: 2^20 x 2,
+//    nnz 8: 300 / 95; 30000 x 32, nnz 8, s = 1000: 39 / 51; 131072 x 16, nnz 1: 66 / 42; 8000 x 500, nnz 16,
+//    s = 1000, column-major operand: 235 / 47.  Short columns: 50 x 100000, nnz 3 Float64 71 / 196, 200 x
+//    40000, nnz 8 131 / 79.
+//  * Rows off 32-byte boundaries leave neighbouring tiles parts of one sector, and the result
+//    does not stay in L2 until both are written: Float64, row-major operand, odd leading dimension,
+//    nnz 1, 30000 x 1000: s = 2000 160 / 296; s = 1000 with nnz 3 209 / 257, but nnz 8 272 / 243;
+//    column-major operand, s = 1 149 / 224, s = 1000 197 / 187.
 //  * Two lanes per entry, Float64: tiles of 4 vectors write 32-byte pieces of rows (2^20 x 64, nnz 1:
 //    302 / 401), and with nnz 3 the words of 2^20 long indices are read again for every four
-//    columns (2^20 x 64: 415 / 485; 131072 x 200: 226 / 178).
+//    columns (2^20 x 64: 415 / 485; 131072 x 200: 226 / 178); with beta 229508 x 198, nnz 1: 304 / 379.
 template <class T>
-static bool lift_pays(const rla_sketch *sk, int lpe, int64_t x_es, int64_t nv, int64_t y_es) {
+static bool lift_pays(const rla_sketch *sk, const LiftGrid &g, int lpe, int64_t x_es, int64_t nv, int64_t y_es, bool beta) {
     if (nv < 2) return false;
     const int64_t L = sk->L, nnz = sk->nnz, staged = sk->s * lpe;
     const bool unrolled = nnz == 1 || nnz == 2 || nnz == 4 || nnz == 8, narrow64 = sizeof(T) == 8 && lpe == 2;
-    if (y_es != 1) {
-        if (narrow64 && nv > 32 && nnz != 8) return false;
-        return L * ceil_div(nv, 128) * (8 + nnz) >= std::max<int64_t>(115 * staged, 300000);
+    const bool rows_in = x_es != 1, rows_out = y_es != 1;
+    if (rows_out) {
+        if (narrow64 && nv > 32 && nnz != 8 && rows_in) return false;
+        if (y_es * sizeof(T) % 32 != 0 && L * nv * (int64_t)sizeof(T) > 110000000 && g.tiles > 3) {
+            if (rows_in && (sizeof(T) == 8 ? lpe < 8 || nnz < 8 : lpe == 2)) return false;
+            if (!rows_in && sizeof(T) == 8 && nnz == 1 && (sk->s <= 300 || lpe < 8)) return false;
+        }
+    } else {
+        if (narrow64 && ((beta && nnz <= 2) || (!unrolled && nnz < 8 && L >= (1 << 19)))) return false;
+        if (L >= 1024) {
+            if (nv < (nnz >= 8 ? 4 : unrolled ? 8 : 16)) return false;
+            return L * nv * (2 + nnz) >= std::max<int64_t>(1000 * staged * (rows_in ? 2 : 1), 6000000);
+        }
     }
-    if (narrow64 && !unrolled && nnz < 8 && L >= (1 << 19)) return false;
-    if (nv < (nnz >= 8 ? 4 : unrolled ? 8 : 16)) return false;
-    return L * nv * (2 + nnz) >= std::max<int64_t>(1000 * staged * (x_es == 1 ? 1 : 2), 6000000);
+    // us: that kernel's blocks of 128 outputs, gathered values and output bytes; here the stagings, their
+    // rows (of one staging for row-major results, of all of them for short columns), bytes and values
+    // (least squares over 5200 calls of nnz 1 to 16, s up to 4000, both types)
+    struct Cost {
+        double block, value, byte, staging, row, byte_here, value_here;
+    };
+    static constexpr Cost costs[2][2] = {{{10.1e-5, 1.33e-6, 0.22e-6, 2.3, 0.72e-3, 0.13e-6, 0.041e-6},
+                                          {0.0, 2.52e-6, 0.31e-6, 2.3, 0.82e-3, 0.12e-6, 0.045e-6}},
+                                         {{16.2e-5, 2.14e-6, 0.20e-6, 1.5, 0.92e-3, 0.33e-6, 0.043e-6},
+                                          {19.9e-5, 0.56e-6, 0.28e-6, 2.0, 1.15e-3, 0.29e-6, 0.048e-6}}};
+    const Cost &c = costs[rows_out][rows_in];
+    const double values = (double)L * nv * nnz, bytes = (double)L * nv * sizeof(T);
+    const double there = c.block * (rows_out ? L * ceil_div(nv, 128) : ceil_div(L, 128) * nv) + c.value * values + c.byte * bytes;
+    const double here = c.staging * g.stagings + c.row * staged * (rows_out ? 1 : g.stagings) + c.byte_here * bytes +
+                        c.value_here * values * sizeof(T);
+    return there > here + (beta ? 6.0 : 1.5);  // beta: the old values add latency here
 }
 
 template <class T>
@@ -280,19 +329,16 @@ int sparse_lift(rla_ctx *ctx, const rla_sketch *sk, const T *X, int64_t x_es, in
                 int64_t y_es, int64_t y_vs, T alpha, T beta, bool beta_zero, bool *taken) {
     size_t smem = 0;
     const int lpe = lift_lanes<T>(ctx, sk, &smem);
-    *taken = lpe != 0 && lift_pays<T>(sk, lpe, x_es, nv, y_es);
+    *taken = false;
+    if (!lpe) return RLA_OK;
+    const LiftGrid g = LiftGrid::make(ctx, sk->L, nv, lpe * (16 / (int64_t)sizeof(T)));
+    *taken = lift_pays<T>(sk, g, lpe, x_es, nv, y_es, !beta_zero);
     if (!*taken) return RLA_OK;
-    const int64_t C = lpe * (16 / (int64_t)sizeof(T)), nblk = ceil_div(sk->L, 32);
-    // fewer warps per CTA while that spreads a small call over more SMs (every CTA stages X)
-    int warps = LIFT_WARPS;
-    while (warps > 4 && ceil_div(nv, C) * ceil_div(nblk, warps) < ctx->sm_count) warps /= 2;
-    const int64_t units = ceil_div(nv, C) * ceil_div(nblk, warps);
-    const int W = (int)std::min<int64_t>(ctx->sm_count, units);
     LiftParams<T> p{X, x_es, x_vs, sk->L, nv, sk->s, sk->bucket, sk->negative, (int)sk->nnz, ((int)sk->nnz + 1) / 2 * 2,
-                    Y, y_es, y_vs, alpha, beta, beta_zero, nblk, Split::make(units, W)};
+                    Y, y_es, y_vs, alpha, beta, beta_zero, ceil_div(sk->L, 32), Split::make(g.units, g.W)};
     auto go = [&](auto kern) -> int {
         RLA_CUDA_TRY(ctx, set_smem_max(kern));
-        kern<<<W, warps * 32, smem, ctx->stream>>>(p);
+        kern<<<g.W, g.warps * 32, smem, ctx->stream>>>(p);
         return check_launch(ctx, "sparse_lift");
     };
     auto by_nnz = [&](auto lanes) -> int {

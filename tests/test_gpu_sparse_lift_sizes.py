@@ -16,9 +16,9 @@ from test_gpu_sparse_tile import column_major
 pytestmark = pytest.mark.gpu
 
 #        L, s, nnz, nv, lanes per entry
-SIZES = [(20011, 40, 8, 37, 8), (120011, 1095, 1, 33, 8), (30011, 300, 3, 50, 8), (20001, 64, 16, 21, 8),
-         (10007, 64, 32, 19, 8), (60013, 1200, 2, 61, 4), (40009, 2380, 8, 131, 4), (60007, 3000, 4, 29, 2),
-         (62003, 4309, 8, 40, 2), (63001, 3000, 3, 30, 2)]
+SIZES = [(60011, 40, 8, 37, 8), (120011, 1095, 1, 33, 8), (60021, 300, 3, 50, 8), (40001, 64, 16, 21, 8),
+         (30007, 64, 32, 19, 8), (120027, 1200, 2, 61, 4), (40009, 2380, 8, 131, 4), (120007, 3000, 4, 29, 2),
+         (124003, 4309, 8, 40, 2), (126001, 3000, 3, 30, 2)]
 #          row-major Y, row-major C, padding, alpha, beta
 LAYOUTS = {"col": (False, False, 0, 1.0, 0.0), "col_odd": (False, False, 1, 0.5, -2.0), "row": (True, True, 0, 1.0, 0.0),
            "row_beta": (True, True, 0, 0.5, -2.0), "row_to_col": (True, False, 0, 1.0, 0.0),

@@ -229,3 +229,32 @@ def test_window_sizes_run_the_tile_kernel_up_to_its_limits(fake, dtype, card, ro
         tile = s <= 8320 and nnz <= 32 and (nnz > 1 or s <= 2080 or (card == RIGHT and strided))
         assert ("tile_compress" in fake.launches()[0]) == tile, (L, s, nnz, nv, fake.launches())
         fake.lib.rla_sketch_destroy(sk)
+
+
+#      L, s, nnz, nv, dtype, row-major Y, row-major C, leading dimension + , beta, staged
+EXPAND_COSTS = [
+    # row-major results: a column-major operand is read across by the kernel with a thread per output
+    (8000, 1000, 16, 500, F32, False, True, 0, 0.0, True), (1000, 1000, 8, 3000, F32, False, True, 0, 0.0, True),
+    (1030, 840, 16, 3863, F32, False, True, 1, 0.0, True), (27284, 3088, 16, 346, F64, False, True, 0, 0.0, True),
+    (8000, 1000, 3, 32, F32, False, True, 0, 0.0, False),
+    # rows off 32-byte boundaries, results beyond L2
+    (30000, 2000, 1, 1000, F64, True, True, 1, 0.0, False), (30000, 1000, 3, 1000, F64, True, True, 1, 0.0, False),
+    (30000, 300, 8, 1000, F64, True, True, 1, 0.0, True), (30000, 1, 1, 1000, F64, False, True, 1, 0.0, False),
+    (30000, 2000, 1, 1000, F64, True, True, 0, 0.0, True),
+    # short columns
+    (50, 50, 3, 100000, F64, False, False, 0, 0.0, False), (50, 10, 3, 100000, F32, False, False, 0, 0.0, False),
+    (200, 50, 8, 40000, F64, False, False, 0, 0.0, True), (155, 12, 12, 49361, F64, True, False, 0, 0.0, True),
+    # old values of the result
+    (3683, 23, 2, 181, F32, True, True, 0, 0.5, False), (1599, 18, 1, 848, F32, True, True, 0, 0.5, False),
+    (229508, 3223, 1, 198, F64, False, False, 0, 0.5, False), (229508, 3223, 1, 198, F64, False, False, 0, 0.0, True),
+]
+
+
+@pytest.mark.parametrize("case", EXPAND_COSTS)
+def test_expand_cost_rules(fake, case):
+    L, s, nnz, nv, dtype, row_y, row_c, pad, beta, staged = case
+    ctx = fake.context()
+    sk = fake.sketch(ctx, "sparse_sign", s, L, dtype=dtype, nnz=nnz)
+    fake.reset()
+    assert fake.mul(ctx, sk, (s, L, nv), LEFT, adjoint=True, row_a=row_y, row_c=row_c, pad=pad, beta=beta) == 0
+    assert len(fake.launches()) == 1 and ("lift_kernel" in fake.launches()[0]) == staged, fake.launches()
