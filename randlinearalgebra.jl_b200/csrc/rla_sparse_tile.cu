@@ -359,7 +359,8 @@ __device__ __forceinline__ double ld_ahead(const double *a) {
 // with 16-byte aligned rows, strided vectors at any alignment.
 enum { TILE_CONTIG = 0, TILE_SHIFT = 1, TILE_ROWS = 2, TILE_ROWS_ANY = 3 };
 
-template <class T, int MODE, int GS>
+// STEP: items of 16 bytes per thread whose old values (beta) are read before the first one is written.
+template <class T, int MODE, int GS, int STEP>
 __global__ void __launch_bounds__(BL_WARPS * 32, 1) tile_compress_kernel(TileParams<T> p) {
     using V = typename TileVec<T>::type;
     constexpr int VR = TileCfg<T>::VR, C = TileCfg<T>::C;
@@ -586,19 +587,37 @@ __global__ void __launch_bounds__(BL_WARPS * 32, 1) tile_compress_kernel(TilePar
         if (u0 <= gbeg && gbeg + nchunk <= u1) {
             // lanes along the dimension that is contiguous in memory
             const bool down = p.y_es == 1;
-            for (int i = t; i < (down ? (cnt + 31) / 32 * 32 : cnt) * 8; i += BL_WARPS * 32) {
-                const int b = down ? (i >> 8) * 32 + lane : i >> 3, q = down ? (i >> 5) & 7 : i & 7;
-                if (b >= cnt || q * VR >= nc) continue;
-                const V a = bin(b, q);
-                const T *ae = reinterpret_cast<const T *>(&a);
-                T *yp = p.Y + (lo + b) * p.y_es + (v0 + q * VR) * p.y_vs;
+            const int items = (down ? (cnt + 31) / 32 * 32 : cnt) * 8;
+            for (int i0 = t; i0 < items; i0 += BL_WARPS * 32 * STEP) {
+                T old[STEP][VR];
+                auto item = [&](int k, auto f) {  // f(bucket, 16 bytes of its bins, address, elements left)
+                    const int i = i0 + k * BL_WARPS * 32;
+                    const int b = down ? (i >> 8) * 32 + lane : i >> 3, q = down ? (i >> 5) & 7 : i & 7;
+                    if (b < cnt) f(b, q, p.Y + (lo + b) * p.y_es + (v0 + q * VR) * p.y_vs, nc - q * VR);
+                };
+                if constexpr (STEP > 1) {
 #pragma unroll
-                for (int e = 0; e < VR; ++e)
-                    if (q * VR + e < nc) {
-                        T r = p.alpha * ae[e];
-                        if (!p.beta_zero) r += p.beta * yp[e * p.y_vs];
-                        yp[e * p.y_vs] = r;
-                    }
+                    for (int k = 0; k < STEP; ++k)
+                        item(k, [&](int, int, const T *yp, int left) {
+#pragma unroll
+                            for (int e = 0; e < VR; ++e)
+                                if (e < left) old[k][e] = yp[e * p.y_vs];
+                        });
+                }
+#pragma unroll
+                for (int k = 0; k < STEP; ++k)
+                    item(k, [&](int b, int q, T *yp, int left) {
+                        if (left <= 0) return;
+                        const V a = bin(b, q);
+#pragma unroll
+                        for (int e = 0; e < VR; ++e)
+                            if (e < left) {
+                                T r = p.alpha * reinterpret_cast<const T *>(&a)[e];
+                                if constexpr (STEP > 1) r += p.beta * old[k][e];
+                                else if (!p.beta_zero) r += p.beta * yp[e * p.y_vs];
+                                yp[e * p.y_vs] = r;
+                            }
+                    });
             }
         } else {
             V *part = reinterpret_cast<V *>(p.partials + (int64_t)p.split.slot(blockIdx.x, gbeg) * p.g.sw * C);
@@ -706,12 +725,19 @@ int tile_compress(rla_ctx *ctx, const rla_sketch *sk, const T *X, int64_t x_es, 
         kern<<<W, BL_WARPS * 32, smem, ctx->stream>>>(p);
         return check_launch(ctx, "tile_compress");
     };
-    auto by_mode = [&](auto gs) -> int {
-        constexpr int GS = decltype(gs)::value;
-        if (contig) return vec ? go(tile_compress_kernel<T, TILE_CONTIG, GS>) : go(tile_compress_kernel<T, TILE_SHIFT, GS>);
-        return vec ? go(tile_compress_kernel<T, TILE_ROWS, GS>) : go(tile_compress_kernel<T, TILE_ROWS_ANY, GS>);
+    auto by_mode = [&](auto gs, auto step) -> int {
+        constexpr int GS = decltype(gs)::value, ST = decltype(step)::value;
+        if (contig) return vec ? go(tile_compress_kernel<T, TILE_CONTIG, GS, ST>) : go(tile_compress_kernel<T, TILE_SHIFT, GS, ST>);
+        return vec ? go(tile_compress_kernel<T, TILE_ROWS, GS, ST>) : go(tile_compress_kernel<T, TILE_ROWS_ANY, GS, ST>);
     };
-    RLA_TRY(g.gs == 4 ? by_mode(std::integral_constant<int, 4>()) : by_mode(std::integral_constant<int, 1>()));
+    // With beta a tile of few chunks waits longer for the old values, one by one, than for its
+    // sums (1002 x 43482 Float64 to 1002, nnz 4: 710 us a call, 527 with four at a time); their
+    // registers slow down the sums of longer ones (490312 x 99 Float32 from the right, s = 3194: 345 / 422).
+    using One = std::integral_constant<int, 1>;
+    using Four = std::integral_constant<int, 4>;
+    const bool ahead = !beta_zero && g.nchunk <= 16;
+    if (g.gs == 4) RLA_TRY(ahead ? by_mode(Four(), Four()) : by_mode(Four(), One()));
+    else RLA_TRY(ahead ? by_mode(One(), Four()) : by_mode(One(), One()));
     if (!shared) return RLA_OK;
     const int by_cut = groups > W - 1;
     const unsigned gx = (unsigned)(by_cut ? W - 1 : groups);

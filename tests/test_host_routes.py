@@ -258,3 +258,15 @@ def test_expand_cost_rules(fake, case):
     fake.reset()
     assert fake.mul(ctx, sk, (s, L, nv), LEFT, adjoint=True, row_a=row_y, row_c=row_c, pad=pad, beta=beta) == 0
     assert len(fake.launches()) == 1 and ("lift_kernel" in fake.launches()[0]) == staged, fake.launches()
+
+
+@pytest.mark.parametrize("L,ahead", [(600, True), (10240, True), (10241, False), (150001, False)])
+def test_tiles_of_few_chunks_read_old_values_ahead(fake, L, ahead):
+    """With beta a short tile reads four old values per thread before it writes; the registers would slow
+    down the sums of a long one, and there is nothing to read without beta."""
+    ctx = fake.context()
+    sk = fake.sketch(ctx, "sparse_sign", 300, L, nnz=4)
+    for beta in (0.0, 0.5):
+        fake.reset()
+        assert fake.mul(ctx, sk, (300, L, 40), LEFT, beta=beta) == 0
+        assert ("ELi4EEEvNS_10TileParams" in fake.launches()[0]) == (ahead and beta != 0), fake.launches()
