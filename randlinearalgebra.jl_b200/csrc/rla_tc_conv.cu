@@ -364,12 +364,18 @@ int gemm_f32_tc(rla_ctx *ctx, int64_t M, int64_t N, int64_t K, const float *A, i
         return set_error(ctx, RLA_E_UNSUPPORTED, "tensor-core GEMM: dimension above 2^31");
     // every tile of 64 columns converts its 128 rows of A again: above four of them splitting A once in
     // memory is faster (16000 x 512 to 1000 rows: 389 us converting, 363 us split before), unless K is
-    // so short that the FP64 partial tiles of the other kernel cost more (25756 x 4057, K = 131: 1170
-    // against 1426 us)
+    // so short that the FP64 partial tiles of the other kernel cost more (4096 x 30000, converting / split
+    // before: K = 16 615 / 1246 us, K = 128 1032 / 1415, K = 256 1446 / 1689)
     if (std::min(M, N) > 4 * CV_BN && K > 256)
         return gemm_f32_tc_presplit<TC>(ctx, M, N, K, A, lda, ta, B, ldb, tb, C, ldc, alpha, beta);
     int64_t rs = 1, cs = ldc;
-    if (N > M) {  // C' = op(B)' op(A)'
+    // The larger operand is converted, unless the other way round fills the tiles so much better that
+    // it makes up for splitting the larger one in memory (each tile saved for 64 rows more; 130 x 120,
+    // K = 258299: 2 x 2 or 1 x 3 tiles, 398 / 252 us a call)
+    const int64_t large = std::max(M, N), small = std::min(M, N);
+    auto tiles_of = [](int64_t m, int64_t n) { return ceil_div(m, TC_BM) * ceil_div(n, CV_BN); };
+    const bool turn = 64 * (tiles_of(large, small) - tiles_of(small, large)) > large - small;
+    if (turn ? N < M : N > M) {  // C' = op(B)' op(A)'
         std::swap(M, N);
         std::swap(A, B);
         std::swap(lda, ldb);
@@ -385,12 +391,26 @@ int gemm_f32_tc(rla_ctx *ctx, int64_t M, int64_t N, int64_t K, const float *A, i
     const int64_t budget = ctx->smem_optin - 1024 - 256 - (int64_t)CV_RAW * CV_RAW_BYTES;
     const int stages = (int)std::min<int64_t>(4, budget / cv_stage_bytes(NT));
     const size_t smem = 1024 + 256 + (size_t)stages * cv_stage_bytes(NT) + CV_RAW * CV_RAW_BYTES;
-    // split K while the grid stays within one CTA per SM (one more split puts a second round of CTAs
-    // behind the first: 16384 x 260 to 200 rows, 12 tiles: 117 us a call in 13 splits, 90 in 12), keeping whole chunks per split
-    const int64_t tiles = mt * ntl;
+    // K splits: the rounds of CTAs times the k-blocks of a split (1.2 us each) and of a CTA's start (4),
+    // and the sums of the partial tiles (4 us, 16 bytes an element at 4 TB/s).  16384 x 260 to 200 rows,
+    // 12 tiles: 117 us a call in 13 splits, 90 in 12; 11234 x 2778 to 244, 88 tiles: 465 in one, 321 in five.
+    // At most 64 MB of partial tiles; in a graph capture no more splits than one round holds (a
+    // captured scratch must not be grown later, and calls of a round or more never had one).
+    const int64_t tiles = mt * ntl, sms = ctx->sm_count;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    RLA_CUDA_TRY(ctx, cudaStreamIsCapturing(ctx->stream, &cap));
+    const int64_t most = cap != cudaStreamCaptureStatusNone ? std::max<int64_t>(1, sms / tiles) : 8 * sms / tiles;
     int64_t splits = 1;
-    if (tiles < ctx->sm_count)
-        splits = std::min<int64_t>(ctx->sm_count / tiles, std::max<int64_t>(1, nkb / (2 * CV_CHUNK)));
+    double best = 0.0;
+    for (int64_t sp = 1; sp <= std::min(most, nkb / (2 * CV_CHUNK)); ++sp) {
+        const int64_t len = ceil_div(ceil_div(nkb, sp), CV_CHUNK) * CV_CHUNK, n = ceil_div(nkb, len);
+        if (n > 1 && 8 * M * N * n > (int64_t)64 << 20) break;
+        const double us = 1.2 * (ceil_div(tiles * n, sms) * (std::min(len, nkb) + 4)) + (n > 1 ? 4.0 + 4e-6 * M * N * n : 0.0);
+        if (sp == 1 || us < best) {
+            best = us;
+            splits = n;
+        }
+    }
     const int64_t kbps = ceil_div(ceil_div(nkb, splits), CV_CHUNK) * CV_CHUNK;
     splits = ceil_div(nkb, kbps);
     void *ws = nullptr;

@@ -115,20 +115,36 @@ def test_srht_expand_writes_few_row_major_vectors_directly(fake, dtype, direct, 
 
 
 #       s, L, nv, tiles of 128 x 64, splits of K
-GAUSS_SPLITS = [(64, 16384, 100, 1, 64), (200, 16384, 260, 12, 12), (250, 60000, 260, 12, 12), (100, 16384, 100, 2, 64),
-                (64, 4096, 9600, 75, 1), (64, 4096, 9472, 74, 2)]
+GAUSS_SPLITS = [(64, 16384, 100, 1, 64), (200, 16384, 260, 10, 13), (250, 60000, 260, 10, 14), (100, 16384, 100, 2, 64),
+                (64, 4096, 9600, 75, 3), (64, 4096, 9472, 74, 2), (64, 4096, 18944, 148, 1), (244, 11234, 2778, 88, 5),
+                (130, 258299, 120, 3, 49), (64, 256, 9600, 75, 1), (256, 4096, 60000, 1876, 1)]
 
 
 @pytest.mark.parametrize("case", GAUSS_SPLITS)
-def test_gaussian_k_splits_stay_in_one_round(fake, case):
-    """The K splits of a Gaussian product are not more CTAs than SMs."""
+def test_gaussian_k_splits_fill_whole_rounds(fake, case):
+    """The K splits of a Gaussian product leave no round of CTAs nearly empty."""
     s, L, nv, tiles, splits = case
     ctx = fake.context()
     sk = fake.sketch(ctx, "gaussian", s, L)
     fake.reset()
     assert fake.mul(ctx, sk, (s, L, nv), LEFT) == 0
     (x, y, _), = grids(fake.log(), "conv_gemm")
-    assert (x, y) == (tiles, splits) and x * y <= 148
+    assert (x, y) == (tiles, splits)
+    rounds = lambda n: -(-tiles * n // 148) / n
+    assert splits == 1 or rounds(splits) <= min(rounds(splits - 1), rounds(splits + 1)) * 1.1
+
+
+@pytest.mark.parametrize("case", [(64, 4096, 9600, 1), (244, 11234, 2778, 1), (64, 4096, 9472, 2)])
+def test_gaussian_takes_no_more_scratch_in_a_capture_than_one_round(fake, case):
+    s, L, nv, splits = case
+    ctx = fake.context()
+    sk = fake.sketch(ctx, "gaussian", s, L)
+    assert fake.mul(ctx, sk, (s, L, nv), LEFT) == 0
+    fake.reset()
+    fake.capturing(True)
+    assert fake.mul(ctx, sk, (s, L, nv), LEFT, wait=False) == 0
+    (_, y, _), = grids(fake.log(), "conv_gemm")
+    assert y == splits
 
 
 @pytest.mark.parametrize("s,nv", [(100, 100), (64, 100), (33, 7)])
