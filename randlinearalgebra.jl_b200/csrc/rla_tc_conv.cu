@@ -56,12 +56,28 @@ __device__ __forceinline__ void conv_warps(const ConvArgs &p, int t, uint32_t ba
                                            unsigned char *stage_gen, int m0, int kb0, int nkb, uint32_t empty0,
                                            uint32_t afull0) {
     const int lane = t & 31, c = t & 3;
+    // A group keeps its rows through all k-blocks: past the last row of A its place in every stage is
+    // zeroed once, and it is neither copied nor converted.
+    auto off = [&](int u) {  // in the tile: 64-byte rows (of box u when A is not K-major)
+        const int row = AK ? u * 32 + (t >> 2) : t >> 2;
+        return (AK ? 0u : (uint32_t)u * 2048u) + (uint32_t)row * 64u + (uint32_t)((c ^ ((row >> 1) & 3)) << 4);
+    };
+    auto live = [&](int u) { return (AK ? m0 + u * 32 + (t >> 2) : m0 + 32 * u + 8 * c) < p.M; };
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+        if (!live(u))
+            for (int s = 0; s < p.stages; ++s)
+#pragma unroll
+                for (int q = 0; q < NT; ++q)
+                    *reinterpret_cast<uint4 *>(stage_gen + (size_t)s * cv_stage_bytes(NT) + (size_t)q * TC_A_BYTES + off(u)) =
+                        make_uint4(0, 0, 0, 0);
     auto issue = [&](int kb) {
         if (kb < nkb) {
             const int k0 = (kb0 + kb) * TC_BK;
             const uint32_t slot = raw + (uint32_t)(kb % CV_RAW) * CV_RAW_BYTES + (uint32_t)t * 16u;
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
+                if (!live(u)) continue;
                 const int m = AK ? m0 + u * 32 + (t >> 2) : m0 + 32 * u + 8 * c;
                 const int k = AK ? k0 + 8 * c : k0 + (t >> 2);
                 const int valid = AK ? (m < p.M ? min(8, p.K - k) : 0) : (k < p.K ? min(8, p.M - m) : 0);
@@ -92,16 +108,15 @@ __device__ __forceinline__ void conv_warps(const ConvArgs &p, int t, uint32_t ba
         unsigned char *st = stage_gen + (size_t)s * cv_stage_bytes(NT);
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
+            if (!live(u)) continue;
             const float4 a = *reinterpret_cast<const float4 *>(slot + u * 4096);
             const float4 b = *reinterpret_cast<const float4 *>(slot + u * 4096 + 2048);
             const float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
             uint4 o[NT];
             split_terms8<NT>(v, o);
-            const int row = AK ? u * 32 + (t >> 2) : t >> 2;  // 64-byte row of the tile (of box u when not K-major)
-            const uint32_t off = (AK ? 0u : (uint32_t)u * 2048u) + (uint32_t)row * 64u + (uint32_t)((c ^ ((row >> 1) & 3)) << 4);
 #pragma unroll
             for (int q = 0; q < NT; ++q)
-                *reinterpret_cast<uint4 *>(st + (size_t)q * TC_A_BYTES + off) = o[q];
+                *reinterpret_cast<uint4 *>(st + (size_t)q * TC_A_BYTES + off(u)) = o[q];
         }
         // the MMAs read the tile through the async proxy
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
