@@ -286,3 +286,13 @@ def test_tiles_of_few_chunks_read_old_values_ahead(fake, L, ahead):
         fake.reset()
         assert fake.mul(ctx, sk, (300, L, 40), LEFT, beta=beta) == 0
         assert ("ELi4EEEvNS_10TileParams" in fake.launches()[0]) == (ahead and beta != 0), fake.launches()
+
+
+@pytest.mark.parametrize("kind,s,L", [("srht", 5610, 22574), ("fjlt", 40, 5000), ("fjlt", 40, 60000)])
+def test_transforms_with_beta_read_old_values_ahead(fake, kind, s, L):
+    ctx = fake.context()
+    sk = fake.sketch(ctx, kind, s, L)
+    for beta in (0.0, 0.5):
+        fake.reset()
+        assert fake.mul(ctx, sk, (s, L, 6), LEFT, adjoint=True, beta=beta) == 0
+        assert ("ELi2EEEvNS_9WhtParams" in fake.launches()[-1] or "ELi2EEEvNS_9WhtParamsIT_EEi" in fake.launches()[-1]) == (beta != 0)
