@@ -1124,12 +1124,12 @@ int srht_expand(rla_ctx *ctx, const rla_sketch *sk, const T *X, int64_t x_es, in
     p.beta_zero = beta == 0.0;
     const int64_t nb = std::min<int64_t>(wht_batch<T>(sk->N, nv), 65535 * 32);
     // not for a few vectors, whose 32-wide tiles are mostly empty (2^20 long, direct / staged in us:
-    // Float32 x 2 38 / 122, x 12 108 / 139, x 16 144 / 145, x 32 600 / 271; Float64 x 12 118 / 273, x 16
-    // 359 / 285), nor in a graph capture: the graph would keep the scratch after a later call had
-    // grown it
+    // Float32 x 2 47 / 132, x 12 156 / 200, x 16 214 / 228, x 32 600 / 271; Float64 x 12 243 / 427, x 16
+    // 486 / 486; with beta Float32 x 6 131 / 163, x 12 248 / 214; 22574 x 6 from 5610 55 / 52, with beta
+    // 60 / 53), nor in a graph capture: the graph would keep the scratch after a later call had grown it
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     RLA_CUDA_TRY(ctx, cudaStreamIsCapturing(ctx->stream, &cap));
-    if (y_es == 1 || nv <= (sizeof(T) == 4 ? 16 : 12) || cap != cudaStreamCaptureStatusNone)
+    if (y_es == 1 || nv <= (sk->L < 65536 ? 3 : beta != 0.0 ? 6 : sizeof(T) == 4 ? 16 : 12) || cap != cudaStreamCaptureStatusNone)
         return launch_near<T, WHT_IN_SAMPLES, WHT_OUT_Y>(ctx, p);
     void *w;
     RLA_TRY(scratch_get(ctx, (size_t)(sk->N * nb) * sizeof(T), &w));
