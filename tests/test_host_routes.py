@@ -6,6 +6,7 @@ import pytest
 
 import test_gpu_sparse_lift_sizes as lift
 import test_gpu_sparse_tile_windows as windows
+import test_gpu_presplit as presplit
 import test_gpu_srht_short as srht_short
 from fake_cuda import F32, F64, LEFT, RIGHT, fake  # noqa: F401 (fixture)
 
@@ -296,3 +297,20 @@ def test_transforms_with_beta_read_old_values_ahead(fake, kind, s, L):
         fake.reset()
         assert fake.mul(ctx, sk, (s, L, 6), LEFT, adjoint=True, beta=beta) == 0
         assert ("ELi2EEEvNS_9WhtParams" in fake.launches()[-1] or "ELi2EEEvNS_9WhtParamsIT_EEi" in fake.launches()[-1]) == (beta != 0)
+
+
+@pytest.mark.parametrize("adjoint", [False, True])
+@pytest.mark.parametrize("card", [LEFT, RIGHT])
+def test_presplit_sizes_are_split_beforehand(fake, card, adjoint):
+    """Both result dimensions and the inner one above 256: the operands are split in memory."""
+    ctx = fake.context()
+    other = 0
+    for L, s, nv in presplit.SPLITS + [(256, 300, 300), (300, 256, 300), (300, 300, 256)]:
+        sk = fake.sketch(ctx, "gaussian", s, L, card=card)
+        fake.reset()
+        assert fake.mul(ctx, sk, (s, L, nv), card, adjoint=adjoint) == 0
+        before = min(s, L, nv) > 256
+        assert any("tc_gemm_f64acc" in k for k in fake.launches()) == before, (L, s, nv, fake.launches())
+        other += any("conv_gemm" in k for k in fake.launches())
+        fake.lib.rla_sketch_destroy(sk)
+    assert other == 3
