@@ -48,7 +48,7 @@ template <class T>
 static int dense_gemm(rla_ctx *ctx, int64_t M, int64_t N, int64_t K, const T *A, int64_t lda, int ta, const T *B,
                       int64_t ldb, int tb, T *C, int64_t ldc, double alpha, double beta) {
     if constexpr (std::is_same<T, float>::value)
-        return gemm_f32_tc<float>(ctx, M, N, K, A, lda, ta, B, ldb, tb, C, ldc, alpha, beta);
+        return gemm_f32_tc(ctx, M, N, K, A, lda, ta, B, ldb, tb, C, ldc, alpha, beta);
     else
         return gemm<T, T, T, double>(ctx, M, N, K, A, lda, ta, B, ldb, tb, C, ldc, alpha, beta);
 }

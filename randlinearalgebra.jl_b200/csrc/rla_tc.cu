@@ -1069,16 +1069,15 @@ int tc_gemm_f64acc(rla_ctx *ctx, int64_t M, int64_t N, int64_t K, const bf16 *co
     return check_launch(ctx, "splitk_reduce");
 }
 
-// C (M x N, ld ldc, TC) = alpha * op(A) * op(B) + beta * C for Float32 A and B on the
+// C (M x N, ld ldc) = alpha * op(A) * op(B) + beta * C for Float32 A and B on the
 // tensor cores with three BF16 terms per operand and FP64 accumulation across k-chunks (an
 // FP32-accurate product).  op(A) may be
 // A or A' (both layouts are read by TMA); op(B) must be K-major for the MMA, so B' (tb = 1)
 // is transposed while it is split.  The split copies come from the context's memory pool.
-template <class TC>
 int gemm_f32_tc_presplit(rla_ctx *ctx, int64_t M, int64_t N, int64_t K, const float *A, int64_t lda, int ta, const float *B,
-                int64_t ldb, int tb, TC *C, int64_t ldc, double alpha, double beta) {
+                int64_t ldb, int tb, float *C, int64_t ldc, double alpha, double beta) {
     if (M <= 0 || N <= 0) return RLA_OK;
-    if (K <= 0) return gemm<float, float, TC, double>(ctx, M, N, K, A, lda, ta, B, ldb, tb, C, ldc, alpha, beta);
+    if (K <= 0) return gemm<float, float, float, double>(ctx, M, N, K, A, lda, ta, B, ldb, tb, C, ldc, alpha, beta);
     const int64_t a_rows = ta ? K : M, a_cols = ta ? M : K;
     const int64_t lda2 = ceil_div(a_rows, 8) * 8, ldb2 = ceil_div(K, 8) * 8;
     const size_t na = (size_t)lda2 * a_cols, nb = (size_t)ldb2 * N;
@@ -1091,16 +1090,12 @@ int gemm_f32_tc_presplit(rla_ctx *ctx, int64_t M, int64_t N, int64_t K, const fl
                               : split_terms_launch<3>(ctx, B, K, N, ldb, 0, b3, ldb2);
     if (rc == RLA_OK) {
         const bf16 *ac[3] = {a3[0], a3[1], a3[2]}, *bc[3] = {b3[0], b3[1], b3[2]};
-        rc = tc_gemm_f64acc<TC>(ctx, M, N, K, ac, lda2, ta, bc, ldb2, C, ldc, alpha, beta);
+        rc = tc_gemm_f64acc<float>(ctx, M, N, K, ac, lda2, ta, bc, ldb2, C, ldc, alpha, beta);
     }
     cudaFreeAsync(buf, ctx->stream);
     return rc;
 }
 
-template int gemm_f32_tc_presplit<float>(rla_ctx *, int64_t, int64_t, int64_t, const float *, int64_t, int, const float *,
-                                        int64_t, int, float *, int64_t, double, double);
-template int gemm_f32_tc_presplit<double>(rla_ctx *, int64_t, int64_t, int64_t, const float *, int64_t, int, const float *,
-                                         int64_t, int, double *, int64_t, double, double);
 template int tc_gemm_f64acc<float>(rla_ctx *, int64_t, int64_t, int64_t, const bf16 *const *, int64_t, int, const bf16 *const *,
                                    int64_t, float *, int64_t, double, double);
 template int tc_gemm_f64acc<double>(rla_ctx *, int64_t, int64_t, int64_t, const bf16 *const *, int64_t, int,

@@ -52,14 +52,12 @@ int tc_gemm_bf16x3(rla_ctx *ctx, int64_t M, int64_t N, int64_t K, const bf16 *Ah
 // C (M x N, ld ldc) = alpha * op(A) * op(B) + beta * C for Float32 column-major A, B with an
 // FP32-accurate product on the tensor cores (three BF16 terms per operand, six MMAs per
 // k-step, FP64 accumulation across k-chunks).  Asynchronous.
-template <class TC>
 int gemm_f32_tc(rla_ctx *ctx, int64_t M, int64_t N, int64_t K, const float *A, int64_t lda, int ta, const float *B,
-                int64_t ldb, int tb, TC *C, int64_t ldc, double alpha, double beta);
+                int64_t ldb, int tb, float *C, int64_t ldc, double alpha, double beta);
 
 // The same product with both operands split into BF16 terms in memory beforehand.
-template <class TC>
 int gemm_f32_tc_presplit(rla_ctx *ctx, int64_t M, int64_t N, int64_t K, const float *A, int64_t lda, int ta, const float *B,
-                         int64_t ldb, int tb, TC *C, int64_t ldc, double alpha, double beta);
+                         int64_t ldb, int tb, float *C, int64_t ldc, double alpha, double beta);
 
 // C = alpha * op(A) * B + beta * C from three BF16 terms per operand (K-major B), FP64
 // accumulation across chunks of four k-blocks.  Asynchronous.

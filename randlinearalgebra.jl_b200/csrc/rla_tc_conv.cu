@@ -1,11 +1,11 @@
 // rla_tc_conv.cu -- FP32-accurate tensor-core products whose large operand is split into BF16 terms
 // inside the kernel.
 //
-// C = alpha * op(A) * B + beta * C with NT BF16 terms per operand (t0 = bf16(x), t1 = bf16(x - t0),
+// C = alpha * op(A) * B + beta * C with three BF16 terms per operand (t0 = bf16(x), t1 = bf16(x - t0),
 // ...) and FP64 accumulation across chunks of four k-blocks, the products and their order as in
 // tc_gemm_f64acc_kernel (rla_tc.cu).  There the terms of A come from HBM: splitting reads 4 bytes
-// and writes 2 NT per element, and the product reads the 2 NT again.  Here four converter warps
-// copy A's Float32 tile ahead with cp.async (4 k-blocks of 16 KB in flight), turn it into the
+// and writes 6 per element, and the product reads the 6 again.  Here four converter warps
+// copy A's Float32 tile ahead with cp.async (three k-blocks of 16 KB), turn it into the
 // terms and store them where TMA would have put them (64-byte swizzle), so A is read once, at any
 // alignment.  B, the small operand, is split beforehand and loaded by TMA.
 //
@@ -23,15 +23,15 @@ namespace rla {
 constexpr int CV_THREADS = 512, CV_BN = 64, CV_CHUNK = 4, CV_RAW = 4, CV_EPI_WARPS = 8;
 constexpr uint32_t CV_RAW_BYTES = TC_BM * TC_BK * 4;  // 16 KB per k-block of A
 constexpr uint32_t CV_B_BYTES = CV_BN * TC_BK * 2;
-constexpr uint32_t cv_tmem_cols(int NT) { return NT >= 3 ? 512u : (NT == 2 ? 256u : 128u); }
-constexpr uint32_t cv_stage_bytes(int NT) { return NT * (TC_A_BYTES + CV_B_BYTES); }
+constexpr int NT = 3;  // BF16 terms per operand
+constexpr uint32_t CV_TMEM_COLS = 512, CV_STAGE_BYTES = NT * (TC_A_BYTES + CV_B_BYTES);
 
 struct ConvArgs {
     const float *A;  // a_kmajor: element (m, k) at A[k + m*lda]; else at A[m + k*lda]
     int64_t lda;
     int a_vec;       // every 8-element group of A starts on 16 bytes
     int M, N, K;
-    void *out, *out2;  // element (m, n) at out[m*rs + n*cs]; out2 (optional) likewise
+    void *out;  // element (m, n) at out[m*rs + n*cs]
     int64_t rs, cs;
     int out_f64;
     double alpha, beta;  // beta: read and scaled when beta_on
@@ -51,8 +51,8 @@ __device__ __forceinline__ void cp_async4_zfill(uint32_t dst, const void *src, i
 // Converter thread t of 128: four groups of 8 elements of each k-block, in the order in which
 // consecutive lanes read consecutive memory.  A group's raw values stay private to the thread,
 // so waiting for its own copies is enough.
-template <int NT, int AK>
-__device__ __forceinline__ void conv_warps(const ConvArgs &p, int t, uint32_t base, uint32_t raw, unsigned char *raw_gen,
+template <int AK>
+__device__ __forceinline__ void conv_warps(const ConvArgs &p, int t, uint32_t raw, unsigned char *raw_gen,
                                            unsigned char *stage_gen, int m0, int kb0, int nkb, uint32_t empty0,
                                            uint32_t afull0) {
     const int lane = t & 31, c = t & 3;
@@ -69,7 +69,7 @@ __device__ __forceinline__ void conv_warps(const ConvArgs &p, int t, uint32_t ba
             for (int s = 0; s < p.stages; ++s)
 #pragma unroll
                 for (int q = 0; q < NT; ++q)
-                    *reinterpret_cast<uint4 *>(stage_gen + (size_t)s * cv_stage_bytes(NT) + (size_t)q * TC_A_BYTES + off(u)) =
+                    *reinterpret_cast<uint4 *>(stage_gen + (size_t)s * CV_STAGE_BYTES + (size_t)q * TC_A_BYTES + off(u)) =
                         make_uint4(0, 0, 0, 0);
     auto issue = [&](int kb) {
         if (kb < nkb) {
@@ -105,7 +105,7 @@ __device__ __forceinline__ void conv_warps(const ConvArgs &p, int t, uint32_t ba
         if (!__all_sync(FULL, mbar_wait(empty0 + 8u * (uint32_t)s, ph ^ 1u, p.status, p.wait_ns))) break;
         asm volatile("cp.async.wait_group %0;" ::"n"(CV_RAW - 1) : "memory");
         const unsigned char *slot = raw_gen + (size_t)(kb % CV_RAW) * CV_RAW_BYTES + t * 16;
-        unsigned char *st = stage_gen + (size_t)s * cv_stage_bytes(NT);
+        unsigned char *st = stage_gen + (size_t)s * CV_STAGE_BYTES;
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
             if (!live(u)) continue;
@@ -127,7 +127,6 @@ __device__ __forceinline__ void conv_warps(const ConvArgs &p, int t, uint32_t ba
 }
 
 // The 128 x 64 tile (m0, n0) over k-blocks kb0 .. kb0 + nkb - 1.
-template <int NT>
 __device__ __forceinline__ void conv_cta(const CUtensorMap *mb, const ConvArgs &p, int a_kmajor, int m0, int n0, int kb0,
                                          int nkb) {
     extern __shared__ unsigned char smem_raw[];
@@ -135,7 +134,7 @@ __device__ __forceinline__ void conv_cta(const CUtensorMap *mb, const ConvArgs &
     const uint32_t raw0 = smem_u32(smem_raw);
     const uint32_t base = (raw0 + 1023u) & ~1023u;
     unsigned char *gen = smem_raw + (base - raw0);
-    const uint32_t ring = base + (uint32_t)p.stages * cv_stage_bytes(NT);
+    const uint32_t ring = base + (uint32_t)p.stages * CV_STAGE_BYTES;
     const uint32_t bars = ring + CV_RAW * CV_RAW_BYTES;
     const uint32_t afull0 = bars, bfull0 = bars + 64u, empty0 = bars + 128u;  // up to 8 stages each
     auto accf_bar = [&](int x) { return bars + 192u + 8u * (uint32_t)x; };
@@ -162,7 +161,7 @@ __device__ __forceinline__ void conv_cta(const CUtensorMap *mb, const ConvArgs &
     }
     if (warp == 2) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tmem_slot),
-                     "r"(cv_tmem_cols(NT))
+                     "r"(CV_TMEM_COLS)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
@@ -179,7 +178,7 @@ __device__ __forceinline__ void conv_cta(const CUtensorMap *mb, const ConvArgs &
                 const uint32_t ph = (uint32_t)(kb / p.stages) & 1u;
                 if (!mbar_wait(empty0 + 8u * s, ph ^ 1u, p.status, p.wait_ns)) break;
                 issued = kb + 1;
-                const uint32_t b0 = base + (uint32_t)s * cv_stage_bytes(NT) + NT * TC_A_BYTES;
+                const uint32_t b0 = base + (uint32_t)s * CV_STAGE_BYTES + NT * TC_A_BYTES;
                 mbar_arrive_expect_tx(bfull0 + 8u * s, NT * CV_B_BYTES);
 #pragma unroll
                 for (int t = 0; t < NT; ++t)
@@ -194,9 +193,9 @@ __device__ __forceinline__ void conv_cta(const CUtensorMap *mb, const ConvArgs &
             // chunk c accumulates into TMEM columns (c & 1) * 64 NT; A_t x [B_0 | .. | B_(NT-1-t)] is
             // one MMA, column group u collects the products with B_u
             const uint32_t a_mn = a_kmajor ? 0 : 1;
-            const uint32_t idesc_n[3] = {idesc_bf16(TC_BM, CV_BN * NT, a_mn, 0),
-                                         idesc_bf16(TC_BM, CV_BN * (NT >= 2 ? NT - 1 : 1), a_mn, 0),
-                                         idesc_bf16(TC_BM, CV_BN * (NT >= 3 ? NT - 2 : 1), a_mn, 0)};
+            const uint32_t idesc_n[NT] = {idesc_bf16(TC_BM, CV_BN * NT, a_mn, 0),
+                                         idesc_bf16(TC_BM, CV_BN * 2, a_mn, 0),
+                                         idesc_bf16(TC_BM, CV_BN, a_mn, 0)};
             for (int kb = 0; kb < nkb; ++kb) {
                 const int c = kb / CV_CHUNK, x = c & 1;
                 const bool first = kb % CV_CHUNK == 0;
@@ -209,7 +208,7 @@ __device__ __forceinline__ void conv_cta(const CUtensorMap *mb, const ConvArgs &
                 if (!mbar_wait(bfull0 + 8u * s, ph, p.status, p.wait_ns)) break;
                 if (!mbar_wait(afull0 + 8u * s, ph, p.status, p.wait_ns)) break;
                 tc_fence_after();
-                const uint32_t st = base + (uint32_t)s * cv_stage_bytes(NT);
+                const uint32_t st = base + (uint32_t)s * CV_STAGE_BYTES;
                 const uint32_t d = tmem + (uint32_t)x * CV_BN * NT;
 #pragma unroll
                 for (int kk = 0; kk < TC_BK / 16; ++kk) {
@@ -301,8 +300,8 @@ __device__ __forceinline__ void conv_cta(const CUtensorMap *mb, const ConvArgs &
     } else if (warp >= 4 + CV_EPI_WARPS) {
         const int t = threadIdx.x - 32 * (4 + CV_EPI_WARPS);
         unsigned char *ring_gen = gen + (ring - base);
-        if (a_kmajor) conv_warps<NT, 1>(p, t, base, ring, ring_gen, gen, m0, kb0, nkb, empty0, afull0);
-        else conv_warps<NT, 0>(p, t, base, ring, ring_gen, gen, m0, kb0, nkb, empty0, afull0);
+        if (a_kmajor) conv_warps<1>(p, t, ring, ring_gen, gen, m0, kb0, nkb, empty0, afull0);
+        else conv_warps<0>(p, t, ring, ring_gen, gen, m0, kb0, nkb, empty0, afull0);
     }
     // every MMA issued (done_bar is committed on every path) has finished before the
     // accumulators are released
@@ -310,23 +309,21 @@ __device__ __forceinline__ void conv_cta(const CUtensorMap *mb, const ConvArgs &
     tc_fence_before();
     __syncthreads();
     if (warp == 2)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(cv_tmem_cols(NT)) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(CV_TMEM_COLS) : "memory");
 }
 
-template <int NT>
 struct ConvMaps {
     CUtensorMap b[NT];
 };
 
 // CTA (tile, split): tiles with the N index fastest, so that the CTAs that share rows of A run
 // together; split z writes its FP64 partial tile at out + z * stride.
-template <int NT>
 __global__ void __launch_bounds__(CV_THREADS, 1)
-conv_gemm_kernel(const __grid_constant__ ConvMaps<NT> maps, ConvArgs p, int a_kmajor, int ntl, int nkb, int kbps,
+conv_gemm_kernel(const __grid_constant__ ConvMaps maps, ConvArgs p, int a_kmajor, int ntl, int nkb, int kbps,
                  int64_t stride) {
     const int tile = blockIdx.x, kb0 = blockIdx.y * kbps;
     if (blockIdx.y) p.out = (double *)p.out + (int64_t)blockIdx.y * stride;
-    conv_cta<NT>(maps.b, p, a_kmajor, (tile / ntl) * TC_BM, (tile % ntl) * CV_BN, kb0, max(0, min(nkb - kb0, kbps)));
+    conv_cta(maps.b, p, a_kmajor, (tile / ntl) * TC_BM, (tile % ntl) * CV_BN, kb0, max(0, min(nkb - kb0, kbps)));
 }
 
 // C(m, n) (at C[m*rs + n*cs]) = alpha * sum_s P[s](m, n) + beta * C(m, n), P(m, n) at [m + n*M], splits
@@ -335,9 +332,8 @@ conv_gemm_kernel(const __grid_constant__ ConvMaps<NT> maps, ConvArgs p, int a_km
 // latency is all this kernel does (16384 x 100 to 100 rows: 50 us a call, 79 with four elements per
 // thread one after another).
 constexpr int CR_AHEAD = 16, CR_N = 8;
-template <class TC>
 __global__ void __launch_bounds__(256) conv_reduce_kernel(const double *P, int splits, int64_t stride, int64_t M, int64_t N,
-                                                          TC *C, int64_t rs, int64_t cs, double alpha, double beta,
+                                                          float *C, int64_t rs, int64_t cs, double alpha, double beta,
                                                           int beta_on) {
     __shared__ double tile[32][CR_N + 1];
     const int64_t tn = (N + CR_N - 1) / CR_N, m0 = blockIdx.x / tn * 32, n0 = blockIdx.x % tn * CR_N;
@@ -358,23 +354,21 @@ __global__ void __launch_bounds__(256) conv_reduce_kernel(const double *P, int s
     __syncthreads();
     const int i = rs == 1 ? x : (int)threadIdx.x / CR_N, j = rs == 1 ? y : (int)threadIdx.x % CR_N;
     if (m0 + i >= M || n0 + j >= N) return;
-    TC *c = C + (m0 + i) * rs + (n0 + j) * cs;
+    float *c = C + (m0 + i) * rs + (n0 + j) * cs;
     double v = alpha * tile[i][j];
     if (beta_on) v += beta * (double)*c;
-    *c = (TC)v;
+    *c = (float)v;
 }
 
-// C (M x N, ld ldc, TC) = alpha * op(A) * op(B) + beta * C for Float32 A and B (an FP32-accurate
+// C (M x N, ld ldc) = alpha * op(A) * op(B) + beta * C for Float32 A and B (an FP32-accurate
 // product).  The operand with more elements is converted in the kernel; when that is B, the
 // transposed product is computed and written with its strides exchanged.  The other one is split
 // beforehand into K-major terms in the context's memory pool.  Gaussian A * Omega, A 65536 x 1024,
 // Omega 1024 x 128: 304 us a call, 394 us with both operands split in memory.
-template <class TC>
 int gemm_f32_tc(rla_ctx *ctx, int64_t M, int64_t N, int64_t K, const float *A, int64_t lda, int ta, const float *B,
-                int64_t ldb, int tb, TC *C, int64_t ldc, double alpha, double beta) {
-    constexpr int NT = 3;
+                int64_t ldb, int tb, float *C, int64_t ldc, double alpha, double beta) {
     if (M <= 0 || N <= 0) return RLA_OK;
-    if (K <= 0) return gemm<float, float, TC, double>(ctx, M, N, K, A, lda, ta, B, ldb, tb, C, ldc, alpha, beta);
+    if (K <= 0) return gemm<float, float, float, double>(ctx, M, N, K, A, lda, ta, B, ldb, tb, C, ldc, alpha, beta);
     if (M >= (1ll << 31) || K >= (1ll << 31) || N >= (1ll << 31))
         return set_error(ctx, RLA_E_UNSUPPORTED, "tensor-core GEMM: dimension above 2^31");
     // every tile of 64 columns converts its 128 rows of A again: above four of them splitting A once in
@@ -382,7 +376,7 @@ int gemm_f32_tc(rla_ctx *ctx, int64_t M, int64_t N, int64_t K, const float *A, i
     // so short that the FP64 partial tiles of the other kernel cost more (4096 x 30000, converting / split
     // before: K = 16 615 / 1246 us, K = 128 1032 / 1415, K = 256 1446 / 1689)
     if (std::min(M, N) > 4 * CV_BN && K > 256)
-        return gemm_f32_tc_presplit<TC>(ctx, M, N, K, A, lda, ta, B, ldb, tb, C, ldc, alpha, beta);
+        return gemm_f32_tc_presplit(ctx, M, N, K, A, lda, ta, B, ldb, tb, C, ldc, alpha, beta);
     int64_t rs = 1, cs = ldc;
     // The larger operand is converted, unless the other way round fills the tiles so much better that
     // it makes up for splitting the larger one in memory (each tile saved for 64 rows more; 130 x 120,
@@ -404,8 +398,8 @@ int gemm_f32_tc(rla_ctx *ctx, int64_t M, int64_t N, int64_t K, const float *A, i
     int *status = nullptr;
     RLA_TRY(tc_status_get(ctx, &status));
     const int64_t budget = ctx->smem_optin - 1024 - 256 - (int64_t)CV_RAW * CV_RAW_BYTES;
-    const int stages = (int)std::min<int64_t>(4, budget / cv_stage_bytes(NT));
-    const size_t smem = 1024 + 256 + (size_t)stages * cv_stage_bytes(NT) + CV_RAW * CV_RAW_BYTES;
+    const int stages = (int)std::min<int64_t>(4, budget / CV_STAGE_BYTES);
+    const size_t smem = 1024 + 256 + (size_t)stages * CV_STAGE_BYTES + CV_RAW * CV_RAW_BYTES;
     // K splits: the rounds of CTAs times the k-blocks of a split (1.2 us each) and of a CTA's start (4),
     // and the sums of the partial tiles (4 us, 16 bytes an element at 4 TB/s).  16384 x 260 to 200 rows,
     // 12 tiles: 117 us a call in 13 splits, 90 in 12; 11234 x 2778 to 244, 88 tiles: 465 in one, 321 in five.
@@ -436,21 +430,21 @@ int gemm_f32_tc(rla_ctx *ctx, int64_t M, int64_t N, int64_t K, const float *A, i
     RLA_CUDA_TRY(ctx, pool_malloc_s(ctx, (void **)&buf, sizeof(bf16) * 3 * nb + 256, ctx->stream));
     bf16 *b3[3] = {buf, buf + nb, buf + 2 * nb};
     int rc = tb ? split_terms_launch<NT>(ctx, B, N, K, ldb, 1, b3, ldb2) : split_terms_launch<NT>(ctx, B, K, N, ldb, 0, b3, ldb2);
-    ConvMaps<NT> maps;
+    ConvMaps maps;
     for (int t = 0; t < NT && rc == RLA_OK; ++t) rc = tc_make_map(ctx, &maps.b[t], b3[t], K, N, ldb2, TC_BK, CV_BN);
     auto launch = [&]() -> int {
         const bool part = splits > 1;
         ConvArgs p{A, lda, lda % 4 == 0 && (uintptr_t)A % 16 == 0, (int)M, (int)N, (int)K,
-                   part ? ws : (void *)C, nullptr, part ? 1 : rs, part ? M : cs, part || sizeof(TC) == 8,
+                   part ? ws : (void *)C, part ? 1 : rs, part ? M : cs, part,
                    part ? 1.0 : alpha, beta, !part && beta != 0.0, stages, status, ctx->wait_ns};
-        RLA_CUDA_TRY(ctx, set_smem_max(conv_gemm_kernel<NT>));
+        RLA_CUDA_TRY(ctx, set_smem_max(conv_gemm_kernel));
         cudaEvent_t e0 = timing_begin(ctx);
-        conv_gemm_kernel<NT><<<dim3((unsigned)tiles, (unsigned)splits), CV_THREADS, smem, ctx->stream>>>(
+        conv_gemm_kernel<<<dim3((unsigned)tiles, (unsigned)splits), CV_THREADS, smem, ctx->stream>>>(
             maps, p, ta, (int)ntl, (int)nkb, (int)kbps, M * N);
         RLA_TRY(check_launch(ctx, "conv_gemm"));
         timing_end(ctx, 0, e0);
         if (!part) return RLA_OK;
-        conv_reduce_kernel<TC><<<(unsigned)(ceil_div(M, 32) * ceil_div(N, CR_N)), 256, 0, ctx->stream>>>(
+        conv_reduce_kernel<<<(unsigned)(ceil_div(M, 32) * ceil_div(N, CR_N)), 256, 0, ctx->stream>>>(
             (const double *)ws, (int)splits, M * N, M, N, C, rs, cs, alpha, beta, beta != 0.0);
         return check_launch(ctx, "conv_reduce");
     };
@@ -458,10 +452,5 @@ int gemm_f32_tc(rla_ctx *ctx, int64_t M, int64_t N, int64_t K, const float *A, i
     cudaFreeAsync(buf, ctx->stream);
     return rc;
 }
-
-template int gemm_f32_tc<float>(rla_ctx *, int64_t, int64_t, int64_t, const float *, int64_t, int, const float *,
-                                int64_t, int, float *, int64_t, double, double);
-template int gemm_f32_tc<double>(rla_ctx *, int64_t, int64_t, int64_t, const float *, int64_t, int, const float *,
-                                 int64_t, int, double *, int64_t, double, double);
 
 }  // namespace rla
