@@ -685,7 +685,7 @@ def sparse_sign_arm(args):
             "config": {"workload": SS_WORKLOAD, "m": SS_M, "n": SS_N, "s": SS_S, "nnz": SS_NNZ,
                        "parallelism": f"replicas x{world}",
                        "l2": "A and C (9.4 MB) stay in L2 between steps: an L2 rate, not an HBM rate"},
-            "roofline": {"bound": "hbm", "kernel": "compress_contig_kernel", "achieved": round(value / world, 2),
+            "roofline": {"bound": "hbm", "kernel": "tile_compress_kernel", "achieved": round(value / world, 2),
                          "peak": peak, "peak_source": peak_kind, "unit": "GB/s",
                          "frac": round(value / world / peak, 4), "traffic": None,
                          "note": "L2-resident workload; the fraction is of HBM peak for scale only"},

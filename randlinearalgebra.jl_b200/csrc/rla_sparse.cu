@@ -5,8 +5,12 @@
 // magnitude `scale`.  The reference applies it through SparseArrays' CSC kernels
 // (sparse_sign.jl:339-361, count_sketch.jl:166-213); here:
 //
-//  * compress, contiguous vectors (S*A with Left S on column-major A, the sketch hot
-//    path): each warp owns private shared-memory bins for one output vector and streams
+//  * SparseSign (nnz <= 32, s <= 8320), CountSketches with up to 2080 buckets and the strided vectors
+//    of a Right CountSketch take the tile kernel of rla_sparse_tile.cu; the two compress forms here
+//    the rest (CountSketches with more buckets, as in the headline sketch, and what lies beyond
+//    the tile kernel's limits).
+//  * compress, contiguous vectors (S*A with Left S on column-major A): each warp owns private
+//    shared-memory bins for one output vector and streams
 //    its input vector with 16-byte loads.  Buckets that would collide inside a warp access
 //    were scheduled away when the sketch was drawn (CountSketch: moved to a per-warp list
 //    folded in by extra rounds; SparseSign: extra rounds), so no atomics are used and the
@@ -15,7 +19,8 @@
 //    arrive, which adds the partial bins in warp order.
 //  * compress, strided vectors (A*S with Right S: rows of column-major A): lane = vector,
 //    the bucket is warp-uniform, bins are [bucket][lane] (conflict-free).
-//  * expand (S'*A, A*S' ...): a gather, one thread per output element.
+//  * expand (S'*A, A*S' ...): a gather, on staged rows (rla_sparse_lift.cu) or, where that does not
+//    pay, one thread per output element.
 #include "rla_internal.cuh"
 #include "rla_kernels.cuh"
 
@@ -690,7 +695,7 @@ int sparse_compress(rla_ctx *ctx, const rla_sketch *sk, const T *X, int64_t x_es
     const bool beta_zero = beta == 0.0;
     const T a = (T)(alpha * sk->scale);
     if (nv == 0) return RLA_OK;
-    // nnz > 1: the tile kernel for every layout (150001 -> 1332 of 333 columns: 257 us against 603 us
+    // nnz > 1: the tile kernel for every layout (150001 -> 1332 of 333 columns: 254 us against 603 us
     // below); nnz = 1: for strided vectors, while contiguous ones keep the batch kernel, whose
     // warps read each element's word once and fill HBM better (s = 4096 would take four windows).
     if (sk->bl_ok && (x_es != 1 || !sk->batch_mode))

@@ -6,8 +6,8 @@
 // bytes.  Each warp takes 32 long indices at a time: it packs their entries into 16-bit words,
 // sums the nnz rows of four (32/LPE) long indices per step in registers, and turns the 32 x C
 // block of results through shared memory into 16-byte column stores.  Bound by the row reads
-// (nnz wavefronts per 128 bytes of output; shared-memory pipe 68 % busy, the output's HBM
-// traffic alone would take 32 us): 131072 x 200 Float64, s = 1000, nnz = 8 in 122 us, 436 us with
+// (nnz wavefronts per 128 bytes of output; shared-memory pipe 79 % busy, the output's HBM
+// traffic alone would take 32 us): 131072 x 200 Float64, s = 1000, nnz = 8 in 120 us, 436 us with
 // a thread per output element.  The entry loop is unrolled for the usual nnz (154 us without).
 //
 // LPE = 8 / 4 / 2 lanes per entry (rows of 128 / 64 / 32 bytes) for s up to 1095 / 2380 / 4309 at

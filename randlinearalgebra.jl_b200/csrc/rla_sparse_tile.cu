@@ -11,12 +11,12 @@
 // last group of a bucket filled up with a row of zeros: a step of the kernel adds one group per octet to its bucket, with no
 // branches.  With e = R * nnz / s entries per bucket and chunk and g = ceil(e/4) groups,
 //   wavefronts per bucket and chunk = g * (4 rows + 2 bins + 1/4 words).
-// Measured (unprofiled call): 150001 -> 1332 (nnz 8) of 333 Float32 columns 257 us, 603 us with one
-// output vector per warp and private bins; 3000 -> 100 (nnz 8) of 30011 Float32 rows 307 us,
-// 1526 us with lane = vector bins; 4096 -> 512 of 256 Float64 columns 40 against 71 us.  The
-// shared-memory pipe is 73 % busy at the second size.  Entry by entry with an end-of-run
-// flag instead of filled groups takes fewer wavefronts and half again as many instructions: 258
-// and 308 us.
+// Measured (unprofiled call): 150001 -> 1332 (nnz 8) of 333 Float32 columns 254 us, 603 us with one
+// output vector per warp and private bins; 3000 -> 100 (nnz 8) of 30011 Float32 rows 297 us,
+// 1526 us with lane = vector bins; 4096 -> 512 of 256 Float64 columns 39 against 71 us.  The
+// shared-memory pipe is 72 % busy at the second size.  Entry by entry with an end-of-run
+// flag instead of filled groups takes fewer wavefronts and half again as many instructions, and came
+// out the same (258 and 308 us, when groups took 257 and 307).
 // A CTA of 16 warps walks (vector tile, bucket window, chunk) units; each warp owns the
 // buckets congruent to it modulo 16, so there are no atomics and the result is reproducible bit
 // for bit.  Vectors that are contiguous in j (columns of a column-major A) are transposed on the

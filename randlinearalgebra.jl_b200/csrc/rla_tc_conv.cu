@@ -12,7 +12,7 @@
 // Warps: 0 TMA producer of B, 1 MMA issuer, 2 TMEM allocator, 4..11 chunk drain / epilogue (lane
 // quarter by warp mod 4, 32 of the 64 columns each), 12..15 converters.  A tile is 128 x 64.
 // Bound by the converters' chain per k-block (copy, convert, store, proxy fence, arrive; four warps):
-// the tensor pipe is 17 % and the ALU pipe 24 % busy at 65536 x 1024 x 128.
+// the tensor pipe is 18 % and the ALU pipe 25 % busy at 65536 x 1024 x 128.
 #include "rla_internal.cuh"
 #include "rla_kernels.cuh"
 #include "rla_tc.cuh"
@@ -364,7 +364,7 @@ __global__ void __launch_bounds__(256) conv_reduce_kernel(const double *P, int s
 // product).  The operand with more elements is converted in the kernel; when that is B, the
 // transposed product is computed and written with its strides exchanged.  The other one is split
 // beforehand into K-major terms in the context's memory pool.  Gaussian A * Omega, A 65536 x 1024,
-// Omega 1024 x 128: 304 us a call, 394 us with both operands split in memory.
+// Omega 1024 x 128: 289 us a call, 394 us with both operands split in memory.
 int gemm_f32_tc(rla_ctx *ctx, int64_t M, int64_t N, int64_t K, const float *A, int64_t lda, int ta, const float *B,
                 int64_t ldb, int tb, float *C, int64_t ldc, double alpha, double beta) {
     if (M <= 0 || N <= 0) return RLA_OK;

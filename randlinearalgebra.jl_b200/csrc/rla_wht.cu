@@ -547,7 +547,7 @@ __global__ void srht_expand_kernel(const T *X, int64_t x_es, int64_t x_vs, int64
 // between the first read and the last write stay in L2 (126 MB).
 //
 // Bound by the loads' latency in the near kernel (2 CTAs per SM, all of a thread's loads in flight
-// together) and by L2 in the rest.  FJLT 100003 -> 600 of 96 Float32 columns: 88 us a call
+// together) and by L2 in the rest.  FJLT 100003 -> 600 of 96 Float32 columns: 83 us a call
 // (near 30, far 10, gather 19), 324 us with a padding pass, scalar shared-memory stages and one
 // pass over the workspace per bit above 2^12; SRHT expand to 360737 x 61: 156 against 416 us, SRHT
 // 5003 -> 300 of 200 columns 28 against 85 us.
