@@ -820,7 +820,9 @@ int sparse_expand(rla_ctx *ctx, const rla_sketch *sk, const T *X, int64_t x_es, 
     RLA_TRY(sparse_lift<T>(ctx, sk, X, x_es, x_vs, nv, Y, y_es, y_vs, (T)(alpha * sk->scale), (T)beta, beta == 0.0, &taken));
     if (taken) return RLA_OK;
     const int64_t L = sk->L;
-    const int out_contig = y_es == 1;
+    // threads along the contiguous dimension; one vector with strides: along its elements (551399 x 1,
+    // nnz 4, every second element, Float64: 149 us with a block per element, 26 now)
+    const int out_contig = y_es == 1 || nv == 1;
     const int64_t fast = out_contig ? L : nv, slow = out_contig ? nv : L;
     dim3 block(128, 2);
     dim3 grid(ceil_div_i(fast, 128), (unsigned)std::min<int64_t>(ceil_div(slow, 2), 65535));

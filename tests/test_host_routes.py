@@ -314,3 +314,14 @@ def test_presplit_sizes_are_split_beforehand(fake, card, adjoint):
         other += any("conv_gemm" in k for k in fake.launches())
         fake.lib.rla_sketch_destroy(sk)
     assert other == 3
+
+
+@pytest.mark.parametrize("dtype", [F32, F64])
+def test_expand_of_one_strided_vector_has_threads_along_it(fake, dtype):
+    ctx = fake.context()
+    L, s = 551399, 6
+    sk = fake.sketch(ctx, "sparse_sign", s, L, card=RIGHT, dtype=dtype, nnz=4)
+    fake.reset()
+    assert fake.mul(ctx, sk, (s, L, 1), RIGHT, adjoint=True, pad=1) == 0  # a row of a column-major result
+    (x, y, threads), = grids(fake.log(), "expand_kernel")
+    assert x * y * threads < 3 * L
