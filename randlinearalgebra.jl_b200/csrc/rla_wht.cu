@@ -1129,11 +1129,25 @@ int srht_expand(rla_ctx *ctx, const rla_sketch *sk, const T *X, int64_t x_es, in
     // 60 / 53), nor in a graph capture: the graph would keep the scratch after a later call had grown it
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     RLA_CUDA_TRY(ctx, cudaStreamIsCapturing(ctx->stream, &cap));
-    if (y_es == 1 || nv <= (sk->L < 65536 ? 3 : beta != 0.0 ? 6 : sizeof(T) == 4 ? 16 : 12) || cap != cudaStreamCaptureStatusNone)
-        return launch_near<T, WHT_IN_SAMPLES, WHT_OUT_Y>(ctx, p);
-    void *w;
-    RLA_TRY(scratch_get(ctx, (size_t)(sk->N * nb) * sizeof(T), &w));
-    p.W = (T *)w;
+    const bool fixed = cap != cudaStreamCaptureStatusNone;
+    const bool staged = y_es != 1 && nv > (sk->L < 65536 ? 3 : beta != 0.0 ? 6 : sizeof(T) == 4 ? 16 : 12) && !fixed;
+    // Every chunk of a column gathers all of its samples: rows of a row-major operand are turned into
+    // columns once for that (44736 x 820 from 6810, Float64: 1278 us a call across the rows, 1014 now)
+    const bool turn = x_es != 1 && sk->N > ((int64_t)1 << WhtCfg<T>::CH) && sk->s * nv >= (1 << 18) && nv <= 65535 * 32 && !fixed;
+    const size_t w_bytes = staged ? ((size_t)(sk->N * nb) * sizeof(T) + 255) / 256 * 256 : 0;
+    if (staged || turn) {
+        void *w;
+        RLA_TRY(scratch_get(ctx, w_bytes + (turn ? (size_t)(sk->s * nv) * sizeof(T) : 0), &w));
+        p.W = (T *)w;
+        if (turn) {
+            T *xt = (T *)((char *)w + w_bytes);
+            RLA_TRY(to_contiguous(ctx, X, x_es, x_vs, sk->s, nv, xt));
+            X = p.X = xt;
+            p.x_es = 1;
+            p.x_vs = x_vs = sk->s;
+        }
+    }
+    if (!staged) return launch_near<T, WHT_IN_SAMPLES, WHT_OUT_Y>(ctx, p);
     for (int64_t v = 0; v < nv; v += nb) {
         p.nv = std::min(nb, nv - v);
         p.X = X + v * x_vs;

@@ -325,3 +325,23 @@ def test_expand_of_one_strided_vector_has_threads_along_it(fake, dtype):
     assert fake.mul(ctx, sk, (s, L, 1), RIGHT, adjoint=True, pad=1) == 0  # a row of a column-major result
     (x, y, threads), = grids(fake.log(), "expand_kernel")
     assert x * y * threads < 3 * L
+
+
+#       L, s, nv, row-major Y, turned
+SRHT_TURNED = [(44736, 6810, 820, True, True), (1 << 18, 4096, 100, True, True), (44736, 6810, 820, False, False),
+               (16000, 4096, 820, True, False), (1 << 18, 40, 100, True, False), (44736, 6810, 1, True, False)]
+
+
+@pytest.mark.parametrize("row_c", [False, True])
+@pytest.mark.parametrize("case", SRHT_TURNED)
+def test_srht_expand_turns_row_major_samples(fake, case, row_c):
+    """Every chunk of a long column gathers all samples: rows are turned into columns once, but not in
+    a graph capture, which would keep the scratch."""
+    L, s, nv, row_y, turned = case
+    ctx = fake.context()
+    sk = fake.sketch(ctx, "srht", s, L)
+    for capturing in (False, True):
+        fake.reset()
+        fake.capturing(capturing)
+        assert fake.mul(ctx, sk, (s, L, nv), LEFT, adjoint=True, row_a=row_y, row_c=row_c, wait=False) == 0
+        assert ("gather_columns" in fake.launches()[0]) == (turned and not capturing), fake.launches()
