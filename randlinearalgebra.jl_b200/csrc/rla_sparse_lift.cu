@@ -149,6 +149,16 @@ __global__ void __launch_bounds__(LIFT_WARPS * 32, 1) lift_kernel(LiftParams<T> 
                     (uint16_t)((uint32_t)__ldg(p.bucket + j0 * nnz + i) | ((uint32_t)__ldg(p.negative + j0 * nnz + i) << 15));
             }
         }
+        if (!p.beta_zero) {  // the old values of the block come into L2 during its sums
+            const T *yb = p.Y + j0 * p.y_es + v0 * p.y_vs;
+            if (p.y_es == 1) {
+                for (int c = 0; c < nc; ++c)
+                    if (lane < cnt) asm volatile("prefetch.global.L2 [%0];" ::"l"(yb + lane + c * p.y_vs));
+            } else {
+                for (int i = lane; i < cnt * C; i += 32)
+                    if (i % C < nc) asm volatile("prefetch.global.L2 [%0];" ::"l"(yb + i / C * p.y_es + i % C * p.y_vs));
+            }
+        }
         __syncwarp();
         // ---- sums of JS long indices per step ----
         const int l = lane % LPE, g = lane / LPE;
@@ -194,8 +204,8 @@ __global__ void __launch_bounds__(LIFT_WARPS * 32, 1) lift_kernel(LiftParams<T> 
         T *yb = p.Y + j0 * p.y_es + v0 * p.y_vs;
         if (!p.beta_zero) {
             // lanes along the contiguous dimension; the old values of eight elements per lane are read
-            // before the first one is written (509022 x 100 Float64 from 43, nnz 2: 562 us a call one by
-            // one, 308 now)
+            // before the first one is written (131072 x 200 Float64 from 1000, nnz 8: 281 us a call one by
+            // one, 189 now)
             constexpr int STEP = 8;
             const bool down = p.y_es == 1;
             for (int i0 = 0; i0 < (down ? C : cnt * C / 32 + 1); i0 += STEP) {
@@ -274,7 +284,8 @@ struct LiftGrid {
 //    16, nnz 8, s = 1000: 33 / 38; 131072 x 32, nnz 1: 42 / 36.  A tile of 32 (Float64: 16) vectors
 //    that is mostly empty costs as much as a full one: 2^20 long indices of nnz 8, 1 vector
 //    38 / 73, 4 vectors 81 / 72; nnz 1, 4 vectors 41 / 48, 8 vectors 57 / 49; nnz 3 (no unrolled
-//    loop) 8 vectors 67 / 73, 16 vectors 110 / 81.
+//    loop) 8 vectors 67 / 73, 16 vectors 110 / 81.  With beta the old values take this one longer: Float64
+//    1000481 x 22, nnz 3 155 / 220, 131072 x 200, nnz 8 442 / 189; 4239 x 179, nnz 12: 30 / 40.
 //  * Other results by the sum of what each kernel spends (below).  Row-major: that kernel's blocks
 //    hold 128 vectors whatever their number is, and read a column-major operand across: 2^20 x 2,
 //    nnz 8: 300 / 95; 30000 x 32, nnz 8, s = 1000: 39 / 51; 131072 x 16, nnz 1: 66 / 42; 8000 x 500, nnz 16,
@@ -286,13 +297,15 @@ struct LiftGrid {
 //    column-major operand, s = 1 149 / 224, s = 1000 197 / 187.
 //  * Two lanes per entry, Float64: tiles of 4 vectors write 32-byte pieces of rows (2^20 x 64, nnz 1:
 //    302 / 401), and with nnz 3 the words of 2^20 long indices are read again for every four
-//    columns (2^20 x 64: 415 / 485; 131072 x 200: 226 / 178); with beta 229508 x 198, nnz 1: 304 / 379.
+//    columns (2^20 x 64: 415 / 485; 131072 x 200: 226 / 178); with beta 229508 x 198, nnz 1: 304 / 379, and 29150 x
+//    1119, nnz 2, row-major: 335 / 480.
 template <class T>
 static bool lift_pays(const rla_sketch *sk, const LiftGrid &g, int lpe, int64_t x_es, int64_t nv, int64_t y_es, bool beta) {
     if (nv < 2) return false;
     const int64_t L = sk->L, nnz = sk->nnz, staged = sk->s * lpe;
     const bool unrolled = nnz == 1 || nnz == 2 || nnz == 4 || nnz == 8, narrow64 = sizeof(T) == 8 && lpe == 2;
     const bool rows_in = x_es != 1, rows_out = y_es != 1;
+    if (narrow64 && beta && nnz <= 2) return false;
     if (rows_out) {
         if (narrow64 && nv > 32 && nnz != 8 && rows_in) return false;
         if (y_es * sizeof(T) % 32 != 0 && L * nv * (int64_t)sizeof(T) > 110000000 && g.tiles > 3) {
@@ -300,10 +313,10 @@ static bool lift_pays(const rla_sketch *sk, const LiftGrid &g, int lpe, int64_t 
             if (!rows_in && sizeof(T) == 8 && nnz == 1 && (sk->s <= 300 || lpe < 8)) return false;
         }
     } else {
-        if (narrow64 && ((beta && nnz <= 2) || (!unrolled && nnz < 8 && L >= (1 << 19)))) return false;
+        if (narrow64 && !unrolled && nnz < 8 && L >= (1 << 19)) return false;
         if (L >= 1024) {
-            if (nv < (nnz >= 8 ? 4 : unrolled ? 8 : 16)) return false;
-            return L * nv * (2 + nnz) >= std::max<int64_t>(1000 * staged * (rows_in ? 2 : 1), 6000000);
+            if (nv < (nnz >= 8 ? 4 : unrolled ? 8 : 16) || (beta && nnz < 4)) return false;
+            return L * nv * (2 + nnz) >= (beta ? 2 : 1) * std::max<int64_t>(1000 * staged * (rows_in ? 2 : 1), 6000000);
         }
     }
     // us: that kernel's blocks of 128 outputs, gathered values and output bytes; here the stagings, their

@@ -20,14 +20,15 @@ SIZES = [(60011, 40, 8, 37, 8), (120011, 1095, 1, 33, 8), (60021, 300, 3, 50, 8)
          (30007, 64, 32, 19, 8), (120027, 1200, 2, 61, 4), (40009, 2380, 8, 131, 4), (120007, 3000, 4, 29, 2),
          (124003, 4309, 8, 40, 2), (126001, 3000, 3, 30, 2)]
 #          row-major Y, row-major C, padding, alpha, beta
-LAYOUTS = {"col": (False, False, 0, 1.0, 0.0), "col_odd": (False, False, 1, 0.5, -2.0), "row": (True, True, 0, 1.0, 0.0),
+LAYOUTS = {"col": (False, False, 0, 1.0, 0.0), "col_odd": (False, False, 1, 0.5, 0.0), "col_beta": (False, False, 1, 0.5, -2.0), "row": (True, True, 0, 1.0, 0.0),
            "row_beta": (True, True, 0, 0.5, -2.0), "row_to_col": (True, False, 0, 1.0, 0.0),
            "col_to_row": (False, True, 0, 1.0, 0.0)}
 
 
 def sizes(layout):
-    """The sizes of a layout: staging a row-major Y for a column-major result pays later."""
-    return [z for z in SIZES if layout != "row_to_col" or z[1] * z[4] <= 2400]
+    """The sizes of a layout: staging a row-major Y for a column-major result pays later, with beta only for
+    four entries and more."""
+    return [z for z in SIZES if (layout != "row_to_col" or z[1] * z[4] <= 2400) and (layout != "col_beta" or z[2] >= 4)]
 
 
 @pytest.mark.parametrize("dtype", [np.float32, np.float64])

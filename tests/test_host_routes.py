@@ -263,6 +263,8 @@ EXPAND_COSTS = [
     (200, 50, 8, 40000, F64, False, False, 0, 0.0, True), (155, 12, 12, 49361, F64, True, False, 0, 0.0, True),
     # old values of the result
     (3683, 23, 2, 181, F32, True, True, 0, 0.5, False), (1599, 18, 1, 848, F32, True, True, 0, 0.5, False),
+    (1000481, 3, 3, 22, F64, True, False, 1, 0.5, False), (4239, 90, 12, 179, F32, False, False, 0, 0.5, False),
+    (131072, 1000, 8, 200, F64, False, False, 0, 0.5, True), (29150, 3884, 2, 1119, F64, False, True, 1, 0.5, False),
     (229508, 3223, 1, 198, F64, False, False, 0, 0.5, False), (229508, 3223, 1, 198, F64, False, False, 0, 0.0, True),
 ]
 
